@@ -44,7 +44,7 @@ namespace cg = cooperative_groups;
 
 namespace cvdv {
 
-constexpr int kRowMinLogN = 8;  // shorter registers use the pass kernels
+constexpr int kRowMinLogN = 4;  // shorter registers use the pass kernels
 
 template <typename C> struct RowCfg;
 template <> struct RowCfg<double2> {
@@ -97,6 +97,7 @@ struct RowProgram {
   int logTwN;
   int loadT;    // cluster rows: start transposed (1: from the natural layout, 2: from the blocked one)
   int storeBlocked;  // cluster rows ending transposed: write the blocked layout
+  int rowMask;       // k_rowr: rows (columns) of the state less one, at most those of a CTA less one
   int logS;          // k_rowr on a strided register: log2 of the amplitudes below it (0: rows)
   const double2* tw;
   double* rowSums;        // non-null: per-warp partial sums of |psi|^2 of every row's result
@@ -594,10 +595,14 @@ __device__ __forceinline__ void row_sum_part(const C (&v)[E], double* out) {
   if ((threadIdx.x & (W - 1)) == 0) *out = a;
 }
 
+//
+// A state of fewer rows than a CTA holds (nRows < 2^LOGR, both powers of two) runs
+// as one tile whose surplus thread groups repeat its rows: they read the same
+// input and write the same values.
 template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
 __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR) > 8 ? 1 : 2)
     k_rowr(const C* __restrict__ in, C* __restrict__ out, uint64_t nTiles, const __grid_constant__ RowProgram P) {
-  constexpr int E = 1 << LOGE, M = 1 << LOGM, TPR = M >> LOGE, NT = TPR << LOGR, RS = M + (M >> 4);
+  constexpr int E = 1 << LOGE, M = 1 << LOGM, TPR = M >> LOGE, NT = TPR << LOGR, RS = rr_row_slots(LOGM, LOGE);
   constexpr uint32_t TILE_BYTES = (uint32_t)sizeof(C) << (LOGM + LOGR);
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
@@ -606,15 +611,16 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR
   const int tid = threadIdx.x;
   // column form: the CTA's 2^LOGR adjacent columns interleave lane by lane, so a
   // warp's load covers 32 / 2^LOGR points of every column in runs of 2^LOGR
-  const int row = COL ? (tid & ((1 << LOGR) - 1)) : tid >> (LOGM - LOGE);
+  int row = COL ? (tid & ((1 << LOGR) - 1)) : tid >> (LOGM - LOGE);
   const int t = COL ? (tid >> LOGR) : tid & (TPR - 1);
   C* smrow = sm + row * RS;
   const int logS = COL ? P.logS : 0;
+  if constexpr (LOGM < 8) row &= P.rowMask;  // (longer rows: LOGR = 0 where rows are few)
 
   const int scM = P.logTwN - LOGM;
-  for (int i = tid; i < 64 + (M >> 6); i += NT) {
+  for (int i = tid; i < rr_tw_slots(LOGM); i += NT) {
     const int e = i < 64 ? i : (i - 64) << 6;
-    lo[i] = __ldg(P.tw + ((size_t)e << scM));  // lo and hi are one array
+    if (e < M) lo[i] = __ldg(P.tw + ((size_t)e << scM));  // lo and hi are one array
   }
   __syncthreads();
   // No barrier between tiles: after a transform's last exchange (which ends in a
@@ -653,21 +659,24 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR
 static int rowr_max_log(int precision) { return precision == kC128 ? 13 : 14; }
 
 // complex64 rows of 2^13 and 2^14 points keep 32 amplitudes per thread (256 / 512
-// threads); everything else 16
+// threads); everything else 16, and rows shorter than 2^8 points 8
 template <typename C, int LOGM>
 struct RrShape {
-  static constexpr int LOGE = (sizeof(C) == sizeof(float2) && LOGM >= 13) ? 5 : 4;
-  static constexpr int LOGR = LOGM - LOGE < 8 ? 8 - (LOGM - LOGE) : 0;
+  static constexpr int LOGE = LOGM < 8 ? 3 : (sizeof(C) == sizeof(float2) && LOGM >= 13) ? 5 : 4;
+  static constexpr int LOGR = LOGM < 8 ? 10 - LOGM : LOGM - LOGE < 8 ? 8 - (LOGM - LOGE) : 0;
 };
 
-template <typename C, int LOGM, bool COL>
-static cudaError_t launch_rowr_t(Context* ctx, const RowProgram& P) {
-  constexpr int LOGE = RrShape<C, LOGM>::LOGE, LOGR0 = RrShape<C, LOGM>::LOGR;
-  // column form: at least two columns a CTA while it stays within 512 threads
-  constexpr int LOGR = (COL && LOGR0 == 0 && (LOGM - LOGE) < 9) ? 1 : LOGR0;
+// Rows of 2^8 .. 2^12 points of a state below 2^kRowrSmallLog amplitudes run one row
+// per CTA at 8 amplitudes a thread (radix-8 stages): such a state does not fill the
+// chip, so a program takes the latency of one CTA's chain, and twice the warps on a
+// row shorten it.
+constexpr int kRowrSmallLog = 19;
+static bool rowr_small(Context* ctx) { return ctx->totalQbt < kRowrSmallLog; }
+
+template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
+static cudaError_t launch_rowr_s(Context* ctx, const RowProgram& P) {
   constexpr int NT = 1 << (LOGM - LOGE + LOGR);
-  constexpr int M = 1 << LOGM;
-  const size_t smem = (size_t)(M + (M >> 4)) * (1 << LOGR) * sizeof(C) + (64 + (M >> 6)) * sizeof(double2);
+  const size_t smem = (size_t)rr_row_slots(LOGM, LOGE) * (1 << LOGR) * sizeof(C) + rr_tw_slots(LOGM) * sizeof(double2);
   auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL>;
   static int resident = 0;  // CTAs per SM of this instantiation, asked once
   cudaError_t e = cudaSuccess;
@@ -677,16 +686,32 @@ static cudaError_t launch_rowr_t(Context* ctx, const RowProgram& P) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, NT, smem);
     if (e != cudaSuccess || resident < 1) return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
   }
-  const uint64_t nTiles = ctx->size() >> (LOGM + LOGR);
+  uint64_t nTiles = ctx->size() >> (LOGM + LOGR);
+  if (nTiles < 1) nTiles = 1;
   uint64_t grid = NT > 256 ? (uint64_t)ctx->numSMs * resident : nTiles;
   if (grid > nTiles) grid = nTiles;
   kern<<<(unsigned)grid, NT, smem, ctx->stream>>>((const C*)ctx->state(), (C*)ctx->other(), nTiles, P);
   return cudaGetLastError();
 }
 
+template <typename C, int LOGM, bool COL>
+static cudaError_t launch_rowr_t(Context* ctx, const RowProgram& P) {
+  constexpr int LOGE = RrShape<C, LOGM>::LOGE, LOGR0 = RrShape<C, LOGM>::LOGR;
+  // column form: at least two columns a CTA while it stays within 512 threads
+  constexpr int LOGR = (COL && LOGR0 == 0 && (LOGM - LOGE) < 9) ? 1 : LOGR0;
+  if constexpr (LOGM >= 8 && LOGM <= 12) {
+    if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, 0, 3, COL>(ctx, P);
+  }
+  return launch_rowr_s<C, LOGM, LOGR, LOGE, COL>(ctx, P);
+}
+
 template <typename C, bool COL>
 static cudaError_t launch_rowr(Context* ctx, const RowProgram& P, int q) {
   switch (q) {
+    case 4: return launch_rowr_t<C, 4, COL>(ctx, P);
+    case 5: return launch_rowr_t<C, 5, COL>(ctx, P);
+    case 6: return launch_rowr_t<C, 6, COL>(ctx, P);
+    case 7: return launch_rowr_t<C, 7, COL>(ctx, P);
     case 8: return launch_rowr_t<C, 8, COL>(ctx, P);
     case 9: return launch_rowr_t<C, 9, COL>(ctx, P);
     case 10: return launch_rowr_t<C, 10, COL>(ctx, P);
@@ -708,13 +733,15 @@ static cudaError_t launch_rowr(Context* ctx, const RowProgram& P, int q) {
 // column kernel anyway.
 bool col_program_ok(Context* ctx, int reg) {
   const int q = ctx->q[reg];
-  if (!ctx->colProg || ctx->flw[reg] == 0 || q <= 8 ||
+  if (!ctx->colProg || ctx->flw[reg] == 0 || q < kRowMinLogN ||
       q > rowr_max_log(ctx->precision))
     return false;
+  if (q <= 8) return !(ctx->colFft && col_fft_ok(ctx, reg));  // the column kernel holds whole runs on these
   if (ctx->colFft && col_fft_ok(ctx, reg) && tc_col_ok(ctx, reg)) return false;  // chained tensor-core passes
   const int logE = (ctx->precision == kC64 && q >= 13) ? 5 : 4;
   const int logR = q - logE < 8 ? 8 - (q - logE) : (q - logE < 9 ? 1 : 0);
-  return ctx->totalQbt - q >= logR;
+  // (states below the small-state line run one column per CTA)
+  return (q <= 12 && rowr_small(ctx)) || ctx->totalQbt - q >= logR;
 }
 
 // ---------------------------------------------------------------- cluster register-resident rows
@@ -1093,9 +1120,12 @@ bool row_eligible(Context* ctx, int reg) {
   if (ctx->flw[reg] != 0) return false;
   int lt = row_log_tile(ctx->precision);
   int q = ctx->q[reg];
-  if (q > lt + 3 || q < kRowMinLogN) return false;  // big tile x cluster of 4 at most
-  if (ctx->totalQbt < lt) return false;            // tile larger than the state
-  return true;
+  return q <= lt + 3 && q >= kRowMinLogN;  // big tile x cluster of 4 at most
+}
+
+// Rows of fewer than 2^8 points, and states smaller than k_row's tile, run on k_rowr only.
+static bool rowr_only(Context* ctx, int reg) {
+  return ctx->flw[reg] != 0 || ctx->q[reg] < 8 || ctx->totalQbt < row_log_tile(ctx->precision);
 }
 
 // Split a diagonal run for a row program on `reg`.  Returns false when it does
@@ -1174,13 +1204,14 @@ static bool all_linear(Context* ctx, int reg, const std::vector<Term>& elemTerms
   return true;
 }
 
-// Programs on a strided register run on k_rowr only, which takes no per-element
-// factor other than linear phases.
+// Programs on a strided register, and those on short rows or small states, run on
+// k_rowr only, which takes no per-element factor other than linear phases (at most
+// kMaxXX of them).
 bool row_diag_fits(Context* ctx, int reg, const std::vector<Term>& terms) {
   std::vector<Term> a, b, c;
   std::vector<int> bits;
   if (!split_row_diag(ctx, reg, terms, &a, &bits, &b, &c)) return false;
-  return ctx->flw[reg] == 0 || all_linear(ctx, reg, c);
+  return !rowr_only(ctx, reg) || all_linear(ctx, reg, c);
 }
 
 template <typename C, int LOGC, int LOGT>
@@ -1260,14 +1291,18 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
     toRowr = split_row_diag(ctx, reg, h.terms, &regTerms, &bits, &rowTerms, &elemTerms) &&
              all_linear(ctx, reg, elemTerms);
   }
-  if (col && !toRowr) {
-    set_error(ctx, kErrUnsupported, "column program on register %d needs per-element factors", reg);
+  if (!toRowr && rowr_only(ctx, reg)) {
+    set_error(ctx, kErrUnsupported, "program on register %d needs per-element factors", reg);
     return false;
   }
   P.logS = col ? ctx->flw[reg] : 0;
   P.logN = q;
   P.logM = q - logC;
   P.logRows = q < lt ? lt - q : 0;
+  {
+    const uint64_t rows = ctx->size() >> q;
+    P.rowMask = rows > (1ull << 16) ? (1 << 16) - 1 : (int)rows - 1;
+  }
   P.logTwN = 0;
   while ((1 << P.logTwN) < ctx->twN) ++P.logTwN;
   P.tw = ctx->twiddle;
@@ -1424,7 +1459,8 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
       return false;
     }
     if (rowSums && !col) {
-      const int logE = (ctx->precision == kC64 && q >= 13) ? 5 : 4, tpr = 1 << (q - logE);
+      const int logE = q < 8 || (q <= 12 && rowr_small(ctx)) ? 3 : (ctx->precision == kC64 && q >= 13) ? 5 : 4;
+      const int tpr = 1 << (q - logE);
       P.rowSums = ctx->rowSums;
       ctx->rowSumParts = tpr < 32 ? 1 : tpr / 32;
     }

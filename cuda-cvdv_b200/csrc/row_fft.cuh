@@ -15,6 +15,13 @@ __device__ __forceinline__ int rpad(int e) {
   return e + (e >> LOGP);
 }
 
+// shared-memory elements of a padded row of 2^logM points (8 amplitudes a thread pad
+// every 8), and twiddle entries (w^e, e < 64, then w^(64 h)) for it
+__host__ __device__ constexpr int rr_row_slots(int logM, int logE) {
+  return (1 << logM) + ((1 << logM) >> (logE == 3 ? 3 : 4));
+}
+__host__ __device__ constexpr int rr_tw_slots(int logM) { return 64 + (logM > 6 ? 1 << (logM - 6) : 1); }
+
 // ---------------------------------------------------------------- butterflies
 template <typename C, int DIR>
 __device__ __forceinline__ C rot_mi(C a) {  // * (-DIR i)
