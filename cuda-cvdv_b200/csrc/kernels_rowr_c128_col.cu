@@ -1,0 +1,6 @@
+// k_rowr on columns of complex128 states (one translation unit each, so they build in parallel).
+#include "rowr.cuh"
+
+namespace cvdv {
+template cudaError_t launch_rowr<double2, true>(Context*, const RowProgram&, int);
+}  // namespace cvdv

@@ -1,0 +1,321 @@
+// A row program as the kernels take it, and the register-resident row kernel k_rowr
+// with its launcher, instantiated per precision and form in kernels_rowr_*.cu.
+#pragma once
+
+#include "cvdv_internal.cuh"
+#include "row_fft.cuh"
+
+namespace cvdv {
+
+struct RowOp {
+  int kind;
+  int dir;   // fft: +1 forward, -1 inverse
+  int diag;  // diag: index into RowProgram::diag
+};
+
+struct RowDiag {
+  const double2* tab;  // [2^nCtrl][N] combined factor of the row register, or null
+  int permuted;        // tab stored as [seg][rank][m] for k = rank + C m (transposed layout)
+  int nCtrl;
+  int ctrlShift[2];    // flat-index bits selecting the table segment (row bits)
+  int hasRowF, hasElemF;
+  FactorList rowF;     // factors constant along a row
+  FactorList elemF;    // per-element factors (bilinear terms with the row register)
+  // Bilinear terms c x_row x_other (other register and control bit off the row)
+  // taken out of elemF for k_rowr: along one row they are the linear phase
+  // a (m - regC) regDx with a = sum c x_other (+-1 by the control bit), so a
+  // thread needs two sincos per run instead of one per amplitude.  The other
+  // register is side 1 of each XXFactor.
+  int nLin;
+  double regC, regDx;
+  XXFactor lin[kMaxXX];
+  // k_rowq: a run whose register terms are linear phases (no table): transform
+  // twiddles, the sum of their signs s giving exp(i pi s (N-1)(2n-N+1)/(2N)) at
+  // point n, and terms c x_n (x_n = (n - regC) regDx), each negated when its
+  // control bit (a row bit, or none: -1) is set
+  int ftSign;
+  int nPl;
+  double plC[2];
+  int plCtrl[2];
+};
+
+struct RowProgram {
+  int logN;     // register length
+  int logM;     // row elements held by one CTA
+  int logRows;  // rows per CTA (cluster size 1 only)
+  int nOps;
+  int nDiag;
+  int logTwN;
+  int loadT;    // cluster rows: start transposed (1: from the natural layout, 2: from the blocked one)
+  int storeBlocked;  // cluster rows ending transposed: write the blocked layout
+  int rowMask;       // k_rowr: rows (columns) of the state less one, at most those of a CTA less one
+  int logS;          // k_rowr on a strided register: log2 of the amplitudes below it (0: rows)
+  const double2* tw;
+  double* rowSums;        // non-null: per-warp partial sums of |psi|^2 of every row's result
+  unsigned int* waitErr;  // set when a bounded wait on the cluster peers gives up
+  RowOp ops[kMaxRowOps];
+  RowDiag diag[kMaxRowDiags];
+};
+
+// ---------------------------------------------------------------- register-resident rows
+// Rows that fit one CTA (up to 2^13 complex128 / 2^14 complex64 points) run in
+// k_rowr: each thread keeps E = 16 (or 32) amplitudes of one row in registers
+// for the whole program -- elements t + TPR v (v < E) of its row, TPR = M / E
+// threads per row.  A Stockham stage of radix R gives thread t the butterflies
+// j = t + b TPR (b < E/R); their inputs j + u M/R are exactly the thread's E
+// elements (register b + (E/R) u), and the last stage's outputs land on the same
+// positions.  So the global load, the store and every diagonal run between
+// transforms work on registers in place; only the stages inside a transform
+// exchange data, through one padded shared-memory row.  Row length, radices and
+// strides are template constants, so every shared-memory address is a
+// per-thread base plus an immediate offset.
+
+// exp(i pi s (N-1)(2n-N+1)/(2N)) with the angle reduced exactly in integers, and
+// its ratio between n + d and n, exp(i pi s (N-1) d / N)
+__device__ __forceinline__ double2 ft_tw_at(long long n, long long N, int s) {
+  long long m = ((N - 1) * (2 * n - N + 1) * s) % (4 * N);
+  if (m < 0) m += 4 * N;
+  double sn, c;
+  sincospi((double)m / (double)(2 * N), &sn, &c);
+  return make_double2(c, sn);
+}
+__device__ __forceinline__ double2 ft_tw_ratio(long long d, long long N, int s) {
+  long long m = ((N - 1) * d * s) % (2 * N);
+  if (m < 0) m += 2 * N;
+  double sn, c;
+  sincospi((double)m / (double)N, &sn, &c);
+  return make_double2(c, sn);
+}
+
+template <typename C, int LOGM, int LOGE>
+__device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uint64_t rowBase, int t) {
+  constexpr int E = 1 << LOGE, TPR = 1 << (LOGM - LOGE);
+  const double2 rs = D.hasRowF ? eval_factor(D.rowF, rowBase) : make_double2(1.0, 0.0);
+  // running factor of element t + k TPR: rs times the linear phase, advanced by st per k
+  double2 f = rs, st = make_double2(1.0, 0.0);
+  const bool lin = D.nLin || D.nPl || D.ftSign;
+  if (lin) {
+    // bilinear terms with other registers and c x terms (controls off the row) are
+    // one linear phase a (m - regC) regDx along the row; the transform twiddle is
+    // exact at the first point and as a ratio per step
+    double a = 0.0;
+    for (int l = 0; l < D.nLin; ++l) {
+      const XXFactor& X = D.lin[l];
+      const int j = (int)((rowBase >> X.shift1) & (uint64_t)X.mask1);
+      double c = X.coeff * (((double)j - X.c1) * X.dx1);
+      if (X.ctrlShift >= 0 && ((rowBase >> X.ctrlShift) & 1ull)) c = -c;
+      a += c;
+    }
+    for (int k = 0; k < D.nPl; ++k)
+      a += (D.plCtrl[k] >= 0 && ((rowBase >> D.plCtrl[k]) & 1ull)) ? -D.plC[k] : D.plC[k];
+    a *= D.regDx;
+    double s0, c0;
+    sincos(a * ((double)t - D.regC), &s0, &c0);
+    sincos(a * (double)TPR, &st.y, &st.x);
+    f = dmul(rs, make_double2(c0, s0));
+    if (D.ftSign) {
+      f = dmul(f, ft_tw_at(t, 1ll << LOGM, D.ftSign));
+      st = dmul(st, ft_tw_ratio(TPR, 1ll << LOGM, D.ftSign));
+    }
+  }
+  if (D.tab) {
+    int seg = 0;
+    for (int c = 0; c < D.nCtrl; ++c) seg |= (int)((rowBase >> D.ctrlShift[c]) & 1ull) << c;
+    const double2* tp = D.tab + ((size_t)seg << LOGM) + t;
+#pragma unroll
+    for (int k0 = 0; k0 < E; k0 += 8) {
+      double2 w[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w[k] = __ldg(tp + (k0 + k) * TPR);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if (D.hasRowF || lin) w[k] = dmul(w[k], f);
+        if (lin) f = dmul(f, st);
+        v[k0 + k] = cmul(v[k0 + k], fromd<C>(w[k]));
+      }
+    }
+  } else if (lin) {
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+      v[k] = cmul(v[k], fromd<C>(f));
+      f = dmul(f, st);
+    }
+  } else if (D.hasRowF) {
+    const C c = fromd<C>(rs);
+#pragma unroll
+    for (int k = 0; k < E; ++k) v[k] = cmul(v[k], c);
+  }
+}
+
+// 256-thread CTAs run two per SM; 512- and 1024-thread CTAs one
+// Ask L2 to fetch [p, p + bytes) ahead of use: bulk prefetches of 16 KB, one per
+// lane of the first warp (bytes a multiple of 16 KB, at most 32 x 16 KB).
+__device__ __forceinline__ void l2_prefetch_tile(const void* p, uint32_t bytes) {
+  const uint32_t chunk = 16384;
+  const uint32_t i = threadIdx.x;
+  if (i < bytes / chunk) {
+    const char* a = static_cast<const char*>(p) + (size_t)i * chunk;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(chunk) : "memory");
+  }
+}
+
+// Tiles of one CTA per SM (more than 256 threads) run persistent: each CTA walks
+// tiles blockIdx.x, + gridDim.x, ... and asks L2 for its next tile before working
+// on the current one, so the next load finds its data on chip while this tile's
+// butterflies run.  Smaller tiles run two CTAs per SM, which already overlap one
+// CTA's loads with the other's work; they get one tile per CTA.
+//
+// With COL the "rows" are the columns of a strided register (P.logS amplitudes
+// below it): column c is inner index c mod S and outer index c / S, and element m
+// sits m S amplitudes after its first.  The CTA's 2^LOGR columns (at least two
+// within 512 threads) are adjacent inner indices interleaved lane by lane, so a
+// warp's load covers runs of 2^LOGR amplitudes; the rest of each sector is read
+// from L2 by the CTAs of the neighbouring columns.
+// The sum of |psi|^2 (FP64) over the E amplitudes of each of a group of W lanes
+// (W = 32, or the lanes of one row when a warp holds several), written by the
+// group's first lane.
+template <typename C, int E, int W>
+__device__ __forceinline__ void row_sum_part(const C (&v)[E], double* out) {
+  double a = 0.0;
+#pragma unroll
+  for (int k = 0; k < E; ++k) a += (double)v[k].x * (double)v[k].x + (double)v[k].y * (double)v[k].y;
+#pragma unroll
+  for (int o = W / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if ((threadIdx.x & (W - 1)) == 0) *out = a;
+}
+
+//
+// A state of fewer rows than a CTA holds (nRows < 2^LOGR, both powers of two) runs
+// as one tile whose surplus thread groups repeat its rows: they read the same
+// input and write the same values.
+template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
+__global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR) > 8 ? 1 : 2)
+    k_rowr(const C* __restrict__ in, C* __restrict__ out, uint64_t nTiles, const __grid_constant__ RowProgram P) {
+  constexpr int E = 1 << LOGE, M = 1 << LOGM, TPR = M >> LOGE, NT = TPR << LOGR, RS = rr_row_slots(LOGM, LOGE);
+  constexpr uint32_t TILE_BYTES = (uint32_t)sizeof(C) << (LOGM + LOGR);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C* sm = reinterpret_cast<C*>(smraw);
+  double2* lo = reinterpret_cast<double2*>(sm + (RS << LOGR));  // w_M^e, e < 64
+  double2* hi = lo + 64;                                         // w_M^(64 h), h < M / 64
+  const int tid = threadIdx.x;
+  // column form: the CTA's 2^LOGR adjacent columns interleave lane by lane, so a
+  // warp's load covers 32 / 2^LOGR points of every column in runs of 2^LOGR
+  int row = COL ? (tid & ((1 << LOGR) - 1)) : tid >> (LOGM - LOGE);
+  const int t = COL ? (tid >> LOGR) : tid & (TPR - 1);
+  C* smrow = sm + row * RS;
+  const int logS = COL ? P.logS : 0;
+  if constexpr (LOGM < 8) row &= P.rowMask;  // (longer rows: LOGR = 0 where rows are few)
+
+  const int scM = P.logTwN - LOGM;
+  for (int i = tid; i < rr_tw_slots(LOGM); i += NT) {
+    const int e = i < 64 ? i : (i - 64) << 6;
+    if (e < M) lo[i] = __ldg(P.tw + ((size_t)e << scM));  // lo and hi are one array
+  }
+  __syncthreads();
+  // No barrier between tiles: after a transform's last exchange (which ends in a
+  // barrier) a thread touches shared memory again only in the next tile's first
+  // exchange, and every thread has left the old tile's exchanges by then.
+  for (uint64_t tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
+    uint64_t rowBase;
+    if constexpr (COL) {
+      const uint64_t c = (tile << LOGR) + (uint64_t)row;
+      rowBase = (c & ((1ull << logS) - 1)) + ((c >> logS) << (LOGM + logS));
+    } else {
+      if (NT > 256 && tile + gridDim.x < nTiles)
+        l2_prefetch_tile(in + ((tile + gridDim.x) << (LOGM + LOGR)), TILE_BYTES);
+      rowBase = (tile << (LOGM + LOGR)) + ((uint64_t)row << LOGM);
+    }
+    C v[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) v[k] = in[rowBase + ((uint64_t)(t + k * TPR) << logS)];
+    for (int o = 0; o < P.nOps; ++o) {
+      const RowOp& op = P.ops[o];
+      if (op.kind == kRowDiag) rr_diag<C, LOGM, LOGE>(v, P.diag[op.diag], rowBase, t);
+      else if (op.dir > 0) rr_stages<C, 1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
+      else rr_stages<C, -1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
+    }
+    if constexpr (!COL) {
+      // the row's |psi|^2 in TPR / 32 partials (one when a warp holds several rows)
+      constexpr int W = TPR < 32 ? TPR : 32, PARTS = TPR < 32 ? 1 : TPR / 32;
+      if (P.rowSums) row_sum_part<C, E, W>(v, P.rowSums + (rowBase >> LOGM) * PARTS + t / 32);
+    }
+#pragma unroll
+    for (int k = 0; k < E; ++k) out[rowBase + ((uint64_t)(t + k * TPR) << logS)] = v[k];
+  }
+}
+
+// largest row k_rowr takes (one CTA: 2^13 complex128 / 2^14 complex64 points)
+inline int rowr_max_log(int precision) { return precision == kC128 ? 13 : 14; }
+
+// complex64 rows of 2^13 and 2^14 points keep 32 amplitudes per thread (256 / 512
+// threads); everything else 16, and rows shorter than 2^8 points 8
+template <typename C, int LOGM>
+struct RrShape {
+  static constexpr int LOGE = LOGM < 8 ? 3 : (sizeof(C) == sizeof(float2) && LOGM >= 13) ? 5 : 4;
+  static constexpr int LOGR = LOGM < 8 ? 10 - LOGM : LOGM - LOGE < 8 ? 8 - (LOGM - LOGE) : 0;
+};
+
+// Rows of 2^8 .. 2^12 points of a state below 2^kRowrSmallLog amplitudes run one row
+// per CTA at 8 amplitudes a thread (radix-8 stages): such a state does not fill the
+// chip, so a program takes the latency of one CTA's chain, and twice the warps on a
+// row shorten it.
+constexpr int kRowrSmallLog = 19;
+inline bool rowr_small(Context* ctx) { return ctx->totalQbt < kRowrSmallLog; }
+
+template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
+static cudaError_t launch_rowr_s(Context* ctx, const RowProgram& P) {
+  constexpr int NT = 1 << (LOGM - LOGE + LOGR);
+  const size_t smem = (size_t)rr_row_slots(LOGM, LOGE) * (1 << LOGR) * sizeof(C) + rr_tw_slots(LOGM) * sizeof(double2);
+  auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL>;
+  static int resident = 0;  // CTAs per SM of this instantiation, asked once
+  cudaError_t e = cudaSuccess;
+  if (!resident) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, NT, smem);
+    if (e != cudaSuccess || resident < 1) return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+  }
+  uint64_t nTiles = ctx->size() >> (LOGM + LOGR);
+  if (nTiles < 1) nTiles = 1;
+  uint64_t grid = NT > 256 ? (uint64_t)ctx->numSMs * resident : nTiles;
+  if (grid > nTiles) grid = nTiles;
+  kern<<<(unsigned)grid, NT, smem, ctx->stream>>>((const C*)ctx->state(), (C*)ctx->other(), nTiles, P);
+  return cudaGetLastError();
+}
+
+template <typename C, int LOGM, bool COL>
+static cudaError_t launch_rowr_t(Context* ctx, const RowProgram& P) {
+  constexpr int LOGE = RrShape<C, LOGM>::LOGE, LOGR0 = RrShape<C, LOGM>::LOGR;
+  // column form: at least two columns a CTA while it stays within 512 threads
+  constexpr int LOGR = (COL && LOGR0 == 0 && (LOGM - LOGE) < 9) ? 1 : LOGR0;
+  if constexpr (LOGM >= 8 && LOGM <= 12) {
+    if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, 0, 3, COL>(ctx, P);
+  }
+  return launch_rowr_s<C, LOGM, LOGR, LOGE, COL>(ctx, P);
+}
+
+template <typename C, bool COL>
+cudaError_t launch_rowr(Context* ctx, const RowProgram& P, int q) {
+  switch (q) {
+    case 4: return launch_rowr_t<C, 4, COL>(ctx, P);
+    case 5: return launch_rowr_t<C, 5, COL>(ctx, P);
+    case 6: return launch_rowr_t<C, 6, COL>(ctx, P);
+    case 7: return launch_rowr_t<C, 7, COL>(ctx, P);
+    case 8: return launch_rowr_t<C, 8, COL>(ctx, P);
+    case 9: return launch_rowr_t<C, 9, COL>(ctx, P);
+    case 10: return launch_rowr_t<C, 10, COL>(ctx, P);
+    case 11: return launch_rowr_t<C, 11, COL>(ctx, P);
+    case 12: return launch_rowr_t<C, 12, COL>(ctx, P);
+    case 13: return launch_rowr_t<C, 13, COL>(ctx, P);
+    default:
+      if constexpr (sizeof(C) == sizeof(float2)) return launch_rowr_t<C, 14, COL>(ctx, P);
+      return cudaErrorInvalidValue;
+  }
+}
+
+extern template cudaError_t launch_rowr<double2, false>(Context*, const RowProgram&, int);
+extern template cudaError_t launch_rowr<double2, true>(Context*, const RowProgram&, int);
+extern template cudaError_t launch_rowr<float2, false>(Context*, const RowProgram&, int);
+extern template cudaError_t launch_rowr<float2, true>(Context*, const RowProgram&, int);
+
+}  // namespace cvdv
