@@ -338,45 +338,11 @@ CVDVContext* cvdvCreate(int numReg, int* numQubits) {
 
 }  // extern "C"
 
-namespace cvdv {
-
-Context* factor_context(Context* ctx, int r) {
-  if ((int)ctx->factorCtx.size() < ctx->numReg) ctx->factorCtx.resize(ctx->numReg, nullptr);
-  if (ctx->factorCtx[r]) return ctx->factorCtx[r];
-  int q = ctx->q[r];
-  CVDVContext* h = cvdvCreateEx(1, &q, kC128);
-  if (!h) {
-    set_error(ctx, kErrAlloc, "register %d context: out of host memory", r);
-    return nullptr;
-  }
-  Context* f = h;
-  if (f->numReg != 1) {
-    set_error(ctx, f->lastErr != kOk ? f->lastErr : kErrAlloc, "register %d context: %s", r,
-              f->lastMsg.c_str());
-    cvdvDestroy(h);
-    return nullptr;
-  }
-  cudaStreamSynchronize(f->stream);  // its twiddle table
-  cudaStreamDestroy(f->stream);
-  f->stream = ctx->stream;  // stream order keeps its kernels between this context's
-  cudaFreeHost(f->waitErr);
-  f->waitErr = ctx->waitErr;  // its kernels' failed waits show at this context's syncs
-  ctx->factorCtx[r] = f;
-  return f;
-}
-
-}  // namespace cvdv
-
 extern "C" {
 
 static void release(Context* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (Context* f : c->factorCtx)
-    if (f) {
-      f->stream = nullptr;  // this context's stream and wait flag, released with it
-      f->waitErr = nullptr;
-      cvdvDestroy(static_cast<CVDVContext*>(f));
-    }
+  for (Context* f : c->factorCtx) delete f;  // (they own no device memory)
   c->factorCtx.clear();
   if (c->factors) cudaFree(c->factors);
   c->factors = nullptr;

@@ -31,9 +31,9 @@ void set_error(Context* ctx, int code, const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(buf, sizeof(buf), fmt, ap);
   va_end(ap);
-  if (ctx) {
-    ctx->lastErr = code;
-    ctx->lastMsg = buf;
+  for (Context* c = ctx; c; c = c->parent) {  // (a register's context reports to its parent)
+    c->lastErr = code;
+    c->lastMsg = buf;
   }
   std::lock_guard<std::mutex> lk(g_errMu);
   g_lastErr = code;
@@ -118,6 +118,7 @@ bool stream_sync(Context* ctx, const char* what) {
 // invalidates pointers handed out since the last reset: when the arena is full
 // a new block is chained; the next reset merges all blocks into one.
 void arena_reset(Context* ctx) {
+  if (ctx->parent) return;  // shared with the parent, which resets it
   if (!ctx->arenaExtra.empty()) {
     size_t total = ctx->arenaCap;
     for (auto& b : ctx->arenaExtra) total += b.cap;
@@ -134,6 +135,7 @@ void arena_reset(Context* ctx) {
 }
 
 void* arena_alloc(Context* ctx, size_t bytes) {
+  if (ctx->parent) return arena_alloc(ctx->parent, bytes);
   bytes = (bytes + 255) & ~(size_t)255;
   if (ctx->arena && ctx->arenaTop + bytes <= ctx->arenaCap) {
     void* p = ctx->arena + ctx->arenaTop;
@@ -566,6 +568,28 @@ static Stage factor_stage(Context* ctx, Stage s, int r) {
   return s;
 }
 
+// The complex128 context of the one register r: it borrows this context's stream,
+// twiddles, arena and wait flag, and is given its buffers for each flush.
+static Context* factor_context(Context* ctx, int r) {
+  if ((int)ctx->factorCtx.size() < ctx->numReg) ctx->factorCtx.resize(ctx->numReg, nullptr);
+  if (ctx->factorCtx[r]) return ctx->factorCtx[r];
+  Context* f = new Context();
+  f->parent = ctx;
+  f->numReg = 1;
+  f->totalQbt = ctx->q[r];
+  f->q = {ctx->q[r]};
+  f->flw = {0};
+  f->dx = {ctx->dx[r]};
+  f->stream = ctx->stream;
+  f->numSMs = ctx->numSMs;
+  f->device = ctx->device;
+  f->twiddle = ctx->twiddle;
+  f->twN = ctx->twN;
+  f->waitErr = ctx->waitErr;
+  ctx->factorCtx[r] = f;
+  return f;
+}
+
 static bool run_factors(Context* ctx, std::vector<Stage>& stages, std::vector<const double2*>& arrs) {
   const int R = ctx->numReg;
   std::vector<std::vector<Stage>> per(R);
@@ -597,23 +621,27 @@ static bool run_factors(Context* ctx, std::vector<Stage>& stages, std::vector<co
   for (int r = 0; r < R; ++r) {
     if (per[r].empty()) continue;
     Context* f = factor_context(ctx, r);
-    if (!f) return false;
     const size_t bytes = ((size_t)1 << ctx->q[r]) * sizeof(double2);
-    bool ok = ensure_state(f) &&
-              cuda_ok(f, cudaMemcpyAsync(f->state(), arrs[r], bytes, cudaMemcpyDeviceToDevice, f->stream),
-                      "register array in");
+    // its programs read the register array in place and alternate with a buffer of
+    // the arena; the product is formed from whichever holds the result
+    f->buf[0] = const_cast<double2*>(arrs[r]);
+    f->buf[1] = arena_alloc(ctx, bytes);
+    f->cur = 0;
+    bool ok = f->buf[1] != nullptr;
     if (ok) {
+      f->allocElems = (size_t)1 << ctx->q[r];
       f->initialized = true;
       f->cancelFt = ctx->cancelFt;
       f->fuseSeq = ctx->fuseSeq;
       f->colFft = ctx->colFft;
       f->colProg = ctx->colProg;
+      f->plan = ctx->plan;
       // (transform pairs were cancelled when they were queued on this context, so
       // cvdvCancelledTransforms already counts them)
       f->pending = std::move(per[r]);
-      ok = flush(f) && cuda_ok(f, cudaMemcpyAsync((void*)arrs[r], f->state(), bytes,
-                                                   cudaMemcpyDeviceToDevice, f->stream),
-                               "register array out");
+      ok = flush(f);
+      f->plan = nullptr;
+      arrs[r] = (const double2*)f->state();
     }
     if (!ok) {
       set_error(ctx, f->lastErr != kOk ? f->lastErr : kErrCuda, "register %d before the product: %s", r,
@@ -659,10 +687,12 @@ static bool blocked_array(Context* ctx, std::vector<const double2*>& arrs, int b
   const size_t M = ((size_t)1 << ctx->q[blockedReg]) / nC;
   double2* t = (double2*)arena_alloc(ctx, nC * M * sizeof(double2));
   bool ok = t != nullptr;
+  const double2* src = arrs[blockedReg];
   for (int h = 0; ok && h < nC; ++h)
-    ok = cuda_ok(ctx, cudaMemcpy2DAsync(t + h * M, sizeof(double2), arrs[blockedReg] + h, nC * sizeof(double2),
-                                        sizeof(double2), M, cudaMemcpyDeviceToDevice, ctx->stream),
-                 "blocked register array");
+    ok = enqueue(ctx, -1, "blocked register array", [=] {
+      return cudaMemcpy2DAsync(t + h * M, sizeof(double2), src + h, nC * sizeof(double2), sizeof(double2), M,
+                               cudaMemcpyDeviceToDevice, ctx->stream);
+    });
   if (ok) arrs[blockedReg] = t;
   return ok;
 }
@@ -694,13 +724,9 @@ static bool launch_product(Context* ctx, std::vector<const double2*>& arrs, int 
   return ok;
 }
 
-bool flush(Context* ctx) {
-  if (ctx->pending.empty() && !ctx->productPending) return true;
-  if (!ctx->initialized) {
-    set_error(ctx, kErrNotInitialized, "gates queued before the state was initialised");
-    ctx->pending.clear();
-    return false;
-  }
+// Plans the queue: every kernel's parameters are fixed and its launch kept in
+// ctx->plan, with the tables they read.
+static bool plan_flush(Context* ctx) {
   arena_reset(ctx);
   std::vector<Stage> stages;
   stages.swap(ctx->pending);
@@ -885,6 +911,30 @@ bool flush(Context* ctx) {
     if (!run_leftover(ctx, lpost)) return false;
   }
   return true;
+}
+
+bool flush(Context* ctx) {
+  if (ctx->pending.empty() && !ctx->productPending) return true;
+  if (!ctx->initialized) {
+    set_error(ctx, kErrNotInitialized, "gates queued before the state was initialised");
+    ctx->pending.clear();
+    return false;
+  }
+  if (ctx->plan) return plan_flush(ctx);  // a register's context: part of its parent's flush
+  FlushPlan plan;
+  const bool product = ctx->productPending;
+  const int cur = ctx->cur;
+  ctx->plan = &plan;
+  bool ok = plan_flush(ctx);
+  ctx->plan = nullptr;
+  if (!ok) {  // nothing was launched: the state is still where it was
+    ctx->cur = cur;
+    return false;
+  }
+  ok = launch_tables(ctx, plan.tables);
+  for (size_t k = 0; ok && k < plan.launches.size(); ++k) ok = plan.launches[k]();
+  if (!ok && product) ctx->initialized = false;  // the product state was not formed
+  return ok;
 }
 
 }  // namespace cvdv

@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -216,6 +217,31 @@ struct TimingRec {
   int kind;
 };
 
+struct Context;
+
+// A factor table to build: entry [seg][j] of register length 2^logN, seg over the
+// 2^ctrl values of the external control bits (launch_build_table_ext).
+struct TableTerm {
+  signed char kind, power, sign, bit;  // kTermPoly / kTermFtTw / kTermBit; bit inside the register
+  signed char ctrlMode, ctrlLocal;     // 0 none, 1 external control (segment bit), 2 bit inside the register
+  double coeff;
+  double2 g0, g1;
+};
+struct TableJob {
+  double2* out;
+  double dx;
+  int logN, ctrl, permLogC;
+  std::vector<TableTerm> terms;
+};
+
+// What a flush will launch.  Planning allocates tables and fixes every kernel's
+// parameters (the ping-pong buffers alternate as the launches are planned); then
+// all tables are built by one launch and the planned launches run in order.
+struct FlushPlan {
+  std::vector<TableJob> tables;
+  std::vector<std::function<bool()>> launches;
+};
+
 struct Context {
   // per-launch timing (off by default): event pairs around every launch
   bool timing = false;
@@ -274,9 +300,11 @@ struct Context {
   // couples it to another register, have run on that register's array.
   bool deferProduct = true;
   bool productPending = false;
+  FlushPlan* plan = nullptr;        // inside a flush, while it is planned
+  Context* parent = nullptr;        // of a register's context (factorCtx): shares its arena, stream and twiddles
   double2* factors = nullptr;       // the register arrays, concatenated (complex128)
   size_t factorsCap = 0;            // in elements
-  std::vector<Context*> factorCtx;  // one-register contexts for them, made on first use
+  std::vector<Context*> factorCtx;  // one-register contexts for them, made on first use (no memory of their own)
   // Inside one flush, between a forward and an inverse 2^14-point transform of
   // the last register run by a cluster row kernel of C = 2^permLogC CTAs, that
   // register may be stored "blocked": position r M + k2 (M = N / C) holds logical
@@ -321,6 +349,10 @@ struct LaunchScope {
   ~LaunchScope() { launch_end(c); }
 };
 void harvest_timing(Context* ctx);
+// Runs f() -> cudaError_t (one kernel launch of the given kind, or a copy for kind
+// < 0), or, while a flush is being planned, keeps it for the flush to run.
+template <typename F>
+bool enqueue(Context* ctx, int kind, const char* what, F f);
 extern std::atomic<unsigned long long> g_launches;
 
 void set_error(Context* ctx, int code, const char* fmt, ...);
@@ -332,8 +364,6 @@ void arena_reset(Context* ctx);
 void* big_scratch(Context* ctx, size_t bytes);   // persistent, grown on demand
 double* host_scratch(Context* ctx, size_t count);
 bool ensure_state(Context* ctx);                  // allocate both buffers
-// complex128 context of the one register r of ctx, on ctx's stream (api_gates.cu)
-Context* factor_context(Context* ctx, int r);
 bool flush(Context* ctx);                         // run pending stages
 // scratch address of cvdvMeasureMultipleNoAlloc on device dev (current), with its
 // device code loaded; nullptr on failure (recorded as the last error if report)
@@ -350,6 +380,7 @@ bool launch_build_table(Context* ctx, int r, bool ctrl, const Term* terms, int n
 // transposed layout: position rank * (N >> permLogC) + m holds index rank + (m << permLogC)
 bool launch_build_table_ext(Context* ctx, int r, int nExt, const int* extBits, const Term* terms,
                             int nTerms, double2* out, int permLogC = 0);
+bool launch_tables(Context* ctx, const std::vector<TableJob>& jobs);  // one launch for all (kernels_elementwise.cu)
 bool launch_diag(Context* ctx, const FactorList& F);
 bool launch_pair(Context* ctx, int bit, const double2 m[4], const FactorList& pre,
                  const FactorList& post);
@@ -410,5 +441,22 @@ bool launch_fft_into(Context* ctx, int reg, int dir, const FactorList& pre, void
 int global_error(char* msg, int len);
 bool make_twiddle(Context* ctx, int logN);
 bool launch_convert_c128_to_c64(Context* ctx, const double2* src, float2* dst, uint64_t n);
+
+template <typename F>
+bool enqueue(Context* ctx, int kind, const char* what, F f) {
+  auto go = [ctx, kind, what, f]() -> bool {
+    cudaError_t e;
+    if (kind < 0) {
+      e = f();
+    } else {
+      LaunchScope _ls(ctx, kind);
+      e = f();
+    }
+    return cuda_ok(ctx, e, what);
+  };
+  if (!ctx->plan) return go();
+  ctx->plan->launches.emplace_back(std::move(go));
+  return true;
+}
 
 }  // namespace cvdv

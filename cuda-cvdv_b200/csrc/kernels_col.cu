@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kColThreads, CE >= 4 ? 2 : (sizeof(C) == sizeo
 }
 
 template <typename C, int LOGL, int KIND, int D1, int D2>
-static cudaError_t col_launch_t(Context* ctx, const ColPass& P) {
+static cudaError_t col_launch_t(Context* ctx, const void* in, void* out, const ColPass& P) {
   using S = ColShape<LOGL, ColCE<C>::v>;
   const int nHiN = P.logN >= 6 ? 1 << (P.logN - 6) : 1;
   const size_t smem = (size_t)S::W * S::RS * sizeof(C) + (64 + S::HI + 64 + nHiN) * sizeof(double2);
@@ -188,37 +188,39 @@ static cudaError_t col_launch_t(Context* ctx, const ColPass& P) {
   auto kern = k_colr<C, LOGL, KIND, D1, D2>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<grid, kColThreads, smem, ctx->stream>>>((const C*)ctx->state(), (C*)ctx->other(), P);
+  kern<<<grid, kColThreads, smem, ctx->stream>>>((const C*)in, (C*)out, P);
   return cudaGetLastError();
 }
 
 template <typename C, int LOGL>
-static cudaError_t col_launch(Context* ctx, const ColPass& P, int kind, int d1, int d2) {
+static cudaError_t col_launch(Context* ctx, const void* in, void* out, const ColPass& P, int kind, int d1, int d2) {
   switch (kind) {
     case kColFirst:
-      return d1 > 0 ? col_launch_t<C, LOGL, kColFirst, 1, 0>(ctx, P) : col_launch_t<C, LOGL, kColFirst, -1, 0>(ctx, P);
+      return d1 > 0 ? col_launch_t<C, LOGL, kColFirst, 1, 0>(ctx, in, out, P) : col_launch_t<C, LOGL, kColFirst, -1, 0>(ctx, in, out, P);
     case kColLast:
-      return d1 > 0 ? col_launch_t<C, LOGL, kColLast, 1, 0>(ctx, P) : col_launch_t<C, LOGL, kColLast, -1, 0>(ctx, P);
+      return d1 > 0 ? col_launch_t<C, LOGL, kColLast, 1, 0>(ctx, in, out, P) : col_launch_t<C, LOGL, kColLast, -1, 0>(ctx, in, out, P);
     case kColMiddle:
-      if (d1 > 0) return d2 > 0 ? col_launch_t<C, LOGL, kColMiddle, 1, 1>(ctx, P) : col_launch_t<C, LOGL, kColMiddle, 1, -1>(ctx, P);
-      return d2 > 0 ? col_launch_t<C, LOGL, kColMiddle, -1, 1>(ctx, P) : col_launch_t<C, LOGL, kColMiddle, -1, -1>(ctx, P);
+      if (d1 > 0) return d2 > 0 ? col_launch_t<C, LOGL, kColMiddle, 1, 1>(ctx, in, out, P) : col_launch_t<C, LOGL, kColMiddle, 1, -1>(ctx, in, out, P);
+      return d2 > 0 ? col_launch_t<C, LOGL, kColMiddle, -1, 1>(ctx, in, out, P) : col_launch_t<C, LOGL, kColMiddle, -1, -1>(ctx, in, out, P);
     default:
-      return col_launch_t<C, LOGL, kColWhole, 1, 0>(ctx, P);
+      return col_launch_t<C, LOGL, kColWhole, 1, 0>(ctx, in, out, P);
   }
 }
 
 template <typename C>
-static cudaError_t col_dispatch(Context* ctx, int logL, const ColPass& P, int kind, int d1, int d2) {
+static cudaError_t col_dispatch(Context* ctx, const void* in, void* out, int logL, const ColPass& P, int kind, int d1,
+                                int d2) {
   switch (logL) {
-    case 4: return col_launch<C, 4>(ctx, P, kind, d1, d2);
-    case 5: return col_launch<C, 5>(ctx, P, kind, d1, d2);
-    case 6: return col_launch<C, 6>(ctx, P, kind, d1, d2);
-    case 7: return col_launch<C, 7>(ctx, P, kind, d1, d2);
-    default: return col_launch<C, 8>(ctx, P, kind, d1, d2);
+    case 4: return col_launch<C, 4>(ctx, in, out, P, kind, d1, d2);
+    case 5: return col_launch<C, 5>(ctx, in, out, P, kind, d1, d2);
+    case 6: return col_launch<C, 6>(ctx, in, out, P, kind, d1, d2);
+    case 7: return col_launch<C, 7>(ctx, in, out, P, kind, d1, d2);
+    default: return col_launch<C, 8>(ctx, in, out, P, kind, d1, d2);
   }
 }
 
-cudaError_t launch_col_tc(Context* ctx, const ColPass& P, int logL, int kind, int d1, int d2);  // kernels_tc.cu
+cudaError_t launch_col_tc(Context* ctx, const void* in, void* out, const ColPass& P, int logL, int kind, int d1,
+                          int d2);  // kernels_tc.cu
 
 // Whether the column kernel takes transforms of register `reg`: 2^4..2^16 points
 // and at least 8 amplitudes below it (runs of 8 contiguous columns for the loads
@@ -305,18 +307,16 @@ static bool run_col_chain(Context* ctx, int reg, const std::vector<int>& dirs,
   // complex64 passes of 64 or 128 points run as DFT-matrix products on the tensor cores
   const bool tc = tc_col_ok(ctx, reg);
   auto go = [&](const ColPass& P, int logL, int kind, int d1, int d2) -> bool {
-    cudaError_t e;
-    if (tc && kind != kColWhole && (logL == 6 || logL == 7) && P.logA >= 7 - logL) {
-      LaunchScope _ls(ctx, kKColTc);
-      e = launch_col_tc(ctx, P, logL, kind, d1, d2);
-    } else {
-      LaunchScope _ls(ctx, kKCol);
-      e = ctx->precision == kC128 ? col_dispatch<double2>(ctx, logL, P, kind, d1, d2)
-                                  : col_dispatch<float2>(ctx, logL, P, kind, d1, d2);
-    }
-    if (!cuda_ok(ctx, e, "column transform launch")) return false;
-    ctx->cur ^= 1;
-    return true;
+    const bool useTc = tc && kind != kColWhole && (logL == 6 || logL == 7) && P.logA >= 7 - logL;
+    const void* in = ctx->state();
+    void* out = ctx->other();
+    const bool ok = enqueue(ctx, useTc ? kKColTc : kKCol, "column transform launch", [=] {
+      if (useTc) return launch_col_tc(ctx, in, out, P, logL, kind, d1, d2);
+      return ctx->precision == kC128 ? col_dispatch<double2>(ctx, in, out, logL, P, kind, d1, d2)
+                                     : col_dispatch<float2>(ctx, in, out, logL, P, kind, d1, d2);
+    });
+    if (ok) ctx->cur ^= 1;
+    return ok;
   };
   auto too_long = [&]() {
     set_error(ctx, kErrUnsupported, "column transform run too long");

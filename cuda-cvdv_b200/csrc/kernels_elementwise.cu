@@ -10,25 +10,19 @@
 namespace cvdv {
 
 // ----------------------------------------------------------------- tables
-struct TTerm {
-  int kind;        // kTermPoly / kTermFtTw / kTermBit
-  int power;
-  int sign;
-  int bit;         // kTermBit: bit inside the register
-  int ctrlMode;    // 0 none, 1 external control (table half), 2 control bit inside the register
-  int ctrlLocal;   // ctrlMode 2: bit inside the register
-  double coeff;
-  double2 g0, g1;
-};
-
-struct TableJob {
-  int N;
-  int ctrl;        // number of external control bits: the table has 2^ctrl segments
-  int permLogC;    // > 0: entries stored permuted (see launch_build_table_ext)
-  int permLogM;
+// Tables of one launch, by value: J tables with T terms between them.  Each table
+// gets a run of consecutive blocks from block0 on.
+struct TableHead {
+  double2* out;
   double dx;
-  int nTerms;
-  TTerm t[kMaxTermsPerTable];
+  int logN, ctrl, permLogC;
+  int nTerms, term0, block0;
+};
+template <int J, int T>
+struct TableBatch {
+  int nJobs;
+  TableHead job[J];
+  TableTerm term[T];
 };
 
 // Table entry (b, j) = prod over terms.  Polynomial terms are summed into one
@@ -37,93 +31,148 @@ struct TableJob {
 // as kernelPhaseX/X2/X3, src/cuda/kernels/gates.cuh:5-16,184-209); the FT
 // twiddle is generated exactly from the integer (N-1)(2j-N+1) mod 4N so its
 // argument carries no rounding however large N is.
-__global__ void k_build_table(TableJob job, double2* out) {
-  int total = job.N << job.ctrl;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    int j = e % job.N;
-    int b = e / job.N;
-    if (job.permLogC) j = ((j & ((1 << job.permLogM) - 1)) << job.permLogC) + (j >> job.permLogM);
-    double x = ((double)j - (double)(job.N - 1) * 0.5) * job.dx;
-    double ph = 0.0;
-    bool anyPoly = false;
-    double2 f = make_double2(1.0, 0.0);
-    for (int t = 0; t < job.nTerms; ++t) {
-      const TTerm& T = job.t[t];
-      if (T.kind == kTermPoly) {
-        double v;
-        if (T.power == 1) v = T.coeff * x;
-        else if (T.power == 2) v = T.coeff * x * x;
-        else v = T.coeff * x * x * x;
-        bool neg = (T.ctrlMode == 1 && ((b >> T.ctrlLocal) & 1)) ||
-                   (T.ctrlMode == 2 && ((j >> T.ctrlLocal) & 1));
-        ph += neg ? -v : v;
-        anyPoly = true;
-      } else if (T.kind == kTermFtTw) {
-        long long N = job.N;
-        long long m = (N - 1) * (2LL * j - N + 1);
-        long long M4 = 4 * N;
-        m %= M4;
-        if (m < 0) m += M4;
-        double s, c;
-        sincospi((double)(T.sign) * (double)m / (double)(2 * N), &s, &c);
-        f = dmul(f, make_double2(c, s));
-      } else if (T.kind == kTermBit) {
-        f = dmul(f, ((j >> T.bit) & 1) ? T.g1 : T.g0);
-      }
-    }
-    if (anyPoly) {
-      double s, c;
-      sincos(ph, &s, &c);
-      f = dmul(make_double2(c, s), f);
-    }
-    out[e] = f;
+//
+// All tables of a flush are built by one launch: a table is 2^8 .. 2^15 entries, a
+// launch of its own took about 3 us however short, and a circuit has several per
+// mode gate (63 tables of a 60-gate circuit: 198 us in 63 launches).
+constexpr int kTableThreads = 256;
+template <int J, int T>
+__global__ void __launch_bounds__(kTableThreads) k_build_tables(const __grid_constant__ TableBatch<J, T> B) {
+  int lo = 0, hi = B.nJobs;  // the table whose run of blocks holds this block
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (B.job[mid].block0 <= (int)blockIdx.x) lo = mid;
+    else hi = mid;
   }
+  const TableHead& H = B.job[lo];
+  const int e = ((int)blockIdx.x - H.block0) * kTableThreads + (int)threadIdx.x;
+  const int N = 1 << H.logN;
+  if (e >= N << H.ctrl) return;
+  int j = e & (N - 1);
+  const int b = e >> H.logN;
+  if (H.permLogC) {
+    const int logM = H.logN - H.permLogC;
+    j = ((j & ((1 << logM) - 1)) << H.permLogC) + (j >> logM);
+  }
+  const double x = ((double)j - (double)(N - 1) * 0.5) * H.dx;
+  double ph = 0.0;
+  bool anyPoly = false;
+  double2 f = make_double2(1.0, 0.0);
+  for (int t = H.term0; t < H.term0 + H.nTerms; ++t) {
+    const TableTerm& D = B.term[t];
+    if (D.kind == kTermPoly) {
+      double v;
+      if (D.power == 1) v = D.coeff * x;
+      else if (D.power == 2) v = D.coeff * x * x;
+      else v = D.coeff * x * x * x;
+      const bool neg = (D.ctrlMode == 1 && ((b >> D.ctrlLocal) & 1)) || (D.ctrlMode == 2 && ((j >> D.ctrlLocal) & 1));
+      ph += neg ? -v : v;
+      anyPoly = true;
+    } else if (D.kind == kTermFtTw) {
+      const long long n = N;
+      const long long m = ((n - 1) * (2LL * j - n + 1)) & (4 * n - 1);  // mod 4N, N a power of two
+      double s, c;
+      sincospi((double)(D.sign) * (double)m / (double)(2 * n), &s, &c);
+      f = dmul(f, make_double2(c, s));
+    } else if (D.kind == kTermBit) {
+      f = dmul(f, ((j >> D.bit) & 1) ? D.g1 : D.g0);
+    }
+  }
+  if (anyPoly) {
+    double s, c;
+    sincos(ph, &s, &c);
+    f = dmul(make_double2(c, s), f);
+  }
+  H.out[e] = f;
+}
+
+// Launch sizes: parameters of up to 4 KB for a few tables, and close to the 32764
+// bytes a kernel may take for many; longer lists go in several launches.
+template <int J, int T>
+static bool launch_table_batch(Context* ctx, const std::vector<TableJob>& jobs, size_t first, size_t count) {
+  static_assert(sizeof(TableBatch<J, T>) <= 32764, "kernel parameters");
+  TableBatch<J, T> B;
+  B.nJobs = (int)count;
+  int nt = 0, blocks = 0;
+  for (size_t k = 0; k < count; ++k) {
+    const TableJob& D = jobs[first + k];
+    TableHead& H = B.job[k];
+    H.out = D.out;
+    H.dx = D.dx;
+    H.logN = D.logN;
+    H.ctrl = D.ctrl;
+    H.permLogC = D.permLogC;
+    H.nTerms = (int)D.terms.size();
+    H.term0 = nt;
+    H.block0 = blocks;
+    for (const TableTerm& t : D.terms) B.term[nt++] = t;
+    blocks += (int)((((size_t)1 << (D.logN + D.ctrl)) + kTableThreads - 1) / kTableThreads);
+  }
+  {
+    LaunchScope _ls(ctx, kKTable);
+    k_build_tables<J, T><<<blocks, kTableThreads, 0, ctx->stream>>>(B);
+  }
+  return cuda_ok(ctx, cudaGetLastError(), "build_table launch");
+}
+
+bool launch_tables(Context* ctx, const std::vector<TableJob>& jobs) {
+  constexpr int JS = 24, TS = 60, JL = 160, TL = 500;
+  size_t i = 0;
+  while (i < jobs.size()) {
+    size_t n = 0, terms = 0, blocks = 0;
+    for (; i + n < jobs.size() && n < (size_t)JL; ++n) {
+      const size_t t = jobs[i + n].terms.size(), b = ((size_t)1 << (jobs[i + n].logN + jobs[i + n].ctrl)) / kTableThreads + 1;
+      if (n > 0 && (terms + t > (size_t)TL || blocks + b > (size_t)1 << 30)) break;
+      terms += t;
+      blocks += b;
+    }
+    if (!(n <= (size_t)JS && terms <= (size_t)TS ? launch_table_batch<JS, TS>(ctx, jobs, i, n)
+                                                 : launch_table_batch<JL, TL>(ctx, jobs, i, n)))
+      return false;
+    i += n;
+  }
+  return true;
 }
 
 // Table over register r with nExt external control bits (extBits, flat-index
 // positions outside r): entry [seg][j], seg bit c = value of extBits[c].
 bool launch_build_table_ext(Context* ctx, int r, int nExt, const int* extBits, const Term* terms,
                             int nTerms, double2* out, int permLogC) {
-  TableJob job{};
-  job.N = 1 << ctx->q[r];
+  TableJob job;
+  job.out = out;
+  job.dx = ctx->dx[r];
+  job.logN = ctx->q[r];
   job.ctrl = nExt;
   job.permLogC = permLogC;
-  job.permLogM = ctx->q[r] - permLogC;
-  job.dx = ctx->dx[r];
-  job.nTerms = nTerms;
-  int lo = ctx->flw[r], hi = ctx->flw[r] + ctx->q[r];
+  job.terms.reserve(nTerms);
+  const int lo = ctx->flw[r], hi = ctx->flw[r] + ctx->q[r];
   for (int t = 0; t < nTerms; ++t) {
     const Term& T = terms[t];
-    TTerm& D = job.t[t];
-    D.kind = T.kind;
-    D.power = T.power;
-    D.sign = T.sign;
-    D.bit = T.bit;
+    TableTerm D{};
+    D.kind = (signed char)T.kind;
+    D.power = (signed char)T.power;
+    D.sign = (signed char)T.sign;
+    D.bit = (signed char)T.bit;
     D.coeff = T.coeff;
     D.g0 = T.g0;
     D.g1 = T.g1;
-    D.ctrlMode = 0;
-    D.ctrlLocal = 0;
     if (T.kind == kTermPoly && T.ctrlBit >= 0) {
       if (T.ctrlBit >= lo && T.ctrlBit < hi) {
         D.ctrlMode = 2;
-        D.ctrlLocal = T.ctrlBit - lo;
+        D.ctrlLocal = (signed char)(T.ctrlBit - lo);
       } else {
         D.ctrlMode = 1;
         for (int c = 0; c < nExt; ++c)
-          if (extBits[c] == T.ctrlBit) D.ctrlLocal = c;
+          if (extBits[c] == T.ctrlBit) D.ctrlLocal = (signed char)c;
       }
     }
+    job.terms.push_back(D);
   }
-  int total = job.N << nExt;
-  int threads = 256;
-  int blocks = (total + threads - 1) / threads;
-  if (blocks > 1184) blocks = 1184;
-  {
-    LaunchScope _ls(ctx, kKTable);
-    k_build_table<<<blocks, threads, 0, ctx->stream>>>(job, out);
+  if (ctx->plan) {
+    ctx->plan->tables.push_back(std::move(job));
+    return true;
   }
-  return cuda_ok(ctx, cudaGetLastError(), "build_table launch");
+  return launch_tables(ctx, {std::move(job)});
 }
 
 bool launch_build_table(Context* ctx, int r, bool ctrl, const Term* terms, int nTerms,
@@ -244,19 +293,14 @@ static int grid_for(uint64_t work, int threads, int perThread) {
 }
 
 bool launch_diag(Context* ctx, const FactorList& F) {
-  uint64_t n = ctx->size();
-  int blocks = grid_for(n, 256, 4);
-  if (ctx->precision == kC128)
-    {
-      LaunchScope _ls(ctx, kKDiag);
-      k_diag<double2><<<blocks, 256, 0, ctx->stream>>>((double2*)ctx->state(), n, F);
-    }
-  else
-    {
-      LaunchScope _ls(ctx, kKDiag);
-      k_diag<float2><<<blocks, 256, 0, ctx->stream>>>((float2*)ctx->state(), n, F);
-    }
-  return cuda_ok(ctx, cudaGetLastError(), "diag launch");
+  const uint64_t n = ctx->size();
+  const int blocks = grid_for(n, 256, 4);
+  void* st = ctx->state();
+  return enqueue(ctx, kKDiag, "diag launch", [=] {
+    if (ctx->precision == kC128) k_diag<double2><<<blocks, 256, 0, ctx->stream>>>((double2*)st, n, F);
+    else k_diag<float2><<<blocks, 256, 0, ctx->stream>>>((float2*)st, n, F);
+    return cudaGetLastError();
+  });
 }
 
 // ----------------------------------------------------------------- pair (2x2)
@@ -319,12 +363,10 @@ __global__ void __launch_bounds__(256) k_pair(C* __restrict__ st, uint64_t npair
 }
 
 template <typename C>
-static void pair_launch(Context* ctx, uint64_t np, int bit, const double2 m[4],
+static void pair_launch(Context* ctx, C* st, uint64_t np, int bit, const double2 m[4],
                         const FactorList& pre, const FactorList& post) {
-  LaunchScope _ls(ctx, kKPair);
   bool none = factor_empty(pre) && factor_empty(post);
   bool small = pre.nTab <= 2 && post.nTab <= 2 && pre.nXX == 0 && post.nXX == 0;
-  C* st = (C*)ctx->state();
   if (none)
     k_pair<C, 0><<<grid_for(np, 256, kPairV), 256, 0, ctx->stream>>>(st, np, bit, m[0], m[1], m[2],
                                                                       m[3], pre, post);
@@ -336,12 +378,20 @@ static void pair_launch(Context* ctx, uint64_t np, int bit, const double2 m[4],
                                                                       m[2], m[3], pre, post);
 }
 
+struct PairMatrix {
+  double2 m[4];
+};
+
 bool launch_pair(Context* ctx, int bit, const double2 m[4], const FactorList& pre,
                  const FactorList& post) {
-  uint64_t np = ctx->size() / 2;
-  if (ctx->precision == kC128) pair_launch<double2>(ctx, np, bit, m, pre, post);
-  else pair_launch<float2>(ctx, np, bit, m, pre, post);
-  return cuda_ok(ctx, cudaGetLastError(), "pair launch");
+  const uint64_t np = ctx->size() / 2;
+  void* st = ctx->state();
+  const PairMatrix M = {{m[0], m[1], m[2], m[3]}};
+  return enqueue(ctx, kKPair, "pair launch", [=] {
+    if (ctx->precision == kC128) pair_launch<double2>(ctx, (double2*)st, np, bit, M.m, pre, post);
+    else pair_launch<float2>(ctx, (float2*)st, np, bit, M.m, pre, post);
+    return cudaGetLastError();
+  });
 }
 
 // ----------------------------------------------------------------- permutations
@@ -409,23 +459,19 @@ bool launch_perm(Context* ctx, const Stage& st, const FactorList& pre, const Fac
   P.q1 = ctx->q[st.reg];
   P.shift2 = st.reg2 >= 0 ? ctx->flw[st.reg2] : 0;
   P.ctrlBit = st.bit;
-  uint64_t n = ctx->size();
-  int blocks = grid_for(n, 256, 4);
-  if (ctx->precision == kC128)
-    {
-      LaunchScope _ls(ctx, kKPerm);
-      k_perm<double2><<<blocks, 256, 0, ctx->stream>>>((const double2*)ctx->state(),
-                                                       (double2*)ctx->other(), n, P, pre, post);
-    }
-  else
-    {
-      LaunchScope _ls(ctx, kKPerm);
-      k_perm<float2><<<blocks, 256, 0, ctx->stream>>>((const float2*)ctx->state(),
-                                                      (float2*)ctx->other(), n, P, pre, post);
-    }
-  if (!cuda_ok(ctx, cudaGetLastError(), "perm launch")) return false;
-  ctx->cur ^= 1;
-  return true;
+  const uint64_t n = ctx->size();
+  const int blocks = grid_for(n, 256, 4);
+  const void* in = ctx->state();
+  void* out = ctx->other();
+  const bool ok = enqueue(ctx, kKPerm, "perm launch", [=] {
+    if (ctx->precision == kC128)
+      k_perm<double2><<<blocks, 256, 0, ctx->stream>>>((const double2*)in, (double2*)out, n, P, pre, post);
+    else
+      k_perm<float2><<<blocks, 256, 0, ctx->stream>>>((const float2*)in, (float2*)out, n, P, pre, post);
+    return cudaGetLastError();
+  });
+  if (ok) ctx->cur ^= 1;
+  return ok;
 }
 
 // ----------------------------------------------------------------- separable init
@@ -436,8 +482,7 @@ bool launch_perm(Context* ctx, const Stage& st, const FactorList& pre, const Fac
 struct InitDesc {
   int numReg;
   int qLast;
-  const double2* arr;   // concatenated register arrays
-  int off[kMaxRegs];
+  const double2* arr[kMaxRegs];  // the register arrays
   int shift[kMaxRegs];  // flw of each register minus qLast (index into outer)
   int mask[kMaxRegs];
 };
@@ -448,7 +493,7 @@ __global__ void k_init_outer(InitDesc D, double2* outer, uint64_t nOuter) {
     double2 p = make_double2(1.0, 0.0);
     for (int r = D.numReg - 2; r >= 0; --r) {
       int j = (int)((h >> D.shift[r]) & (uint64_t)D.mask[r]);
-      p = dmul(p, D.arr[D.off[r] + j]);
+      p = dmul(p, D.arr[r][j]);
     }
     outer[h] = p;
   }
@@ -472,9 +517,8 @@ static InitDesc init_desc(Context* ctx, const double2* const* regArrays) {
   InitDesc D{};
   D.numReg = R;
   D.qLast = qLast;
-  D.arr = regArrays[0];
   for (int r = 0; r < R; ++r) {
-    D.off[r] = (int)(regArrays[r] - regArrays[0]);
+    D.arr[r] = regArrays[r];
     D.shift[r] = ctx->flw[r] - qLast;
     D.mask[r] = (1 << ctx->q[r]) - 1;
   }
@@ -483,43 +527,38 @@ static InitDesc init_desc(Context* ctx, const double2* const* regArrays) {
 
 bool launch_outer(Context* ctx, const double2* const* regArrays, double2* outer) {
   int R = ctx->numReg;
-  uint64_t nOuter = 1ull << (ctx->totalQbt - ctx->q[R - 1]);
+  const uint64_t nOuter = 1ull << (ctx->totalQbt - ctx->q[R - 1]);
   if (R >= 2) {
-    InitDesc D = init_desc(ctx, regArrays);
-    {
-      LaunchScope _ls(ctx, kKInit);
+    const InitDesc D = init_desc(ctx, regArrays);
+    return enqueue(ctx, kKInit, "outer launch", [=] {
       k_init_outer<<<grid_for(nOuter, 256, 1), 256, 0, ctx->stream>>>(D, outer, nOuter);
-    }
-    return cuda_ok(ctx, cudaGetLastError(), "outer launch");
+      return cudaGetLastError();
+    });
   }
   static const double2 one = {1.0, 0.0};
-  return cuda_ok(ctx, cudaMemcpyAsync(outer, &one, sizeof(one), cudaMemcpyHostToDevice, ctx->stream),
-                 "outer copy");
+  return enqueue(ctx, -1, "outer copy", [=] {
+    return cudaMemcpyAsync(outer, &one, sizeof(one), cudaMemcpyHostToDevice, ctx->stream);
+  });
 }
 
 bool launch_init_product(Context* ctx, const double2* const* regArrays) {
-  // regArrays: device pointers to our own copies (arena), one per register
-  int R = ctx->numReg;
-  int qLast = ctx->q[R - 1];
-  uint64_t nOuter = 1ull << (ctx->totalQbt - qLast);
+  // regArrays: device pointers to our own copies, one per register
+  const int R = ctx->numReg, qLast = ctx->q[R - 1];
+  const uint64_t nOuter = 1ull << (ctx->totalQbt - qLast);
   double2* outer = (double2*)arena_alloc(ctx, nOuter * sizeof(double2));
   if (!outer) return false;
   if (!launch_outer(ctx, regArrays, outer)) return false;
-  uint64_t n = ctx->size();
-  int blocks = grid_for(n, 256, 4);
-  if (ctx->precision == kC128)
-    {
-      LaunchScope _ls(ctx, kKInit);
-      k_init_product<double2><<<blocks, 256, 0, ctx->stream>>>((double2*)ctx->state(), n, qLast,
-                                                               regArrays[R - 1], outer);
-    }
-  else
-    {
-      LaunchScope _ls(ctx, kKInit);
-      k_init_product<float2><<<blocks, 256, 0, ctx->stream>>>((float2*)ctx->state(), n, qLast,
-                                                              regArrays[R - 1], outer);
-    }
-  return cuda_ok(ctx, cudaGetLastError(), "init launch");
+  const uint64_t n = ctx->size();
+  const int blocks = grid_for(n, 256, 4);
+  const double2* last = regArrays[R - 1];
+  void* st = ctx->state();
+  return enqueue(ctx, kKInit, "init launch", [=] {
+    if (ctx->precision == kC128)
+      k_init_product<double2><<<blocks, 256, 0, ctx->stream>>>((double2*)st, n, qLast, last, outer);
+    else
+      k_init_product<float2><<<blocks, 256, 0, ctx->stream>>>((float2*)st, n, qLast, last, outer);
+    return cudaGetLastError();
+  });
 }
 
 }  // namespace cvdv

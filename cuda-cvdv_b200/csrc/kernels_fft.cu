@@ -309,26 +309,15 @@ static bool run_passes(Context* ctx, const void* src, void* const* dsts, uint64_
     uint64_t blocks = 1ull << (logCols - logB);
     int RP = (P.logR >= 3 ? ((1 << P.logR) + ((1 << P.logR) >> 3)) : (1 << P.logR)) | 1;
     size_t smem = (size_t)RP * (1ull << logB) * sizeof(C);
-    const FactorList& fpre = P.first ? pre : empty;
-    const FactorList& fpost = P.last ? post : empty;
-    if (dir > 0) {
-      cudaFuncSetAttribute(k_fft_pass<C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-      {
-        LaunchScope _ls(ctx, kKFft);
-        k_fft_pass<C, 1><<<(unsigned)blocks, kFftThreads, smem, ctx->stream>>>(
-            (const C*)in, (C*)outp, P, fpre, fpost);
-      }
-    } else {
-      cudaFuncSetAttribute(k_fft_pass<C, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-      {
-        LaunchScope _ls(ctx, kKFft);
-        k_fft_pass<C, -1><<<(unsigned)blocks, kFftThreads, smem, ctx->stream>>>(
-            (const C*)in, (C*)outp, P, fpre, fpost);
-      }
-    }
-    if (!cuda_ok(ctx, cudaGetLastError(), "fft pass launch")) return false;
+    const FactorList fpre = P.first ? pre : empty;
+    const FactorList fpost = P.last ? post : empty;
+    if (!enqueue(ctx, kKFft, "fft pass launch", [=] {
+          auto kern = dir > 0 ? k_fft_pass<C, 1> : k_fft_pass<C, -1>;
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          kern<<<(unsigned)blocks, kFftThreads, smem, ctx->stream>>>((const C*)in, (C*)outp, P, fpre, fpost);
+          return cudaGetLastError();
+        }))
+      return false;
     in = outp;
     logNs += P.logR;
   }

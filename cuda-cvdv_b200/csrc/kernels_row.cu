@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(1 << (LOGN - LOGC - 4), 1 << (LOGC - 1))
   }
 }
 template <typename C, int LOGN, int LOGC, bool XX>
-static cudaError_t launch_rowq_t(Context* ctx, const RowProgram& P) {
+static cudaError_t launch_rowq_t(Context* ctx, const void* in, void* out, const RowProgram& P) {
   constexpr int M = 1 << (LOGN - LOGC), NC = 1 << LOGC;
   const size_t smem = (size_t)(M + (M >> 4)) * sizeof(C) + 2 * (64 + (M >> 6)) * sizeof(double2);
   auto kern = k_rowq<C, LOGN, LOGC, XX>;
@@ -805,7 +805,7 @@ static cudaError_t launch_rowq_t(Context* ctx, const RowProgram& P) {
   }
   const uint64_t nc = nRows < (uint64_t)clusters[dev] ? nRows : (uint64_t)clusters[dev];
   cfg.gridDim = dim3((unsigned)(NC * nc));
-  return cudaLaunchKernelEx(&cfg, kern, (const C*)ctx->state(), (C*)ctx->other(), nRows, P);
+  return cudaLaunchKernelEx(&cfg, kern, (const C*)in, (C*)out, nRows, P);
 }
 
 // ---------------------------------------------------------------- host side
@@ -910,7 +910,8 @@ bool row_diag_fits(Context* ctx, int reg, const std::vector<Term>& terms) {
 }
 
 template <typename C, int LOGC, int LOGT>
-static cudaError_t launch_row_t(Context* ctx, const RowProgram& P, uint64_t nCta, size_t smem) {
+static cudaError_t launch_row_t(Context* ctx, const void* in, void* out, const RowProgram& P, uint64_t nCta,
+                                size_t smem) {
   auto kern = k_row<C, LOGC, LOGT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -926,7 +927,7 @@ static cudaError_t launch_row_t(Context* ctx, const RowProgram& P, uint64_t nCta
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, (const C*)ctx->state(), (C*)ctx->other(), P);
+  return cudaLaunchKernelEx(&cfg, kern, (const C*)in, (C*)out, P);
 }
 
 // 2^14-point complex128 rows run on the eight-CTA kernel (k_rowq).  Complex64 rows
@@ -1130,6 +1131,14 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
       alternating &= P.ops[o].dir != lastDir;
       lastDir = P.ops[o].dir;
     }
+  // the launch, out of place into the other buffer, which then holds the state
+  const void* in = ctx->state();
+  void* out = ctx->other();
+  auto run = [ctx](int kind, auto f) {
+    const bool ok = enqueue(ctx, kind, "row program launch", f);
+    if (ok) ctx->cur ^= 1;
+    return ok;
+  };
   if (useC && !elemF && alternating) {
     if (blockedIn) P.loadT = 2;
     P.storeBlocked = blockedOut ? 1 : 0;
@@ -1137,16 +1146,12 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
       P.rowSums = ctx->rowSums;
       ctx->rowSumParts = 32;  // 8 CTAs x 4 warps
     }
-    cudaError_t er;
-    {
-      LaunchScope _ls(ctx, kKFft);
-      bool xx = false;
-      for (int d = 0; d < P.nDiag; ++d) xx |= P.diag[d].nLin > 0;
-      er = xx ? launch_rowq_t<double2, 14, 3, true>(ctx, P) : launch_rowq_t<double2, 14, 3, false>(ctx, P);
-    }
-    if (!cuda_ok(ctx, er, "row program launch")) return false;
-    ctx->cur ^= 1;
-    return true;
+    bool xx = false;
+    for (int d = 0; d < P.nDiag; ++d) xx |= P.diag[d].nLin > 0;
+    return run(kKFft, [=] {
+      return xx ? launch_rowq_t<double2, 14, 3, true>(ctx, in, out, P)
+                : launch_rowq_t<double2, 14, 3, false>(ctx, in, out, P);
+    });
   }
   if (toRowr) {
     if (elemF) {
@@ -1159,17 +1164,13 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
       P.rowSums = ctx->rowSums;
       ctx->rowSumParts = tpr < 32 ? 1 : tpr / 32;
     }
-    cudaError_t er;
-    {
-      LaunchScope _ls(ctx, col ? kKCol : kKFft);
+    return run(col ? kKCol : kKFft, [=] {
       if (col)
-        er = ctx->precision == kC128 ? launch_rowr<double2, true>(ctx, P, q) : launch_rowr<float2, true>(ctx, P, q);
-      else
-        er = ctx->precision == kC128 ? launch_rowr<double2, false>(ctx, P, q) : launch_rowr<float2, false>(ctx, P, q);
-    }
-    if (!cuda_ok(ctx, er, "row program launch")) return false;
-    ctx->cur ^= 1;
-    return true;
+        return ctx->precision == kC128 ? launch_rowr<double2, true>(ctx, in, out, P, q)
+                                       : launch_rowr<float2, true>(ctx, in, out, P, q);
+      return ctx->precision == kC128 ? launch_rowr<double2, false>(ctx, in, out, P, q)
+                                     : launch_rowr<float2, false>(ctx, in, out, P, q);
+    });
   }
   uint64_t tile = 1ull << lt;
   uint64_t nCta = ctx->size() / tile;
@@ -1177,24 +1178,18 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
   size_t rows = 1ull << P.logRows;
   size_t smem = rs * rows * ctx->elemBytes + (64 + 128 + 64 + 512) * sizeof(double2) +
                 rows * P.nDiag * (sizeof(double2) + sizeof(int)) + 16;
-  cudaError_t e;
-  {
-    LaunchScope _ls(ctx, kKFft);
+  return run(kKFft, [=] {
     if (ctx->precision == kC128) {
-      if (logT == 8) e = launch_row_t<double2, 0, 8>(ctx, P, nCta, smem);
-      else if (logC == 0) e = launch_row_t<double2, 0, 9>(ctx, P, nCta, smem);
-      else if (logC == 1) e = launch_row_t<double2, 1, 9>(ctx, P, nCta, smem);
-      else e = launch_row_t<double2, 2, 9>(ctx, P, nCta, smem);
-    } else {
-      if (logT == 8) e = launch_row_t<float2, 0, 8>(ctx, P, nCta, smem);
-      else if (logC == 0) e = launch_row_t<float2, 0, 9>(ctx, P, nCta, smem);
-      else if (logC == 1) e = launch_row_t<float2, 1, 9>(ctx, P, nCta, smem);
-      else e = launch_row_t<float2, 2, 9>(ctx, P, nCta, smem);
+      if (logT == 8) return launch_row_t<double2, 0, 8>(ctx, in, out, P, nCta, smem);
+      if (logC == 0) return launch_row_t<double2, 0, 9>(ctx, in, out, P, nCta, smem);
+      if (logC == 1) return launch_row_t<double2, 1, 9>(ctx, in, out, P, nCta, smem);
+      return launch_row_t<double2, 2, 9>(ctx, in, out, P, nCta, smem);
     }
-  }
-  if (!cuda_ok(ctx, e, "row program launch")) return false;
-  ctx->cur ^= 1;
-  return true;
+    if (logT == 8) return launch_row_t<float2, 0, 8>(ctx, in, out, P, nCta, smem);
+    if (logC == 0) return launch_row_t<float2, 0, 9>(ctx, in, out, P, nCta, smem);
+    if (logC == 1) return launch_row_t<float2, 1, 9>(ctx, in, out, P, nCta, smem);
+    return launch_row_t<float2, 2, 9>(ctx, in, out, P, nCta, smem);
+  });
 }
 
 }  // namespace cvdv

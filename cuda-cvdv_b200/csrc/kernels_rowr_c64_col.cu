@@ -2,5 +2,5 @@
 #include "rowr.cuh"
 
 namespace cvdv {
-template cudaError_t launch_rowr<float2, true>(Context*, const RowProgram&, int);
+template cudaError_t launch_rowr<float2, true>(Context*, const void*, void*, const RowProgram&, int);
 }  // namespace cvdv

@@ -348,10 +348,10 @@ int seq_max_bits(Context* ctx) {
 }
 
 template <typename C, int NB, int SPLIT, typename IDX>
-static void seq_go(Context* ctx, unsigned blocks, uint64_t nSites, const SeqProgram& P) {
+static void seq_go(Context* ctx, void* state, unsigned blocks, uint64_t nSites, const SeqProgram& P) {
   bool gen = false;
   for (int o = 0; o < P.nOps; ++o) gen |= P.ops[o].kind == kSeqPair || P.ops[o].kind == kSeqPairReal;
-  C* st = (C*)ctx->state();
+  C* st = (C*)state;
   if (P.prodLast) {
     if (gen) k_seq<C, NB, SPLIT, IDX, true, true><<<blocks, 256, 0, ctx->stream>>>(st, (IDX)nSites, P);
     else k_seq<C, NB, SPLIT, IDX, false, true><<<blocks, 256, 0, ctx->stream>>>(st, (IDX)nSites, P);
@@ -362,15 +362,15 @@ static void seq_go(Context* ctx, unsigned blocks, uint64_t nSites, const SeqProg
 }
 
 template <typename C, typename IDX>
-static void seq_dispatch(Context* ctx, int nb, unsigned blocks, uint64_t nSites, const SeqProgram& P) {
+static void seq_dispatch(Context* ctx, void* state, int nb, unsigned blocks, uint64_t nSites, const SeqProgram& P) {
   switch (nb) {
-    case 1: seq_go<C, 1, 0, IDX>(ctx, blocks, nSites, P); break;
-    case 2: seq_go<C, 2, 0, IDX>(ctx, blocks, nSites, P); break;
-    case 3: seq_go<C, 3, 0, IDX>(ctx, blocks, nSites, P); break;
-    case 4: seq_go<C, 4, 0, IDX>(ctx, blocks, nSites, P); break;
+    case 1: seq_go<C, 1, 0, IDX>(ctx, state, blocks, nSites, P); break;
+    case 2: seq_go<C, 2, 0, IDX>(ctx, state, blocks, nSites, P); break;
+    case 3: seq_go<C, 3, 0, IDX>(ctx, state, blocks, nSites, P); break;
+    case 4: seq_go<C, 4, 0, IDX>(ctx, state, blocks, nSites, P); break;
     default:
-      if constexpr (sizeof(C) == sizeof(float2)) seq_go<C, 5, 0, IDX>(ctx, blocks, nSites, P);
-      else seq_go<C, 5, 1, IDX>(ctx, blocks, nSites, P);
+      if constexpr (sizeof(C) == sizeof(float2)) seq_go<C, 5, 0, IDX>(ctx, state, blocks, nSites, P);
+      else seq_go<C, 5, 1, IDX>(ctx, state, blocks, nSites, P);
       break;
   }
 }
@@ -486,17 +486,17 @@ bool launch_seq(Context* ctx, const std::vector<HostSeqOp>& ops) {
   const uint64_t cap = 32ull * (uint64_t)ctx->numSMs;
   if (blocks > cap) blocks = cap;
   const bool narrow = ctx->totalQbt <= 31;  // every flat index fits 32 bits
-  {
-    LaunchScope _ls(ctx, kKSeq);
+  void* st = ctx->state();
+  return enqueue(ctx, kKSeq, "qubit-gate sequence launch", [=] {
     if (ctx->precision == kC128) {
-      if (narrow) seq_dispatch<double2, uint32_t>(ctx, nb, (unsigned)blocks, nSites, P);
-      else seq_dispatch<double2, uint64_t>(ctx, nb, (unsigned)blocks, nSites, P);
+      if (narrow) seq_dispatch<double2, uint32_t>(ctx, st, nb, (unsigned)blocks, nSites, P);
+      else seq_dispatch<double2, uint64_t>(ctx, st, nb, (unsigned)blocks, nSites, P);
     } else {
-      if (narrow) seq_dispatch<float2, uint32_t>(ctx, nb, (unsigned)blocks, nSites, P);
-      else seq_dispatch<float2, uint64_t>(ctx, nb, (unsigned)blocks, nSites, P);
+      if (narrow) seq_dispatch<float2, uint32_t>(ctx, st, nb, (unsigned)blocks, nSites, P);
+      else seq_dispatch<float2, uint64_t>(ctx, st, nb, (unsigned)blocks, nSites, P);
     }
-  }
-  return cuda_ok(ctx, cudaGetLastError(), "qubit-gate sequence launch");
+    return cudaGetLastError();
+  });
 }
 
 }  // namespace cvdv

@@ -447,18 +447,19 @@ bool tc_col_ok(Context* ctx, int reg) {
 }
 
 template <int KIND, int D1, int D2>
-static cudaError_t tc_launch_t(Context* ctx, const TcPass& T) {
+static cudaError_t tc_launch_t(Context* ctx, const void* in, void* out, const TcPass& T) {
   auto kern = k_coltc<KIND, D1, D2>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
   if (e != cudaSuccess) return e;
   const uint64_t grid = T.nTiles < (uint64_t)ctx->numSMs ? T.nTiles : (uint64_t)ctx->numSMs;
-  kern<<<(unsigned)grid, kTcThreads, kTcSmem, ctx->stream>>>((const float2*)ctx->state(), (float2*)ctx->other(), T);
+  kern<<<(unsigned)grid, kTcThreads, kTcSmem, ctx->stream>>>((const float2*)in, (float2*)out, T);
   return cudaGetLastError();
 }
 
 // One pass of a column chain (kernels_col.cu: run_col_chain) on the tensor cores;
 // logL is the pass's DFT length, kind / d1 / d2 as for k_colr.
-cudaError_t launch_col_tc(Context* ctx, const ColPass& P, int logL, int kind, int d1, int d2) {
+cudaError_t launch_col_tc(Context* ctx, const void* in, void* out, const ColPass& P, int logL, int kind, int d1,
+                          int d2) {
   if (logL < 6 || logL > 7 || P.logS < 5 || P.logN > 14 || kind == kColWhole) return cudaErrorInvalidValue;
   const int lpt = 1 << (7 - logL);
   if (P.logA < 7 - logL) return cudaErrorInvalidValue;
@@ -470,11 +471,11 @@ cudaError_t launch_col_tc(Context* ctx, const ColPass& P, int logL, int kind, in
   T.nTiles = P.nCols / (uint64_t)(kTcW * lpt);
   T.err = ctx->waitErr;
   switch (kind) {
-    case kColFirst: return d1 > 0 ? tc_launch_t<kColFirst, 1, 0>(ctx, T) : tc_launch_t<kColFirst, -1, 0>(ctx, T);
-    case kColLast: return d1 > 0 ? tc_launch_t<kColLast, 1, 0>(ctx, T) : tc_launch_t<kColLast, -1, 0>(ctx, T);
+    case kColFirst: return d1 > 0 ? tc_launch_t<kColFirst, 1, 0>(ctx, in, out, T) : tc_launch_t<kColFirst, -1, 0>(ctx, in, out, T);
+    case kColLast: return d1 > 0 ? tc_launch_t<kColLast, 1, 0>(ctx, in, out, T) : tc_launch_t<kColLast, -1, 0>(ctx, in, out, T);
     default:
-      if (d1 > 0) return d2 > 0 ? tc_launch_t<kColMiddle, 1, 1>(ctx, T) : tc_launch_t<kColMiddle, 1, -1>(ctx, T);
-      return d2 > 0 ? tc_launch_t<kColMiddle, -1, 1>(ctx, T) : tc_launch_t<kColMiddle, -1, -1>(ctx, T);
+      if (d1 > 0) return d2 > 0 ? tc_launch_t<kColMiddle, 1, 1>(ctx, in, out, T) : tc_launch_t<kColMiddle, 1, -1>(ctx, in, out, T);
+      return d2 > 0 ? tc_launch_t<kColMiddle, -1, 1>(ctx, in, out, T) : tc_launch_t<kColMiddle, -1, -1>(ctx, in, out, T);
   }
 }
 

@@ -263,7 +263,7 @@ constexpr int kRowrSmallLog = 19;
 inline bool rowr_small(Context* ctx) { return ctx->totalQbt < kRowrSmallLog; }
 
 template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
-static cudaError_t launch_rowr_s(Context* ctx, const RowProgram& P) {
+static cudaError_t launch_rowr_s(Context* ctx, const void* in, void* out, const RowProgram& P) {
   constexpr int NT = 1 << (LOGM - LOGE + LOGR);
   const size_t smem = (size_t)rr_row_slots(LOGM, LOGE) * (1 << LOGR) * sizeof(C) + rr_tw_slots(LOGM) * sizeof(double2);
   auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL>;
@@ -279,43 +279,43 @@ static cudaError_t launch_rowr_s(Context* ctx, const RowProgram& P) {
   if (nTiles < 1) nTiles = 1;
   uint64_t grid = NT > 256 ? (uint64_t)ctx->numSMs * resident : nTiles;
   if (grid > nTiles) grid = nTiles;
-  kern<<<(unsigned)grid, NT, smem, ctx->stream>>>((const C*)ctx->state(), (C*)ctx->other(), nTiles, P);
+  kern<<<(unsigned)grid, NT, smem, ctx->stream>>>((const C*)in, (C*)out, nTiles, P);
   return cudaGetLastError();
 }
 
 template <typename C, int LOGM, bool COL>
-static cudaError_t launch_rowr_t(Context* ctx, const RowProgram& P) {
+static cudaError_t launch_rowr_t(Context* ctx, const void* in, void* out, const RowProgram& P) {
   constexpr int LOGE = RrShape<C, LOGM>::LOGE, LOGR0 = RrShape<C, LOGM>::LOGR;
   // column form: at least two columns a CTA while it stays within 512 threads
   constexpr int LOGR = (COL && LOGR0 == 0 && (LOGM - LOGE) < 9) ? 1 : LOGR0;
   if constexpr (LOGM >= 8 && LOGM <= 12) {
-    if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, 0, 3, COL>(ctx, P);
+    if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, 0, 3, COL>(ctx, in, out, P);
   }
-  return launch_rowr_s<C, LOGM, LOGR, LOGE, COL>(ctx, P);
+  return launch_rowr_s<C, LOGM, LOGR, LOGE, COL>(ctx, in, out, P);
 }
 
 template <typename C, bool COL>
-cudaError_t launch_rowr(Context* ctx, const RowProgram& P, int q) {
+cudaError_t launch_rowr(Context* ctx, const void* in, void* out, const RowProgram& P, int q) {
   switch (q) {
-    case 4: return launch_rowr_t<C, 4, COL>(ctx, P);
-    case 5: return launch_rowr_t<C, 5, COL>(ctx, P);
-    case 6: return launch_rowr_t<C, 6, COL>(ctx, P);
-    case 7: return launch_rowr_t<C, 7, COL>(ctx, P);
-    case 8: return launch_rowr_t<C, 8, COL>(ctx, P);
-    case 9: return launch_rowr_t<C, 9, COL>(ctx, P);
-    case 10: return launch_rowr_t<C, 10, COL>(ctx, P);
-    case 11: return launch_rowr_t<C, 11, COL>(ctx, P);
-    case 12: return launch_rowr_t<C, 12, COL>(ctx, P);
-    case 13: return launch_rowr_t<C, 13, COL>(ctx, P);
+    case 4: return launch_rowr_t<C, 4, COL>(ctx, in, out, P);
+    case 5: return launch_rowr_t<C, 5, COL>(ctx, in, out, P);
+    case 6: return launch_rowr_t<C, 6, COL>(ctx, in, out, P);
+    case 7: return launch_rowr_t<C, 7, COL>(ctx, in, out, P);
+    case 8: return launch_rowr_t<C, 8, COL>(ctx, in, out, P);
+    case 9: return launch_rowr_t<C, 9, COL>(ctx, in, out, P);
+    case 10: return launch_rowr_t<C, 10, COL>(ctx, in, out, P);
+    case 11: return launch_rowr_t<C, 11, COL>(ctx, in, out, P);
+    case 12: return launch_rowr_t<C, 12, COL>(ctx, in, out, P);
+    case 13: return launch_rowr_t<C, 13, COL>(ctx, in, out, P);
     default:
-      if constexpr (sizeof(C) == sizeof(float2)) return launch_rowr_t<C, 14, COL>(ctx, P);
+      if constexpr (sizeof(C) == sizeof(float2)) return launch_rowr_t<C, 14, COL>(ctx, in, out, P);
       return cudaErrorInvalidValue;
   }
 }
 
-extern template cudaError_t launch_rowr<double2, false>(Context*, const RowProgram&, int);
-extern template cudaError_t launch_rowr<double2, true>(Context*, const RowProgram&, int);
-extern template cudaError_t launch_rowr<float2, false>(Context*, const RowProgram&, int);
-extern template cudaError_t launch_rowr<float2, true>(Context*, const RowProgram&, int);
+extern template cudaError_t launch_rowr<double2, false>(Context*, const void*, void*, const RowProgram&, int);
+extern template cudaError_t launch_rowr<double2, true>(Context*, const void*, void*, const RowProgram&, int);
+extern template cudaError_t launch_rowr<float2, false>(Context*, const void*, void*, const RowProgram&, int);
+extern template cudaError_t launch_rowr<float2, true>(Context*, const void*, void*, const RowProgram&, int);
 
 }  // namespace cvdv
