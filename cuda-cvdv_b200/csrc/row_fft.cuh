@@ -20,6 +20,15 @@ __device__ __forceinline__ int rpad(int e) {
 __host__ __device__ constexpr int rr_row_slots(int logM, int logE) {
   return (1 << logM) + ((1 << logM) >> (logE == 3 ? 3 : 4));
 }
+// The same with room for 2^logR columns interleaved lane by lane: the W lanes that one
+// phase of a 16- or 8-byte shared-memory access serves (W = 128 / bytes) are 2^logR
+// columns x W / 2^logR consecutive points, so lines W / 2^logR elements apart modulo W
+// put them on distinct banks; the padded length alone is a multiple of W, which put
+// all columns' points on the same banks.
+__host__ __device__ constexpr int rr_col_slots(int logM, int logE, int logR, int bytes) {
+  const int W = 128 / bytes, step = (W >> logR) > 1 ? (W >> logR) : 1, len = rr_row_slots(logM, logE);
+  return logR == 0 ? len : len + (step - len % W + W) % W;
+}
 __host__ __device__ constexpr int rr_tw_slots(int logM) { return 64 + (logM > 6 ? 1 << (logM - 6) : 1); }
 
 // ---------------------------------------------------------------- butterflies

@@ -171,6 +171,11 @@ __device__ __forceinline__ void l2_prefetch_tile(const void* p, uint32_t bytes) 
 // within 512 threads) are adjacent inner indices interleaved lane by lane, so a
 // warp's load covers runs of 2^LOGR amplitudes; the rest of each sector is read
 // from L2 by the CTAs of the neighbouring columns.
+template <typename C, int LOGM, int LOGE, int LOGR, bool COL>
+constexpr int rr_line_slots() {
+  return COL ? rr_col_slots(LOGM, LOGE, LOGR, (int)sizeof(C)) : rr_row_slots(LOGM, LOGE);
+}
+
 // The sum of |psi|^2 (FP64) over the E amplitudes of each of a group of W lanes
 // (W = 32, or the lanes of one row when a warp holds several), written by the
 // group's first lane.
@@ -191,7 +196,8 @@ __device__ __forceinline__ void row_sum_part(const C (&v)[E], double* out) {
 template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
 __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR) > 8 ? 1 : 2)
     k_rowr(const C* __restrict__ in, C* __restrict__ out, uint64_t nTiles, const __grid_constant__ RowProgram P) {
-  constexpr int E = 1 << LOGE, M = 1 << LOGM, TPR = M >> LOGE, NT = TPR << LOGR, RS = rr_row_slots(LOGM, LOGE);
+  constexpr int E = 1 << LOGE, M = 1 << LOGM, TPR = M >> LOGE, NT = TPR << LOGR;
+  constexpr int RS = rr_line_slots<C, LOGM, LOGE, LOGR, COL>();
   constexpr uint32_t TILE_BYTES = (uint32_t)sizeof(C) << (LOGM + LOGR);
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
@@ -265,7 +271,7 @@ inline bool rowr_small(Context* ctx) { return ctx->totalQbt < kRowrSmallLog; }
 template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
 static cudaError_t launch_rowr_s(Context* ctx, const void* in, void* out, const RowProgram& P) {
   constexpr int NT = 1 << (LOGM - LOGE + LOGR);
-  const size_t smem = (size_t)rr_row_slots(LOGM, LOGE) * (1 << LOGR) * sizeof(C) + rr_tw_slots(LOGM) * sizeof(double2);
+  const size_t smem = (size_t)rr_line_slots<C, LOGM, LOGE, LOGR, COL>() * (1 << LOGR) * sizeof(C) + rr_tw_slots(LOGM) * sizeof(double2);
   auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL>;
   static int resident = 0;  // CTAs per SM of this instantiation, asked once
   cudaError_t e = cudaSuccess;
