@@ -419,24 +419,26 @@ __global__ void __launch_bounds__(1 << LOGT, (LOGC > 0 || LOGT > 8) ? 1 : 2)
   if constexpr (LOGC > 0) cg::this_cluster().sync();  // no CTA leaves while peers may read it
 }
 
-// A program on a register that is not the last one runs on k_rowr in column
-// form for registers of 2^9 .. 2^14 (complex64) or 2^13 (complex128) points, at
-// least as many columns as one CTA takes.  The column loads are strided, but one
-// pass replaces the two per transform of the column kernel (with the linear-phase
-// runs taken without tables this also wins in complex128: 5.1 against 5.7 ms of
-// column work per [13, 13] layer); registers of up to 2^8 points run whole on the
-// column kernel anyway.
+// A program on a register that is not the last one runs on k_rowr in column form
+// for registers of 2^4 .. 2^14 (complex64) or 2^13 (complex128) points with at least
+// as many columns as one CTA takes: one pass over the state.  The column kernel
+// (k_colr) takes T + 1 passes for T transforms of more than 2^8 points, and its
+// whole-register pass for shorter ones evaluates the diagonal runs' factor lists per
+// point.  A rotation, a displacement and a squeeze (seven transforms) on a
+// 2^26-amplitude state, k_rowr against k_colr: complex128 1.42 against 2.45 ms (2^5
+// points), 1.54 against 2.95 (2^8), 2.76 against 4.60 (2^12); complex64 1.31 against
+// 2.10, 1.11 against 2.37, 1.95 against 3.47.  It wins at 2^18 and 2^22 amplitudes too.
 bool col_program_ok(Context* ctx, int reg) {
   const int q = ctx->q[reg];
   if (!ctx->colProg || ctx->flw[reg] == 0 || q < kRowMinLogN ||
       q > rowr_max_log(ctx->precision))
     return false;
-  if (q <= 8) return !(ctx->colFft && col_fft_ok(ctx, reg));  // the column kernel holds whole runs on these
   if (ctx->colFft && col_fft_ok(ctx, reg) && tc_col_ok(ctx, reg)) return false;  // chained tensor-core passes
   const int logE = (ctx->precision == kC64 && q >= 13) ? 5 : 4;
   const int logR = q - logE < 8 ? 8 - (q - logE) : (q - logE < 9 ? 1 : 0);
   // (states below the small-state line run one column per CTA)
-  return (q <= 12 && rowr_small(ctx)) || ctx->totalQbt - q >= logR;
+  // (short registers' surplus thread groups repeat columns)
+  return q < 8 || (q <= 12 && rowr_small(ctx)) || ctx->totalQbt - q >= logR;
 }
 
 // ---------------------------------------------------------------- cluster register-resident rows
