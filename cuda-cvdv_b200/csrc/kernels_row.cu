@@ -561,9 +561,6 @@ __device__ __forceinline__ void rq_diag(C (&v)[16], const RowDiag& D, uint64_t r
 }
 
 // ---- cluster primitives (distributed shared memory pushed by st.async)
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
 __device__ __forceinline__ uint32_t cluster_map(uint32_t a, int rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
@@ -1046,8 +1043,9 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
     D.permuted = opTransposed ? 1 : 0;
     D.ftSign = 0;
     D.nPl = 0;
-    // On the cluster kernel a run whose register terms are linear phases (transform
-    // twiddles, c x terms controlled by row bits) needs no table.
+    // A run whose register terms are linear phases (transform twiddles, c x terms
+    // controlled by row bits) needs no table on k_rowq and k_rowr; on k_rowr it may
+    // have uncontrolled c x^2 terms too (finite ones: the phases are reduced mod 1).
     {
       const int lo = ctx->flw[reg], hi = lo + q;
       bool linOnly = (useC || toRowr) && !regTerms.empty();
@@ -1059,6 +1057,7 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
           ++nPl;
           continue;
         }
+        if (toRowr && t.kind == kTermPoly && t.power == 2 && t.ctrlBit < 0) continue;
         linOnly = false;
       }
       if (linOnly) {
@@ -1067,15 +1066,21 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
             D.ftSign += t.sign;
             continue;
           }
+          if (t.power == 2) {
+            D.hasQuad = 1;
+            D.c2 += t.coeff;
+            continue;
+          }
           D.plC[D.nPl] = t.coeff;
           D.plCtrl[D.nPl++] = t.ctrlBit;
         }
-        D.regC = (double)((1 << q) - 1) * 0.5;
-        D.regDx = ctx->dx[reg];
         regTerms.clear();
         bits.clear();
         D.nCtrl = 0;
       }
+      D.regC = (double)((1 << q) - 1) * 0.5;
+      D.regDx = ctx->dx[reg];
+      D.linTurns = ctx->dx[reg] / (4.0 * CVDV_PI);
     }
     if (!regTerms.empty()) {
       double2* tab = (double2*)arena_alloc(ctx, ((size_t)1 << (q + D.nCtrl)) * sizeof(double2));
@@ -1108,8 +1113,6 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
         X.ctrlShift = t.ctrlBit;
       }
       elemTerms.swap(rest);
-      D.regC = (double)((1 << q) - 1) * 0.5;
-      D.regDx = ctx->dx[reg];
     }
     std::vector<Term> left;
     if (!build_factor_list(ctx, rowTerms, &D.rowF, &left) || !left.empty()) return false;

@@ -2,10 +2,14 @@
 // with its launcher, instantiated per precision and form in kernels_rowr_*.cu.
 #pragma once
 
+#include <cmath>
+
 #include "cvdv_internal.cuh"
 #include "row_fft.cuh"
 
 namespace cvdv {
+
+constexpr int kMaxRowE = 32;  // amplitudes a k_rowr thread holds, at most
 
 struct RowOp {
   int kind;
@@ -23,8 +27,7 @@ struct RowDiag {
   FactorList elemF;    // per-element factors (bilinear terms with the row register)
   // Bilinear terms c x_row x_other (other register and control bit off the row)
   // taken out of elemF for k_rowr: along one row they are the linear phase
-  // a (m - regC) regDx with a = sum c x_other (+-1 by the control bit), so a
-  // thread needs two sincos per run instead of one per amplitude.  The other
+  // a (m - regC) regDx with a = sum c x_other (+-1 by the control bit).  The other
   // register is side 1 of each XXFactor.
   int nLin;
   double regC, regDx;
@@ -34,6 +37,10 @@ struct RowDiag {
   // point n, and terms c x_n (x_n = (n - regC) regDx), each negated when its
   // control bit (a row bit, or none: -1) is set
   int ftSign;
+  int hasQuad;  // k_rowr: the run also has c2 x^2, c2 the sum of its uncontrolled terms
+  double c2;
+  double linTurns;           // turns per unit of u = 2 n - N + 1 of the phase x_n: dx / (4 pi)
+  double2 quad[kMaxRowE];    // exp(2 pi i c2 TPR^2 k^2 / N) for the kernel's E amplitudes a thread
   int nPl;
   double plC[2];
   int plCtrl[2];
@@ -87,17 +94,28 @@ __device__ __forceinline__ double2 ft_tw_ratio(long long d, long long N, int s) 
   return make_double2(c, sn);
 }
 
+// q m mod 1 (in -1/2 .. 1/2) for a phase of q m turns, m an integer that a double holds:
+// one rounding, however many turns
+__device__ __forceinline__ double turns(double q, double m) { return fma(q, m, -rint(q * m)); }
+
+// A diagonal run on the amplitudes t + k TPR (k < E) of a row.  Register terms of
+// degree up to two, transform twiddles and bilinear terms need no table: with
+// u = 2 n - N + 1 and x_n = dx u / 2, dx^2 = 2 pi / N, they are
+//   c2 x^2 = c2 u^2 / (4 N),  a x = a dx u / (4 pi),  twiddle = s (N-1) u / (4 N)
+// turns.  From u0 = 2 t - N + 1 a thread's points are u0 + 2 TPR k, so the factor is
+//   [value at u0] [step]^k [exp(2 pi i (4 c2 / 4 N) TPR^2 k^2)]:
+// two sincospi on turns reduced mod 1 without loss, a running product, and (c2 != 0)
+// E constants in the kernel's parameters.  A table entry per amplitude took 16 bytes
+// from L2 for every run (eight times the state's own traffic in a two-mode network
+// layer).  QUADNOTE
 template <typename C, int LOGM, int LOGE>
 __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uint64_t rowBase, int t) {
-  constexpr int E = 1 << LOGE, TPR = 1 << (LOGM - LOGE);
+  constexpr int E = 1 << LOGE, N = 1 << LOGM, TPR = 1 << (LOGM - LOGE);
   const double2 rs = D.hasRowF ? eval_factor(D.rowF, rowBase) : make_double2(1.0, 0.0);
   // running factor of element t + k TPR: rs times the linear phase, advanced by st per k
   double2 f = rs, st = make_double2(1.0, 0.0);
-  const bool lin = D.nLin || D.nPl || D.ftSign;
+  const bool lin = D.nLin || D.nPl || D.ftSign || D.hasQuad;
   if (lin) {
-    // bilinear terms with other registers and c x terms (controls off the row) are
-    // one linear phase a (m - regC) regDx along the row; the transform twiddle is
-    // exact at the first point and as a ratio per step
     double a = 0.0;
     for (int l = 0; l < D.nLin; ++l) {
       const XXFactor& X = D.lin[l];
@@ -108,15 +126,23 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
     }
     for (int k = 0; k < D.nPl; ++k)
       a += (D.plCtrl[k] >= 0 && ((rowBase >> D.plCtrl[k]) & 1ull)) ? -D.plC[k] : D.plC[k];
-    a *= D.regDx;
-    double s0, c0;
-    sincos(a * ((double)t - D.regC), &s0, &c0);
-    sincos(a * (double)TPR, &st.y, &st.x);
-    f = dmul(rs, make_double2(c0, s0));
-    if (D.ftSign) {
-      f = dmul(f, ft_tw_at(t, 1ll << LOGM, D.ftSign));
-      st = dmul(st, ft_tw_ratio(TPR, 1ll << LOGM, D.ftSign));
+    a *= D.linTurns;
+    const int u0 = 2 * t - N + 1;
+    // s (N-1) u mod 4N in integers: at most 3 2^28 for the runs of a program
+    constexpr double inv4N = 1.0 / (4.0 * N);
+    const int w = (D.ftSign * (N - 1)) & (4 * N - 1);
+    const double t0 = (double)((int)((long long)w * u0) & (4 * N - 1)) * inv4N;
+    const double t1 = (double)((int)((long long)w * (2 * TPR)) & (4 * N - 1)) * inv4N;
+    double p0 = t0 + turns(a, (double)u0), p1 = t1 + turns(a, 2.0 * TPR);
+    if (D.hasQuad) {
+      const double q = D.c2 * inv4N;
+      p0 += turns(q, (double)u0 * (double)u0);
+      p1 += turns(q, 4.0 * TPR * (double)u0);
     }
+    double s0, c0;
+    sincospi(2.0 * p0, &s0, &c0);
+    sincospi(2.0 * p1, &st.y, &st.x);
+    f = dmul(rs, make_double2(c0, s0));
   }
   if (D.tab) {
     int seg = 0;
@@ -134,6 +160,12 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
         v[k0 + k] = cmul(v[k0 + k], fromd<C>(w[k]));
       }
     }
+  } else if (D.hasQuad) {
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+      v[k] = cmul(v[k], fromd<C>(dmul(f, D.quad[k])));
+      f = dmul(f, st);
+    }
   } else if (lin) {
 #pragma unroll
     for (int k = 0; k < E; ++k) {
@@ -146,6 +178,28 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
     for (int k = 0; k < E; ++k) v[k] = cmul(v[k], c);
   }
 }
+
+// ---- asynchronous copies
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+// 16- or 8-byte asynchronous copy from global to shared memory
+template <int BYTES>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src) {
+  if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Runs `f` where its `on` is set: the last transform of a program's tile.
+template <typename F>
+struct HookIf {
+  bool on;
+  F f;
+  __device__ __forceinline__ void operator()() const {
+    if (on) f();
+  }
+};
 
 // 256-thread CTAs run two per SM; 512- and 1024-thread CTAs one
 // Ask L2 to fetch [p, p + bytes) ahead of use: bulk prefetches of 16 KB, one per
@@ -160,10 +214,14 @@ __device__ __forceinline__ void l2_prefetch_tile(const void* p, uint32_t bytes) 
 }
 
 // Tiles of one CTA per SM (more than 256 threads) run persistent: each CTA walks
-// tiles blockIdx.x, + gridDim.x, ... and asks L2 for its next tile before working
-// on the current one, so the next load finds its data on chip while this tile's
-// butterflies run.  Smaller tiles run two CTAs per SM, which already overlap one
-// CTA's loads with the other's work; they get one tile per CTA.
+// tiles blockIdx.x, + gridDim.x, ...  A row's next tile is asked into L2 before the
+// current one is worked on.  Once the current tile's last shared-memory exchange is
+// read, the exchange buffer is free: the next tile is copied into it asynchronously
+// (one bulk copy for a row, 16- or 8-byte copies for columns) while the last
+// butterflies, the runs after them and the stores go on, and the next tile starts
+// from shared memory.  PFNOTE
+// Smaller tiles run two CTAs per SM, which already overlap one CTA's loads with the
+// other's work; they get one tile per CTA.
 //
 // With COL the "rows" are the columns of a strided register (P.logS amplitudes
 // below it): column c is inner index c mod S and outer index c / S, and element m
@@ -199,6 +257,7 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR
   constexpr int E = 1 << LOGE, M = 1 << LOGM, TPR = M >> LOGE, NT = TPR << LOGR;
   constexpr int RS = rr_line_slots<C, LOGM, LOGE, LOGR, COL>();
   constexpr uint32_t TILE_BYTES = (uint32_t)sizeof(C) << (LOGM + LOGR);
+  constexpr bool PF = COL && NT > 256;  // the next tile is copied ahead
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
   double2* lo = reinterpret_cast<double2*>(sm + (RS << LOGR));  // w_M^e, e < 64
@@ -218,27 +277,64 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR
     if (e < M) lo[i] = __ldg(P.tw + ((size_t)e << scM));  // lo and hi are one array
   }
   __syncthreads();
-  // No barrier between tiles: after a transform's last exchange (which ends in a
-  // barrier) a thread touches shared memory again only in the next tile's first
-  // exchange, and every thread has left the old tile's exchanges by then.
+  // copies a tile's amplitudes into sm in thread order (sm[tid + k NT] becomes v[k])
+  auto fetch = [&](uint64_t tile) {
+    // a point's 2^LOGR adjacent columns are one run of up to 16 bytes, or several
+    constexpr int RUN = (int)sizeof(C) << LOGR, CH = RUN < 16 ? RUN : 16, PER = RUN / CH;
+    const uint64_t c = tile << LOGR;
+    const char* src = reinterpret_cast<const char*>(in + (c & ((1ull << logS) - 1)) + ((c >> logS) << (LOGM + logS)));
+    const uint32_t dst = smem_addr(sm);
+    const int logStep = logS + (sizeof(C) == 16 ? 4 : 3);  // bytes between points, log2
+#pragma unroll
+    for (int i = 0; i < (int)(TILE_BYTES / CH / NT); ++i) {
+      const int q = tid + i * NT;
+      cp_async<CH>(dst + q * CH, src + ((uint64_t)(q / PER) << logStep) + (q % PER) * CH);
+    }
+    cp_async_commit();
+  };
+  int lastFft = -1;
+  if constexpr (PF) {
+    for (int o = 0; o < P.nOps; ++o)
+      if (P.ops[o].kind != kRowDiag) lastFft = o;
+    fetch(blockIdx.x);
+  }
+  // Without PF there is no barrier between tiles: after a transform's last exchange
+  // (which ends in a barrier) a thread touches shared memory again only in the next
+  // tile's first exchange, and every thread has left the old tile's exchanges by then.
   for (uint64_t tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
+    const bool more = tile + gridDim.x < nTiles;
     uint64_t rowBase;
     if constexpr (COL) {
       const uint64_t c = (tile << LOGR) + (uint64_t)row;
       rowBase = (c & ((1ull << logS) - 1)) + ((c >> logS) << (LOGM + logS));
     } else {
-      if (NT > 256 && tile + gridDim.x < nTiles)
-        l2_prefetch_tile(in + ((tile + gridDim.x) << (LOGM + LOGR)), TILE_BYTES);
+      if (NT > 256 && more) l2_prefetch_tile(in + ((tile + gridDim.x) << (LOGM + LOGR)), TILE_BYTES);
       rowBase = (tile << (LOGM + LOGR)) + ((uint64_t)row << LOGM);
     }
     C v[E];
+    if constexpr (PF) {
+      cp_async_wait_all();
+      __syncthreads();
 #pragma unroll
-    for (int k = 0; k < E; ++k) v[k] = in[rowBase + ((uint64_t)(t + k * TPR) << logS)];
+      for (int k = 0; k < E; ++k) v[k] = sm[tid + k * NT];
+      __syncthreads();  // the buffer is the exchanges' again
+    } else {
+#pragma unroll
+      for (int k = 0; k < E; ++k) v[k] = in[rowBase + ((uint64_t)(t + k * TPR) << logS)];
+    }
     for (int o = 0; o < P.nOps; ++o) {
       const RowOp& op = P.ops[o];
-      if (op.kind == kRowDiag) rr_diag<C, LOGM, LOGE>(v, P.diag[op.diag], rowBase, t);
-      else if (op.dir > 0) rr_stages<C, 1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
-      else rr_stages<C, -1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
+      if (op.kind == kRowDiag) {
+        rr_diag<C, LOGM, LOGE>(v, P.diag[op.diag], rowBase, t);
+      } else if constexpr (PF) {
+        auto next = [&] { fetch(tile + gridDim.x); };
+        const HookIf<decltype(next)> hook{more && o == lastFft, next};
+        if (op.dir > 0) rr_stages<C, 1, LOGM, 0, LOGE>(v, smrow, t, lo, hi, hook);
+        else rr_stages<C, -1, LOGM, 0, LOGE>(v, smrow, t, lo, hi, hook);
+      } else {
+        if (op.dir > 0) rr_stages<C, 1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
+        else rr_stages<C, -1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
+      }
     }
     if constexpr (!COL) {
       // the row's |psi|^2 in TPR / 32 partials (one when a warp holds several rows)
@@ -268,8 +364,25 @@ struct RrShape {
 constexpr int kRowrSmallLog = 19;
 inline bool rowr_small(Context* ctx) { return ctx->totalQbt < kRowrSmallLog; }
 
+// The constants of the quadratic runs for a kernel of 2^logE amplitudes a thread:
+// 4 c2 TPR^2 k^2 / (4 N) turns, reduced mod 1 before the 64-bit sine and cosine.
+inline void fill_quads(RowProgram& P, int logM, int logE) {
+  const double tpr2 = ldexp(1.0, 2 * (logM - logE)), N = ldexp(1.0, logM);
+  for (int d = 0; d < P.nDiag; ++d) {
+    RowDiag& D = P.diag[d];
+    if (!D.hasQuad) continue;
+    const double q = D.c2 / N;
+    for (int k = 0; k < 1 << logE; ++k) {
+      const double m = tpr2 * (double)(k * k), p = fma(q, m, -rint(q * m));
+      D.quad[k] = make_double2(cos(2.0 * CVDV_PI * p), sin(2.0 * CVDV_PI * p));
+    }
+  }
+}
+
 template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
-static cudaError_t launch_rowr_s(Context* ctx, const void* in, void* out, const RowProgram& P) {
+static cudaError_t launch_rowr_s(Context* ctx, const void* in, void* out, const RowProgram& program) {
+  RowProgram P = program;
+  fill_quads(P, LOGM, LOGE);
   constexpr int NT = 1 << (LOGM - LOGE + LOGR);
   const size_t smem = (size_t)rr_line_slots<C, LOGM, LOGE, LOGR, COL>() * (1 << LOGR) * sizeof(C) + rr_tw_slots(LOGM) * sizeof(double2);
   auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL>;

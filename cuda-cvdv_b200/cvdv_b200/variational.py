@@ -229,8 +229,10 @@ class _GraphPlan:
     sweeps: forward (gates, checkpoints, overlap) and adjoint (gradients)."""
 
     def __init__(self, circ: VariationalCircuit, B: int, psi0_shape, tgt_shape) -> None:
+        # (the plan keeps no reference to the circuit that keeps it: a cycle's graphs
+        # would be destroyed whenever the collector runs, and destroying one while
+        # another plan is captured invalidates that capture)
         dev, cd = "cuda", circ.cdtype
-        self.circ = circ
         self.p = torch.zeros(circ.n_gates, B, dtype=torch.float64, device=dev)
         self.psi0 = torch.zeros(tuple(psi0_shape), dtype=cd, device=dev)
         self.tgt = torch.zeros(tuple(tgt_shape), dtype=cd, device=dev)
@@ -246,18 +248,17 @@ class _GraphPlan:
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
-            self._forward()
-            self._backward()
+            self._forward(circ)
+            self._backward(circ)
         torch.cuda.current_stream().wait_stream(side)
         self.forward_graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.forward_graph):
-            self._forward()
+            self._forward(circ)
         self.backward_graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.backward_graph):
-            self._backward()
+            self._backward(circ)
 
-    def _forward(self) -> None:
-        c = self.circ
+    def _forward(self, c: VariationalCircuit) -> None:
         self.psi.copy_(self.psi0.expand_as(self.psi))
         for g, n in c._steps:
             if g in self.ck:
@@ -265,8 +266,7 @@ class _GraphPlan:
             c._apply_step(self.psi, g, n, self.p)
         self.ov = c._overlap(self.psi, self.tgt)
 
-    def _backward(self) -> None:
-        c = self.circ
+    def _backward(self, c: VariationalCircuit) -> None:
         self.back.copy_(self.psi)
         self.lam.copy_(self.tgt.expand_as(self.lam))
         for g, n in reversed(c._steps):
