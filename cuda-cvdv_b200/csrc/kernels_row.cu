@@ -434,7 +434,7 @@ bool col_program_ok(Context* ctx, int reg) {
       q > rowr_max_log(ctx->precision))
     return false;
   if (ctx->colFft && col_fft_ok(ctx, reg) && tc_col_ok(ctx, reg)) return false;  // chained tensor-core passes
-  const int logE = (ctx->precision == kC64 && q >= 13) ? 5 : 4;
+  const int logE = q >= 13 ? 5 : 4;
   const int logR = q - logE < 8 ? 8 - (q - logE) : (q - logE < 9 ? 1 : 0);
   // (states below the small-state line run one column per CTA)
   // (short registers' surplus thread groups repeat columns)
@@ -1049,6 +1049,7 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
     {
       const int lo = ctx->flw[reg], hi = lo + q;
       bool linOnly = (useC || toRowr) && !regTerms.empty();
+      const bool quads = toRowr && rowr_quads(ctx, q, col);
       int nPl = 0;
       for (const Term& t : regTerms) {
         if (t.kind == kTermFtTw && t.ctrlBit < 0) continue;
@@ -1057,7 +1058,7 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
           ++nPl;
           continue;
         }
-        if (toRowr && t.kind == kTermPoly && t.power == 2 && t.ctrlBit < 0) continue;
+        if (quads && t.kind == kTermPoly && t.power == 2 && t.ctrlBit < 0) continue;
         linOnly = false;
       }
       if (linOnly) {
@@ -1164,7 +1165,7 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
       return false;
     }
     if (rowSums && !col) {
-      const int logE = q < 8 || (q <= 12 && rowr_small(ctx)) ? 3 : (ctx->precision == kC64 && q >= 13) ? 5 : 4;
+      const int logE = q < 8 || (q <= 12 && rowr_small(ctx)) ? 3 : q >= 13 ? 5 : 4;
       const int tpr = 1 << (q - logE);
       P.rowSums = ctx->rowSums;
       ctx->rowSumParts = tpr < 32 ? 1 : tpr / 32;

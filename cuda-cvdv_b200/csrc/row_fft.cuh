@@ -259,4 +259,102 @@ __device__ __forceinline__ void rr_stages(C (&v)[1 << LOGE], C* smrow, int t, co
   }
 }
 
+// ---------------------------------------------------------------- one CTA exchange
+// x[u] *= w^u for u < RAD, w = w_L^e from the tables, the powers as a tree.  w^16 (and
+// w^4 in complex128) come from the tables too: products of w alone multiply its error
+// by u, up to 31 where radix 16 has 15.  Error of a three-layer network on [13, 6]
+// against extended precision: complex128 2.5e-14 with w alone, 1.6e-14 with w^16, 1.1e-14
+// with w^4 and w^16, as with the radix-16 stages (complex64 2.5e-6, 1.7e-6, 2.1e-6).  For radix
+// 32 the upper half is formed as it is applied, so only 17 powers are live at once.
+template <typename C, int DIR, int RAD>
+__device__ __forceinline__ void mul_powers(C (&x)[RAD], const double2* lo, const double2* hi, int e) {
+  constexpr int RT = RAD > 16 ? 16 : RAD;
+  C w[RT + 1];
+#pragma unroll
+  for (int p = 1; p < RT; p <<= 1) {
+    if (p == 1 || (p == 4 && sizeof(C) == 16)) w[p] = tw2<C, DIR>(lo, hi, e * p);
+    else w[p] = cmul(w[p / 2], w[p / 2]);
+#pragma unroll
+    for (int u = 1; u < p; ++u) w[p + u] = cmul(w[p], w[u]);
+  }
+  if constexpr (RAD > 16) w[16] = tw2<C, DIR>(lo, hi, e * 16);
+#pragma unroll
+  for (int u = 1; u < RT; ++u) x[u] = cmul(x[u], w[u]);
+  if constexpr (RAD > 16) {
+    x[16] = cmul(x[16], w[16]);
+#pragma unroll
+    for (int u = 17; u < RAD; ++u) x[u] = cmul(x[u], cmul(w[16], w[u - 16]));
+  }
+}
+
+// Shape of a transform of N = E M points (M = E G threads a row, E amplitudes each)
+// with one exchange across the row's threads and one inside groups of G <= 32 of them:
+//   A  thread tau holds x[tau + M j]; radix E over j, times w_N^{tau k1}: y_k1[tau]
+//   1  y_k1 goes to region k1 of the shared line; group k1's thread g takes y_k1[g + G j]
+//   B  radix E over j, times w_M^{g c}: z_c[g]
+//   2  z_c[g] inside the region; thread g takes z_c for c = g + G i (i < E / G)
+//   C  radix G over g: X[k1 + E (c + E d)]
+// so thread (k1, g) ends with X[tau' + M k], tau' = k1 + E g: the layout it started
+// from, under another thread number.  Only exchange 1 needs the CTA's barriers (one
+// before it is written, one after); exchange 2 is the warp's own, and from one
+// transform's exchange 1 to the next the warps run apart, so one warp's butterflies
+// overlap another's exchange.  The Stockham stages (rr_stages) pass two CTA barriers
+// per exchange, which kept all warps of a row in the same phase ([13, 13] network with
+// 32 amplitudes a thread: complex128 rows 7.95 against 8.39 ms, columns 11.9 against
+// 12.6; complex64 columns 6.5 against 7.4).
+//
+// 2^LOGI lines are interleaved lane by lane (columns); the paddings PAD and RR put the
+// W lanes that one phase of a shared access serves on distinct banks: they are 2^LOGI
+// lines x consecutive g x consecutive k1.
+template <typename C, int LOGM, int LOGE, int LOGI>
+struct RrTwo {
+  static constexpr int LOGG = LOGM - 2 * LOGE;
+  static constexpr bool ok = LOGG >= 0 && LOGG <= LOGE && LOGG + LOGI <= 5;
+  static constexpr int E = 1 << LOGE, G = ok ? 1 << LOGG : 1, M = E * G, W = 128 / (int)sizeof(C), I = 1 << LOGI;
+  static constexpr int PAD = G * I < W ? W / (G * I) : 1;
+  static constexpr int RR0 = M + (PAD * G > E ? PAD * G : E);
+  static constexpr int RR = RR0 + (G < W ? (G - RR0 % W + W) % W : 0);
+  static constexpr int LINE0 = E * RR;
+  static constexpr int LINE = LOGI == 0 ? LINE0 : LINE0 + ((W / I > 1 ? W / I : 1) - LINE0 % W + W) % W;
+};
+
+template <typename C, int DIR, int LOGM, int LOGE, int LOGI, typename H = NoHook>
+__device__ __forceinline__ void rr_two(C (&v)[1 << LOGE], C* line, int t, int& tau, const double2* lo,
+                                       const double2* hi, H after = H()) {
+  using S = RrTwo<C, LOGM, LOGE, LOGI>;
+  constexpr int E = S::E, G = S::G, EG = E / G;
+  bfly<C, DIR, E>(v);
+  mul_powers<C, DIR, E>(v, lo, hi, tau);
+  __syncthreads();  // the line is free: every group has read its last exchange
+  {
+    C* p = line + tau + S::PAD * (tau >> LOGE);
+#pragma unroll
+    for (int k = 0; k < E; ++k) p[k * S::RR] = v[k];
+  }
+  __syncthreads();
+  const int k1 = t >> S::LOGG, g = t & (G - 1);
+  C* reg = line + k1 * S::RR;
+#pragma unroll
+  for (int j = 0; j < E; ++j) v[j] = reg[g + G * j + S::PAD * ((G * j) >> LOGE)];
+  bfly<C, DIR, E>(v);
+  if constexpr (G > 1) {
+    mul_powers<C, DIR, E>(v, lo, hi, g << LOGE);
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < E; ++c) reg[c * (G + 1) + g] = v[c];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < EG; ++i) {
+      C a[G];
+#pragma unroll
+      for (int u = 0; u < G; ++u) a[u] = reg[(g + G * i) * (G + 1) + u];
+      bfly<C, DIR, G>(a);
+#pragma unroll
+      for (int d = 0; d < G; ++d) v[i + EG * d] = a[d];
+    }
+  }
+  tau = k1 + (g << LOGE);
+  after();
+}
+
 }  // namespace cvdv

@@ -37,10 +37,10 @@ struct RowDiag {
   // point n, and terms c x_n (x_n = (n - regC) regDx), each negated when its
   // control bit (a row bit, or none: -1) is set
   int ftSign;
-  int hasQuad;  // k_rowr: the run also has c2 x^2, c2 the sum of its uncontrolled terms
+  int hasQuad;  // k_rowr, 32 amplitudes a thread: the run also has c2 x^2 (uncontrolled terms' sum)
   double c2;
-  double linTurns;           // turns per unit of u = 2 n - N + 1 of the phase x_n: dx / (4 pi)
-  double2 quad[kMaxRowE];    // exp(2 pi i c2 TPR^2 k^2 / N) for the kernel's E amplitudes a thread
+  double linTurns;         // turns per unit of u = 2 n - N + 1 of the phase x_n: dx / (4 pi)
+  double2 quad[kMaxRowE];  // exp(2 pi i c2 TPR^2 k^2 / N) for the kernel's E amplitudes a thread
   int nPl;
   double plC[2];
   int plCtrl[2];
@@ -104,17 +104,19 @@ __device__ __forceinline__ double turns(double q, double m) { return fma(q, m, -
 //   c2 x^2 = c2 u^2 / (4 N),  a x = a dx u / (4 pi),  twiddle = s (N-1) u / (4 N)
 // turns.  From u0 = 2 t - N + 1 a thread's points are u0 + 2 TPR k, so the factor is
 //   [value at u0] [step]^k [exp(2 pi i (4 c2 / 4 N) TPR^2 k^2)]:
-// two sincospi on turns reduced mod 1 without loss, a running product, and (c2 != 0)
-// E constants in the kernel's parameters.  A table entry per amplitude took 16 bytes
-// from L2 for every run (eight times the state's own traffic in a two-mode network
-// layer).  QUADNOTE
-template <typename C, int LOGM, int LOGE>
+// two sincospi on turns reduced mod 1, a running product, and (c2 != 0)
+// E constants in the kernel's parameters.  Runs with a controlled c x^2, a cubic or a
+// qubit term keep a table, and so do quadratic runs on shapes other than rr_quads:
+// the sincospi cost more than the loads with 8 or 16 amplitudes a thread (a 2^8-point
+// register's rotation, displacement and squeeze on a 2^26 complex128 state: 2.38 ms
+// against 1.54 with tables).
+template <typename C, int LOGM, int LOGE, bool QUAD>
 __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uint64_t rowBase, int t) {
   constexpr int E = 1 << LOGE, N = 1 << LOGM, TPR = 1 << (LOGM - LOGE);
   const double2 rs = D.hasRowF ? eval_factor(D.rowF, rowBase) : make_double2(1.0, 0.0);
   // running factor of element t + k TPR: rs times the linear phase, advanced by st per k
   double2 f = rs, st = make_double2(1.0, 0.0);
-  const bool lin = D.nLin || D.nPl || D.ftSign || D.hasQuad;
+  const bool lin = D.nLin || D.nPl || D.ftSign || (QUAD && D.hasQuad);
   if (lin) {
     double a = 0.0;
     for (int l = 0; l < D.nLin; ++l) {
@@ -131,10 +133,9 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
     // s (N-1) u mod 4N in integers: at most 3 2^28 for the runs of a program
     constexpr double inv4N = 1.0 / (4.0 * N);
     const int w = (D.ftSign * (N - 1)) & (4 * N - 1);
-    const double t0 = (double)((int)((long long)w * u0) & (4 * N - 1)) * inv4N;
-    const double t1 = (double)((int)((long long)w * (2 * TPR)) & (4 * N - 1)) * inv4N;
-    double p0 = t0 + turns(a, (double)u0), p1 = t1 + turns(a, 2.0 * TPR);
-    if (D.hasQuad) {
+    double p0 = (double)((int)((long long)w * u0) & (4 * N - 1)) * inv4N + turns(a, (double)u0);
+    double p1 = (double)((int)((long long)w * (2 * TPR)) & (4 * N - 1)) * inv4N + turns(a, 2.0 * TPR);
+    if (QUAD && D.hasQuad) {
       const double q = D.c2 * inv4N;
       p0 += turns(q, (double)u0 * (double)u0);
       p1 += turns(q, 4.0 * TPR * (double)u0);
@@ -160,7 +161,7 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
         v[k0 + k] = cmul(v[k0 + k], fromd<C>(w[k]));
       }
     }
-  } else if (D.hasQuad) {
+  } else if (QUAD && D.hasQuad) {
 #pragma unroll
     for (int k = 0; k < E; ++k) {
       v[k] = cmul(v[k], fromd<C>(dmul(f, D.quad[k])));
@@ -213,25 +214,37 @@ __device__ __forceinline__ void l2_prefetch_tile(const void* p, uint32_t bytes) 
   }
 }
 
-// Tiles of one CTA per SM (more than 256 threads) run persistent: each CTA walks
-// tiles blockIdx.x, + gridDim.x, ...  A row's next tile is asked into L2 before the
-// current one is worked on.  Once the current tile's last shared-memory exchange is
-// read, the exchange buffer is free: the next tile is copied into it asynchronously
-// (one bulk copy for a row, 16- or 8-byte copies for columns) while the last
-// butterflies, the runs after them and the stores go on, and the next tile starts
-// from shared memory.  PFNOTE
-// Smaller tiles run two CTAs per SM, which already overlap one CTA's loads with the
-// other's work; they get one tile per CTA.
-//
-// With COL the "rows" are the columns of a strided register (P.logS amplitudes
-// below it): column c is inner index c mod S and outer index c / S, and element m
-// sits m S amplitudes after its first.  The CTA's 2^LOGR columns (at least two
-// within 512 threads) are adjacent inner indices interleaved lane by lane, so a
-// warp's load covers runs of 2^LOGR amplitudes; the rest of each sector is read
-// from L2 by the CTAs of the neighbouring columns.
+// Whether the shape's transforms run with one CTA exchange (rr_two).  Its results sit
+// in runs of 32 / G points per warp: rows take it where such a run fills a sector
+// (complex64 2^14-point rows store 16-byte pieces with it: 2.33 against 1.63 ms per
+// 2^28 state), and shapes of 8 or 16 amplitudes a thread, which keep tables, read them
+// in short pieces (2^8-point columns 2.23 against 1.54 ms, 2^12-point 3.11 against
+// 2.76; only the 2^7-point shape gains, 1.84 against 2.41).
+template <typename C, int LOGM, int LOGE, int LOGR, bool COL>
+constexpr bool rr_use_two() {
+  using T = RrTwo<C, LOGM, LOGE, COL ? LOGR : 0>;
+  return T::ok && ((LOGE == 5 && (COL || 32 / T::G * sizeof(C) >= 32)) || LOGM == 7);
+}
+// Whether the shape's quadratic runs go without a table: with 32 amplitudes a thread
+// the two sincospi of a run are worth the loads they save, above all after rr_two, whose
+// thread numbering reads a table in short pieces ([13, 13] network, rows / columns:
+// complex128 7.95 / 11.9 ms against 9.1 / 13.2 with tables, complex64 4.4 / 6.5 against
+// 5.6 / 7.1).
+template <typename C, int LOGM, int LOGE, int LOGR, bool COL>
+constexpr bool rr_quads() {
+  return LOGE == 5 && rr_use_two<C, LOGM, LOGE, LOGR, COL>();
+}
+
 template <typename C, int LOGM, int LOGE, int LOGR, bool COL>
 constexpr int rr_line_slots() {
+  using T = RrTwo<C, LOGM, LOGE, COL ? LOGR : 0>;
+  if (rr_use_two<C, LOGM, LOGE, LOGR, COL>()) return T::LINE;
   return COL ? rr_col_slots(LOGM, LOGE, LOGR, (int)sizeof(C)) : rr_row_slots(LOGM, LOGE);
+}
+// whether a CTA has an SM to itself (persistent over its tiles)
+template <typename C, int LOGM, int LOGR, int LOGE>
+constexpr bool rr_one() {
+  return LOGM - LOGE + LOGR > 8 || (sizeof(C) << (LOGM + LOGR)) >= (128u << 10);
 }
 
 // The sum of |psi|^2 (FP64) over the E amplitudes of each of a group of W lanes
@@ -247,17 +260,38 @@ __device__ __forceinline__ void row_sum_part(const C (&v)[E], double* out) {
   if ((threadIdx.x & (W - 1)) == 0) *out = a;
 }
 
+// Tiles of one CTA per SM (rr_one) run persistent: each CTA walks tiles blockIdx.x,
+// + gridDim.x, ...  A row's next tile is asked into L2 before the current one is
+// worked on, so its load finds the data on chip.  A strided tile's loads are 16- or
+// 32-byte pieces that keep the load queue busy: once the current tile's last exchange
+// is read, the line buffer is free and the next tile is copied into it asynchronously
+// while the last runs and the stores go on.  Column programs of the complex128
+// [13, 13] network: 13.5 against 14.8 ms without the copy; copying half of the tile
+// earlier, into a buffer of its own, took 15.1 (the L1 cache it costs holds the
+// tables), and the same copy for rows gained nothing (9.2 against 9.3 ms, complex64
+// 2^14-point rows 1.71 against 1.67).  Smaller tiles run two CTAs per SM, which already
+// overlap one CTA's loads with the other's work; they get one tile per CTA.
+//
+// With COL the "rows" are the columns of a strided register (P.logS amplitudes
+// below it): column c is inner index c mod S and outer index c / S, and element m
+// sits m S amplitudes after its first.  The CTA's 2^LOGR columns (at least two
+// within 512 threads) are adjacent inner indices interleaved lane by lane, so a
+// warp's load covers runs of 2^LOGR amplitudes; the rest of each sector is read
+// from L2 by the CTAs of the neighbouring columns.
 //
 // A state of fewer rows than a CTA holds (nRows < 2^LOGR, both powers of two) runs
 // as one tile whose surplus thread groups repeat its rows: they read the same
 // input and write the same values.
 template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
-__global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR) > 8 ? 1 : 2)
+__global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOGR, LOGE>() ? 1 : 2)
     k_rowr(const C* __restrict__ in, C* __restrict__ out, uint64_t nTiles, const __grid_constant__ RowProgram P) {
   constexpr int E = 1 << LOGE, M = 1 << LOGM, TPR = M >> LOGE, NT = TPR << LOGR;
   constexpr int RS = rr_line_slots<C, LOGM, LOGE, LOGR, COL>();
   constexpr uint32_t TILE_BYTES = (uint32_t)sizeof(C) << (LOGM + LOGR);
-  constexpr bool PF = COL && NT > 256;  // the next tile is copied ahead
+  constexpr bool ONE = rr_one<C, LOGM, LOGR, LOGE>();
+  constexpr int LOGI = COL ? LOGR : 0;
+  constexpr bool TWO = rr_use_two<C, LOGM, LOGE, LOGR, COL>();
+  constexpr bool PF = COL && ONE && TWO;  // the next tile is copied ahead
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
   double2* lo = reinterpret_cast<double2*>(sm + (RS << LOGR));  // w_M^e, e < 64
@@ -308,16 +342,16 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR
       const uint64_t c = (tile << LOGR) + (uint64_t)row;
       rowBase = (c & ((1ull << logS) - 1)) + ((c >> logS) << (LOGM + logS));
     } else {
-      if (NT > 256 && more) l2_prefetch_tile(in + ((tile + gridDim.x) << (LOGM + LOGR)), TILE_BYTES);
+      if (ONE && more) l2_prefetch_tile(in + ((tile + gridDim.x) << (LOGM + LOGR)), TILE_BYTES);
       rowBase = (tile << (LOGM + LOGR)) + ((uint64_t)row << LOGM);
     }
     C v[E];
+    int tau = t;  // v[k] is point tau + k TPR of the row
     if constexpr (PF) {
       cp_async_wait_all();
       __syncthreads();
 #pragma unroll
-      for (int k = 0; k < E; ++k) v[k] = sm[tid + k * NT];
-      __syncthreads();  // the buffer is the exchanges' again
+      for (int k = 0; k < E; ++k) v[k] = sm[tid + k * NT];  // (the exchanges wait for all to be read)
     } else {
 #pragma unroll
       for (int k = 0; k < E; ++k) v[k] = in[rowBase + ((uint64_t)(t + k * TPR) << logS)];
@@ -325,12 +359,17 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR
     for (int o = 0; o < P.nOps; ++o) {
       const RowOp& op = P.ops[o];
       if (op.kind == kRowDiag) {
-        rr_diag<C, LOGM, LOGE>(v, P.diag[op.diag], rowBase, t);
-      } else if constexpr (PF) {
-        auto next = [&] { fetch(tile + gridDim.x); };
-        const HookIf<decltype(next)> hook{more && o == lastFft, next};
-        if (op.dir > 0) rr_stages<C, 1, LOGM, 0, LOGE>(v, smrow, t, lo, hi, hook);
-        else rr_stages<C, -1, LOGM, 0, LOGE>(v, smrow, t, lo, hi, hook);
+        rr_diag<C, LOGM, LOGE, rr_quads<C, LOGM, LOGE, LOGR, COL>()>(v, P.diag[op.diag], rowBase, tau);
+      } else if constexpr (TWO) {
+        auto next = [&] {
+          if constexpr (PF) {
+            __syncthreads();  // every group has read its last exchange
+            fetch(tile + gridDim.x);
+          }
+        };
+        const HookIf<decltype(next)> hook{PF && more && o == lastFft, next};
+        if (op.dir > 0) rr_two<C, 1, LOGM, LOGE, LOGI>(v, smrow, t, tau, lo, hi, hook);
+        else rr_two<C, -1, LOGM, LOGE, LOGI>(v, smrow, t, tau, lo, hi, hook);
       } else {
         if (op.dir > 0) rr_stages<C, 1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
         else rr_stages<C, -1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
@@ -342,18 +381,20 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), (LOGM - LOGE + LOGR
       if (P.rowSums) row_sum_part<C, E, W>(v, P.rowSums + (rowBase >> LOGM) * PARTS + t / 32);
     }
 #pragma unroll
-    for (int k = 0; k < E; ++k) out[rowBase + ((uint64_t)(t + k * TPR) << logS)] = v[k];
+    for (int k = 0; k < E; ++k) out[rowBase + ((uint64_t)(tau + k * TPR) << logS)] = v[k];
   }
 }
 
 // largest row k_rowr takes (one CTA: 2^13 complex128 / 2^14 complex64 points)
 inline int rowr_max_log(int precision) { return precision == kC128 ? 13 : 14; }
 
-// complex64 rows of 2^13 and 2^14 points keep 32 amplitudes per thread (256 / 512
-// threads); everything else 16, and rows shorter than 2^8 points 8
+// Rows of 2^13 and 2^14 points keep 32 amplitudes per thread (256 / 512 threads; two
+// exchanges in shared memory per transform instead of three: complex128 [13, 13] network
+// rows 8.4 against 9.6 ms, columns 12.6 against 13.9), everything else 16, and rows
+// shorter than 2^8 points 8
 template <typename C, int LOGM>
 struct RrShape {
-  static constexpr int LOGE = LOGM < 8 ? 3 : (sizeof(C) == sizeof(float2) && LOGM >= 13) ? 5 : 4;
+  static constexpr int LOGE = LOGM < 8 ? 3 : LOGM >= 13 ? 5 : 4;
   static constexpr int LOGR = LOGM < 8 ? 10 - LOGM : LOGM - LOGE < 8 ? 8 - (LOGM - LOGE) : 0;
 };
 
@@ -382,7 +423,7 @@ inline void fill_quads(RowProgram& P, int logM, int logE) {
 template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
 static cudaError_t launch_rowr_s(Context* ctx, const void* in, void* out, const RowProgram& program) {
   RowProgram P = program;
-  fill_quads(P, LOGM, LOGE);
+  if constexpr (rr_quads<C, LOGM, LOGE, LOGR, COL>()) fill_quads(P, LOGM, LOGE);
   constexpr int NT = 1 << (LOGM - LOGE + LOGR);
   const size_t smem = (size_t)rr_line_slots<C, LOGM, LOGE, LOGR, COL>() * (1 << LOGR) * sizeof(C) + rr_tw_slots(LOGM) * sizeof(double2);
   auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL>;
@@ -396,7 +437,7 @@ static cudaError_t launch_rowr_s(Context* ctx, const void* in, void* out, const 
   }
   uint64_t nTiles = ctx->size() >> (LOGM + LOGR);
   if (nTiles < 1) nTiles = 1;
-  uint64_t grid = NT > 256 ? (uint64_t)ctx->numSMs * resident : nTiles;
+  uint64_t grid = rr_one<C, LOGM, LOGR, LOGE>() ? (uint64_t)ctx->numSMs * resident : nTiles;
   if (grid > nTiles) grid = nTiles;
   kern<<<(unsigned)grid, NT, smem, ctx->stream>>>((const C*)in, (C*)out, nTiles, P);
   return cudaGetLastError();
@@ -406,7 +447,7 @@ template <typename C, int LOGM, bool COL>
 static cudaError_t launch_rowr_t(Context* ctx, const void* in, void* out, const RowProgram& P) {
   constexpr int LOGE = RrShape<C, LOGM>::LOGE, LOGR0 = RrShape<C, LOGM>::LOGR;
   // column form: at least two columns a CTA while it stays within 512 threads
-  constexpr int LOGR = (COL && LOGR0 == 0 && (LOGM - LOGE) < 9) ? 1 : LOGR0;
+  constexpr int LOGR = (COL && LOGR0 == 0 && (sizeof(C) << LOGM) < (128u << 10)) ? 1 : LOGR0;
   if constexpr (LOGM >= 8 && LOGM <= 12) {
     if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, 0, 3, COL>(ctx, in, out, P);
   }
@@ -430,6 +471,13 @@ cudaError_t launch_rowr(Context* ctx, const void* in, void* out, const RowProgra
       if constexpr (sizeof(C) == sizeof(float2)) return launch_rowr_t<C, 14, COL>(ctx, in, out, P);
       return cudaErrorInvalidValue;
   }
+}
+
+// the host's view of rr_quads for a 2^q-point register
+inline bool rowr_quads(Context* ctx, int q, bool col) {
+  if (ctx->precision == kC128) return q == 13 && (col ? rr_quads<double2, 13, 5, 0, true>() : rr_quads<double2, 13, 5, 0, false>());
+  if (q == 13) return col ? rr_quads<float2, 13, 5, 1, true>() : rr_quads<float2, 13, 5, 0, false>();
+  return q == 14 && (col ? rr_quads<float2, 14, 5, 0, true>() : rr_quads<float2, 14, 5, 0, false>());
 }
 
 extern template cudaError_t launch_rowr<double2, false>(Context*, const void*, void*, const RowProgram&, int);
