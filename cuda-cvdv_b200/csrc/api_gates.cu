@@ -320,7 +320,7 @@ CVDVContext* cvdvCreateEx(int numReg, int* numQubits, int precision) {
   size_t cap = 16ull << 20;
   if (cudaMalloc((void**)&c->arena, cap) == cudaSuccess) c->arenaCap = cap;
   else cudaGetLastError();
-  if (!cuda_ok(c, cudaHostAlloc((void**)&c->waitErr, 64, cudaHostAllocMapped), "cvdvCreate wait flag")) {
+  if (!cuda_ok(c, cudaHostAlloc((void**)&c->waitErr, Context::kPinnedBytes, cudaHostAllocMapped), "cvdvCreate wait flag")) {
     c->waitErr = nullptr;
     c->numReg = 0;
     return ctx;
@@ -433,15 +433,7 @@ void cvdvInitFromSeparable(CVDVContext* ctx, void** devicePtrs, int numReg) {
       }
       c->factorsCap = totalN;
     }
-    size_t off = 0;
-    for (int r = 0; r < numReg; ++r) {
-      size_t N = (size_t)1 << c->q[r];
-      if (!cuda_ok(c, cudaMemcpyAsync(c->factors + off, devicePtrs[r], N * sizeof(double2),
-                                      cudaMemcpyDefault, c->stream),
-                   "cvdvInitFromSeparable copy"))
-        return;
-      off += N;
-    }
+    if (!copy_register_arrays(c, devicePtrs, c->factors, "cvdvInitFromSeparable copy")) return;
     c->productPending = true;
     c->initialized = true;
     return;
@@ -449,16 +441,12 @@ void cvdvInitFromSeparable(CVDVContext* ctx, void** devicePtrs, int numReg) {
   arena_reset(c);
   double2* base = (double2*)arena_alloc(c, totalN * sizeof(double2));
   if (!base) return;
+  if (!copy_register_arrays(c, devicePtrs, base, "cvdvInitFromSeparable copy")) return;
   std::vector<const double2*> arrs(numReg);
   size_t off = 0;
   for (int r = 0; r < numReg; ++r) {
-    size_t N = (size_t)1 << c->q[r];
-    if (!cuda_ok(c, cudaMemcpyAsync(base + off, devicePtrs[r], N * sizeof(double2),
-                                    cudaMemcpyDefault, c->stream),
-                 "cvdvInitFromSeparable copy"))
-      return;
     arrs[r] = base + off;
-    off += N;
+    off += (size_t)1 << c->q[r];
   }
   if (!launch_init_product(c, arrs.data())) return;
   c->initialized = true;

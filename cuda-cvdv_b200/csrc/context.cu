@@ -178,6 +178,8 @@ void* big_scratch(Context* ctx, size_t bytes) {
 
 double* host_scratch(Context* ctx, size_t count) {
   size_t bytes = count * sizeof(double);
+  if (ctx->waitErr && bytes <= Context::kPinnedBytes - Context::kPinnedScratchAt)
+    return (double*)((char*)ctx->waitErr + Context::kPinnedScratchAt);
   if (bytes <= ctx->hostScratchCap) return ctx->hostScratch;
   if (ctx->hostScratch) cudaFreeHost(ctx->hostScratch);
   ctx->hostScratch = nullptr;

@@ -332,6 +332,8 @@ struct Context {
   // Mapped pinned word a kernel sets when a bounded wait on its cluster peers
   // gives up; read on the host after every synchronisation (stream_sync).
   unsigned int* waitErr = nullptr;
+  // The pinned block that holds the wait word serves small readbacks too.
+  static constexpr size_t kPinnedBytes = 64 << 10, kPinnedScratchAt = 256;
 
   uint64_t size() const { return 1ull << totalQbt; }
   void* state() const { return buf[cur]; }
@@ -393,6 +395,7 @@ bool launch_col_fft(Context* ctx, int reg, int dir, const FactorList& pre, const
 bool launch_fft_generic(Context* ctx, const void* in, void* out, void* tmp, uint64_t O,
                         int q, uint64_t S, int dir, int prec);
 bool launch_init_product(Context* ctx, const double2* const* regArrays);
+bool copy_register_arrays(Context* ctx, void* const* arrays, double2* dst, const char* what);
 
 // row programs (kernels_row.cu): FFTs and diagonal runs on the contiguous register
 constexpr int kMaxRowOps = 24;

@@ -511,6 +511,62 @@ __global__ void __launch_bounds__(256) k_init_product(C* __restrict__ st, uint64
   }
 }
 
+// The register arrays of a separable state in one launch: dst holds them back to
+// back (a copy call per register took 5-7 us of host time each).
+struct GatherDesc {
+  int numReg;
+  const double2* src[kMaxRegs];
+  unsigned end[kMaxRegs];  // first element after the register in dst
+};
+__global__ void __launch_bounds__(256) k_gather_arrays(const __grid_constant__ GatherDesc D, double2* __restrict__ dst) {
+  const unsigned total = D.end[D.numReg - 1];
+  for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+    int r = 0;
+    while (i >= D.end[r]) ++r;
+    dst[i] = D.src[r][i - (r ? D.end[r - 1] : 0)];
+  }
+}
+
+// Copies the register arrays (of any memory) to dst, back to back, on the context's
+// stream.  Arrays in this device's memory, 16-byte aligned and of 2^16 elements at
+// most in total (larger ones are the copy engine's), are gathered by one kernel.
+bool copy_register_arrays(Context* ctx, void* const* arrays, double2* dst, const char* what) {
+  const int R = ctx->numReg;
+  GatherDesc D;
+  D.numReg = R;
+  size_t total = 0;
+  bool gather = R > 1;
+  for (int r = 0; r < R; ++r) {
+    total += (size_t)1 << ctx->q[r];
+    gather = gather && total <= (size_t)1 << 16 && ((uintptr_t)arrays[r] & 15) == 0;
+    if (!gather) continue;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, arrays[r]) != cudaSuccess) {
+      cudaGetLastError();
+      gather = false;
+    } else {
+      gather = a.type == cudaMemoryTypeDevice && a.device == ctx->device;
+    }
+    D.src[r] = (const double2*)arrays[r];
+    D.end[r] = (unsigned)total;
+  }
+  if (gather) {
+    {
+      LaunchScope _ls(ctx, kKTable);  // (small inputs of a flush, like its tables)
+      k_gather_arrays<<<grid_for(total, 256, 1), 256, 0, ctx->stream>>>(D, dst);
+    }
+    return cuda_ok(ctx, cudaGetLastError(), what);
+  }
+  size_t off = 0;
+  for (int r = 0; r < R; ++r) {
+    const size_t N = (size_t)1 << ctx->q[r];
+    if (!cuda_ok(ctx, cudaMemcpyAsync(dst + off, arrays[r], N * sizeof(double2), cudaMemcpyDefault, ctx->stream), what))
+      return false;
+    off += N;
+  }
+  return true;
+}
+
 static InitDesc init_desc(Context* ctx, const double2* const* regArrays) {
   int R = ctx->numReg;
   int qLast = ctx->q[R - 1];

@@ -197,14 +197,37 @@ __global__ void __launch_bounds__(256) k_marg_smem(const C* __restrict__ st, uin
     part[(size_t)blockIdx.x * D.outSize + b] = hist[b];
 }
 
-__global__ void k_marg_final(const double* __restrict__ part, int nb, long long outSize,
-                             double* __restrict__ out) {
-  for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b < outSize;
-       b += (long long)gridDim.x * blockDim.x) {
-    double a = 0.0;
-    for (int k = 0; k < nb; ++k) a += part[(size_t)k * outSize + b];
-    out[b] = a;
+// out[b] = sum over the nb blocks' partials, in a fixed order: 32 bins per CTA (x, so
+// a warp reads a run of each block's row), kFinalY threads per bin that each add every
+// kFinalY-th partial, then a fixed tree.  One thread per bin added the partials one
+// after the other (up to 592 dependent adds: 33-66 us however few the bins).
+constexpr int kFinalY = 32;
+__device__ __forceinline__ double final_sum(const double* __restrict__ part, int nb, long long stride, long long b,
+                                            bool ok) {
+  __shared__ double red[kFinalY][33];
+  double a = 0.0;
+  if (ok) {
+#pragma unroll 4
+    for (int k = threadIdx.y; k < nb; k += kFinalY) a += part[(size_t)k * stride + b];
   }
+  red[threadIdx.y][threadIdx.x] = a;
+  __syncthreads();
+#pragma unroll
+  for (int o = kFinalY / 2; o > 0; o >>= 1) {
+    if (threadIdx.y < o) red[threadIdx.y][threadIdx.x] += red[threadIdx.y + o][threadIdx.x];
+    __syncthreads();
+  }
+  return red[0][threadIdx.x];
+}
+
+__global__ void __launch_bounds__(32 * kFinalY) k_marg_final(const double* __restrict__ part, int nb, long long outSize,
+                                                            double* __restrict__ out) {
+  const long long b = (long long)blockIdx.x * 32 + threadIdx.x;
+  const double v = final_sum(part, nb, outSize, b, b < outSize);
+  if (threadIdx.y == 0 && b < outSize) out[b] = v;
+}
+static void launch_marg_final(const double* part, int nb, long long outSize, double* out, cudaStream_t s) {
+  k_marg_final<<<(unsigned)((outSize + 31) / 32), dim3(32, kFinalY), 0, s>>>(part, nb, outSize, out);
 }
 
 // large outputs: global atomics (warp-aggregated when the warp shares a bin)
@@ -361,7 +384,169 @@ static bool marginals_tiled(Context* ctx, const std::vector<std::vector<int>>& o
   }
   {
     LaunchScope _ls(ctx, kKReduce);
-    k_marg_final<<<(P.totalBins + 255) / 256, 256, 0, ctx->stream>>>(part, (int)blocks, P.totalBins, dOut);
+    launch_marg_final(part, (int)blocks, P.totalBins, dOut, ctx->stream);
+  }
+  return cuda_ok(ctx, cudaGetLastError(), "marginal launch");
+}
+
+// Marginals of single registers without atomics: every register is a job, all jobs
+// of a readout share one launch, and a CTA works for one job.  With N = 2^q values
+// and S = 2^s amplitudes below the register:
+//   S >= 32: a value's amplitudes are runs of S; G threads (a CTA, or a warp where a
+//     value has few amplitudes) add a slice of one value's amplitudes;
+//   S < 32:  a thread keeps one position of the inner N S amplitudes (or of a CTA's
+//     256) and adds it over a slice of the outer index; the S neighbours of a value
+//     are added at the end.
+// Either way a CTA's loads are contiguous and each partial has one owner.  The slices
+// of a value are added by k_axis_final in a fixed order.  Binning each amplitude with
+// shared-memory atomics, or with one global atomic past 4096 values, and adding the
+// blocks' partials with one thread per value took 126 us for the four registers of a
+// 2^20 complex128 state ([2, 8, 9, 1], now 29) and 589 us for both of a 2^26 one
+// ([13, 13], now 337: two reads of the state, 330 at the copy rate).
+struct AxisJob {
+  int shift, q;
+  int logG;     // S >= 32: log2 of the threads per value (5 or 8)
+  int slices;   // partials per value
+  int block0;   // first CTA
+  double* dst;  // partial [slice][value], or the output itself with one slice
+};
+struct AxisPlan {
+  int nJobs;
+  AxisJob job[kMargMaxOut];
+};
+
+template <typename C>
+__device__ __forceinline__ double prob_at(const C* __restrict__ st, uint64_t i) {
+  const double2 v = tod<C>(st[i]);
+  return v.x * v.x + v.y * v.y;
+}
+
+template <typename C>
+__global__ void __launch_bounds__(256) k_marg_axis(const C* __restrict__ st, int logTotal,
+                                                  const __grid_constant__ AxisPlan A) {
+  __shared__ double red[256];
+  int jb = 0;
+  while (jb + 1 < A.nJobs && (int)blockIdx.x >= A.job[jb + 1].block0) ++jb;
+  const AxisJob& J = A.job[jb];
+  const uint64_t cta = (uint64_t)((int)blockIdx.x - J.block0);
+  const int tid = threadIdx.x, s = J.shift, q = J.q;
+  double a = 0.0;
+  if (s >= 5) {
+    // unit = (slice, value); its amplitudes u map to ((u >> s) << (s + q)) | j << s | (u mod S)
+    const int G = 1 << J.logG;
+    const uint64_t unit = (cta << (8 - J.logG)) + (uint64_t)(tid >> J.logG);
+    const uint64_t j = unit & ((1ull << q) - 1), k = unit >> q;
+    const uint64_t len = (1ull << (logTotal - q)) / (uint64_t)J.slices, sm = (1ull << s) - 1;
+    const bool ok = k < (uint64_t)J.slices;
+    if (ok) {
+      const uint64_t end = (k + 1) * len;
+#pragma unroll 4
+      for (uint64_t u = k * len + (uint64_t)(tid & (G - 1)); u < end; u += G)
+        a += prob_at(st, ((u & ~sm) << q) | (j << s) | (u & sm));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (G > 32) {
+      if ((tid & 31) == 0) red[tid >> 5] = a;
+      __syncthreads();
+      a = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+    }
+    if (ok && (tid & (G - 1)) == 0) J.dst[unit] = a;
+    return;
+  }
+  // positions of the inner block: a CTA holds 256 of them for one slice, or (shorter
+  // blocks) 256 / P outer values at once
+  const int logP = s + q;
+  if (logP >= 8) {
+    const uint64_t chunks = 1ull << (logP - 8), ch = cta & (chunks - 1), k = cta >> (logP - 8);
+    const uint64_t outer = 1ull << (logTotal - logP), len = outer / (uint64_t)J.slices;
+    const uint64_t pos = (ch << 8) + tid;
+#pragma unroll 4
+    for (uint64_t o = k * len; o < (k + 1) * len; ++o) a += prob_at(st, (o << logP) | pos);
+    for (int o = 1; o < (1 << s); o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if ((tid & ((1 << s) - 1)) == 0) J.dst[(k << q) + (pos >> s)] = a;
+    return;
+  }
+  const uint64_t total = 1ull << logTotal, len = total / (uint64_t)J.slices, end = (cta + 1) * len;
+#pragma unroll 4
+  for (uint64_t i = cta * len + tid; i < end; i += 256) a += prob_at(st, i);
+  red[tid] = a;
+  __syncthreads();
+  if (tid < (1 << q)) {  // value tid: threads whose index has it in bits s .. s + q
+    double b = 0.0;
+    for (int u = 0; u < (256 >> q); ++u) b += red[((u >> s) << logP) | (tid << s) | (u & ((1 << s) - 1))];
+    J.dst[(cta << q) + tid] = b;
+  }
+}
+
+// The slices of every job that has more than one, to their outputs.
+struct AxisFinal {
+  int nJobs;
+  struct {
+    const double* part;
+    double* out;
+    int q, slices, block0;
+  } job[kMargMaxOut];
+};
+__global__ void __launch_bounds__(32 * kFinalY) k_axis_final(const __grid_constant__ AxisFinal A) {
+  int jb = 0;
+  while (jb + 1 < A.nJobs && (int)blockIdx.x >= A.job[jb + 1].block0) ++jb;
+  const long long N = 1ll << A.job[jb].q, b = (long long)((int)blockIdx.x - A.job[jb].block0) * 32 + threadIdx.x;
+  const double v = final_sum(A.job[jb].part, A.job[jb].slices, N, b, b < N);
+  if (threadIdx.y == 0 && b < N) A.job[jb].out[b] = v;
+}
+
+// Marginal of register regs[k] to dOut + pos[k], for all k (at most kMargMaxOut).
+static bool marginals_axis(Context* ctx, const std::vector<int>& regs, const std::vector<size_t>& pos, double* dOut) {
+  AxisPlan A{};
+  AxisFinal F{};
+  const int n = ctx->totalQbt;
+  long long blocks = 0, finals = 0;
+  for (size_t k = 0; k < regs.size(); ++k) {
+    AxisJob& J = A.job[A.nJobs++];
+    const int s = ctx->flw[regs[k]], q = ctx->q[regs[k]], logP = s + q;
+    J.shift = s;
+    J.q = q;
+    // slices: CTAs for eight per SM, while a thread keeps at least four loads
+    const long long want = 8ll * ctx->numSMs;
+    int logSl = 0;
+    long long ctas;
+    if (s >= 5) {
+      J.logG = n - q >= 10 ? 8 : 5;  // a CTA per slice where values have 2^10 amplitudes or more
+      while ((((1ll << q) << logSl) >> (8 - J.logG)) < want && n - q - logSl > J.logG + 2) ++logSl;
+      ctas = (((1ll << q) << logSl) + (256 >> J.logG) - 1) >> (8 - J.logG);
+    } else if (logP >= 8) {
+      while (((1ll << (logP - 8)) << logSl) < want && n - logP - logSl > 2) ++logSl;
+      ctas = (1ll << (logP - 8)) << logSl;
+    } else {
+      while ((1ll << logSl) < want && n - logSl > 10) ++logSl;
+      ctas = 1ll << logSl;
+    }
+    J.slices = 1 << logSl;
+    J.block0 = (int)blocks;
+    blocks += ctas;
+    J.dst = dOut + pos[k];
+    if (logSl == 0) continue;
+    J.dst = (double*)arena_alloc(ctx, ((size_t)1 << (q + logSl)) * sizeof(double));
+    if (!J.dst) return false;
+    auto& f = F.job[F.nJobs++];
+    f.part = J.dst;
+    f.out = dOut + pos[k];
+    f.q = q;
+    f.slices = J.slices;
+    f.block0 = (int)finals;
+    finals += ((1ll << q) + 31) / 32;
+  }
+  {
+    LaunchScope _ls(ctx, kKReduce);
+    if (ctx->precision == kC128)
+      k_marg_axis<double2><<<(unsigned)blocks, 256, 0, ctx->stream>>>((const double2*)ctx->state(), n, A);
+    else
+      k_marg_axis<float2><<<(unsigned)blocks, 256, 0, ctx->stream>>>((const float2*)ctx->state(), n, A);
+  }
+  if (finals) {
+    LaunchScope _ls(ctx, kKReduce);
+    k_axis_final<<<(unsigned)finals, dim3(32, kFinalY), 0, ctx->stream>>>(F);
   }
   return cuda_ok(ctx, cudaGetLastError(), "marginal launch");
 }
@@ -397,13 +582,12 @@ __global__ void __launch_bounds__(256) k_row_marg(const double* __restrict__ tot
   if (threadIdx.x == 0) out[blockIdx.x] = s.x;
 }
 
-static bool marginals_from_rows(Context* ctx, const std::vector<std::vector<int>>& outs, int parts, double* dOut) {
+static bool marginals_from_rows(Context* ctx, const std::vector<int>& regs, int parts, double* dOut) {
   const int last = ctx->numReg - 1;
   const uint64_t rows = ctx->size() >> ctx->q[last];
   RowMarg M{};
   int bins = 0;
-  for (const auto& regs : outs) {
-    const int r = regs[0];
+  for (int r : regs) {
     M.shift[M.nOut] = ctx->flw[r] - ctx->q[last];
     M.q[M.nOut] = ctx->q[r];
     M.off[M.nOut++] = bins;
@@ -425,10 +609,10 @@ static bool marginals_from_rows(Context* ctx, const std::vector<std::vector<int>
 
 // Ask the next flush for row sums when every register read is a single register
 // above the last one; false (nothing asked) otherwise.
-static bool request_row_sums(Context* c, const std::vector<std::vector<int>>& outs) {
-  if (c->numReg < 2 || outs.empty()) return false;
-  for (const auto& regs : outs)
-    if (regs.size() != 1 || regs[0] == c->numReg - 1) return false;
+static bool request_row_sums(Context* c, const std::vector<int>& regs) {
+  if (c->numReg < 2) return false;
+  for (int r : regs)
+    if (r == c->numReg - 1) return false;
   const size_t need = (c->size() >> c->q[c->numReg - 1]) * kRowSumMaxParts;
   if (need > c->rowSumCap) {
     cudaStreamSynchronize(c->stream);
@@ -482,10 +666,9 @@ static bool marginal_device(Context* ctx, const int* regs, int nr, double** dOut
         LaunchScope _ls(ctx, kKReduce);
         k_marg_smem<float2><<<blocks, 256, smem, ctx->stream>>>((const float2*)ctx->state(), n, D, part);
       }
-    int fb = (int)((stride + 255) / 256);
     {
       LaunchScope _ls(ctx, kKReduce);
-      k_marg_final<<<fb, 256, 0, ctx->stream>>>(part, blocks, stride, out);
+      launch_marg_final(part, blocks, stride, out, ctx->stream);
     }
   } else {
     if (!cuda_ok(ctx, cudaMemsetAsync(out, 0, (size_t)stride * sizeof(double), ctx->stream), "memset"))
@@ -594,6 +777,30 @@ double cvdvGetNorm(CVDVContext* ctx) {
   return ok ? r.x : 0.0;
 }
 
+// Doubles at src[at .. at + count) of a device buffer to host memory `to`.
+struct HostPart {
+  double* to;
+  size_t at, count;
+};
+// Waits for the parts of a device buffer of `total` doubles: small buffers come back
+// in one copy to pinned memory (a copy per register to pageable memory took 10 us
+// each), large ones straight to their places.
+static bool read_back(Context* c, const std::vector<HostPart>& parts, const double* src, size_t total, const char* what) {
+  constexpr size_t kSmall = 1 << 17;
+  double* hs = total <= kSmall ? host_scratch(c, total) : nullptr;
+  if (hs) {
+    if (!cuda_ok(c, cudaMemcpyAsync(hs, src, total * sizeof(double), cudaMemcpyDeviceToHost, c->stream), what) ||
+        !stream_sync(c, what))
+      return false;
+    for (const HostPart& p : parts) memcpy(p.to, hs + p.at, p.count * sizeof(double));
+    return true;
+  }
+  for (const HostPart& p : parts)
+    if (!cuda_ok(c, cudaMemcpyAsync(p.to, src + p.at, p.count * sizeof(double), cudaMemcpyDeviceToHost, c->stream), what))
+      return false;
+  return stream_sync(c, what);
+}
+
 static bool measure(Context* c, const int* regIdxs, int numRegs, double* probsOut, const char* w) {
   if (!regIdxs || numRegs <= 0 || !probsOut) {
     set_error(c, kErrInvalidArg, "%s: empty register list", w);
@@ -614,16 +821,16 @@ static bool measure(Context* c, const int* regIdxs, int numRegs, double* probsOu
   for (int s = 0; s < numRegs; ++s) bins <<= c->q[regIdxs[s]];
   double* dOut;
   long long outSize = bins;
-  if (tiled_ok(c, bins)) {
+  if (numRegs == 1) {
+    dOut = (double*)arena_alloc(c, (size_t)bins * sizeof(double));
+    if (!dOut || !marginals_axis(c, {regIdxs[0]}, {0}, dOut)) return false;
+  } else if (tiled_ok(c, bins)) {
     dOut = (double*)arena_alloc(c, (size_t)bins * sizeof(double));
     if (!dOut || !marginals_tiled(c, {std::vector<int>(regIdxs, regIdxs + numRegs)}, dOut)) return false;
   } else if (!marginal_device(c, regIdxs, numRegs, &dOut, &outSize)) {
     return false;
   }
-  if (!cuda_ok(c, cudaMemcpyAsync(probsOut, dOut, (size_t)outSize * sizeof(double),
-                                  cudaMemcpyDeviceToHost, c->stream), "marginal copy"))
-    return false;
-  return stream_sync(c, "marginal sync");
+  return read_back(c, {{probsOut, 0, (size_t)outSize}}, dOut, (size_t)outSize, "marginal");
 }
 
 void cvdvMeasureMultiple(CVDVContext* ctx, const int* regIdxs, int numRegs, double* probsOut) {
@@ -649,49 +856,61 @@ void cvdvMeasureEach(CVDVContext* ctx, const int* regIdxs, int numRegs, double* 
       set_error(c, kErrInvalidArg, "%s: invalid register index %d", w, regIdxs[k]);
       return;
     }
-  // registers whose marginals fit the shared histogram go in one pass; larger
-  // ones are read one at a time
-  std::vector<std::vector<int>> outs;
-  std::vector<size_t> outPos, bigPos;
-  std::vector<int> big;
-  size_t off = 0;
-  long long tiledBins = 0;
-  for (int k = 0; k < numRegs; ++k) {
-    const long long b = 1ll << c->q[regIdxs[k]];
-    if (tiled_ok(c, tiledBins + b)) {
-      outs.push_back({regIdxs[k]});
-      outPos.push_back(off);
-      tiledBins += b;
-    } else {
-      big.push_back(regIdxs[k]);
-      bigPos.push_back(off);
-    }
-    off += (size_t)b;
-  }
-  for (size_t k = 0; k < big.size(); ++k)
-    if (!measure(c, &big[k], 1, probsOut + bigPos[k], w)) return;
-  if (outs.empty()) return;
+  const std::vector<int> regs(regIdxs, regIdxs + numRegs);
   // qubit registers after a row program on the last register: the program writes
   // the row sums on its way out and the marginals come from them, not another pass
-  const bool asked = request_row_sums(c, outs);
+  const bool asked = request_row_sums(c, regs);
   const bool ok = ready(c, w);
   c->rowSums = nullptr;
   if (!ok) return;
   const int parts = asked ? c->rowSumParts : 0;
   c->rowSumParts = 0;
   arena_reset(c);
-  double* dOut = (double*)arena_alloc(c, (size_t)tiledBins * sizeof(double));
-  if (!dOut) return;
-  if (!(parts > 0 ? marginals_from_rows(c, outs, parts, dOut) : marginals_tiled(c, outs, dOut))) return;
-  size_t src = 0;
-  for (size_t k = 0; k < outs.size(); ++k) {
-    const size_t b = (size_t)1 << c->q[outs[k][0]];
-    if (!cuda_ok(c, cudaMemcpyAsync(probsOut + outPos[k], dOut + src, b * sizeof(double),
-                                    cudaMemcpyDeviceToHost, c->stream), "marginal copy"))
-      return;
-    src += b;
+  // device order: the registers read by one pass of tiles first (several registers
+  // above the tile, one block sum per tile serves them all), then the others
+  std::vector<int> tiled, axis;
+  long long tiledBins = 0;
+  for (int k = 0; k < numRegs; ++k) {
+    const long long b = 1ll << c->q[regs[k]];
+    if (parts > 0 || (c->flw[regs[k]] >= kMargLogTile && tiled_ok(c, tiledBins + b))) {
+      tiled.push_back(k);
+      tiledBins += b;
+    } else {
+      axis.push_back(k);
+    }
   }
-  stream_sync(c, "marginal sync");
+  if (parts == 0 && tiled.size() < 2) {
+    axis.insert(axis.begin(), tiled.begin(), tiled.end());
+    tiled.clear();
+  }
+  std::vector<size_t> hostPos(numRegs);
+  size_t total = 0;
+  for (int k = 0; k < numRegs; ++k) {
+    hostPos[k] = total;
+    total += (size_t)1 << c->q[regs[k]];
+  }
+  double* dOut = (double*)arena_alloc(c, total * sizeof(double));
+  if (!dOut) return;
+  std::vector<HostPart> host;
+  size_t at = 0;
+  std::vector<std::vector<int>> outs;
+  std::vector<int> first, rest;
+  std::vector<size_t> restPos;
+  for (int k : tiled) {
+    first.push_back(regs[k]);
+    outs.push_back({regs[k]});
+    host.push_back({probsOut + hostPos[k], at, (size_t)1 << c->q[regs[k]]});
+    at += host.back().count;
+  }
+  for (int k : axis) {
+    rest.push_back(regs[k]);
+    restPos.push_back(at);
+    host.push_back({probsOut + hostPos[k], at, (size_t)1 << c->q[regs[k]]});
+    at += host.back().count;
+  }
+  if (!first.empty() && !(parts > 0 ? marginals_from_rows(c, first, parts, dOut) : marginals_tiled(c, outs, dOut))) return;
+  if (!rest.empty() && !marginals_axis(c, rest, restPos, dOut)) return;
+  read_back(c, host, dOut, total, "marginal");
 }
 
 void cvdvGetFidelity(CVDVContext* ctx, void** devicePtrs, int numReg, double* fidOut) {
@@ -713,15 +932,12 @@ void cvdvGetFidelity(CVDVContext* ctx, void** devicePtrs, int numReg, double* fi
   for (int r = 0; r < numReg; ++r) totalN += (size_t)1 << c->q[r];
   double2* base = (double2*)arena_alloc(c, totalN * sizeof(double2));
   if (!base) return;
+  if (!copy_register_arrays(c, devicePtrs, base, "cvdvGetFidelity copy")) return;
   std::vector<const double2*> arrs(numReg);
   size_t off = 0;
   for (int r = 0; r < numReg; ++r) {
-    size_t N = (size_t)1 << c->q[r];
-    if (!cuda_ok(c, cudaMemcpyAsync(base + off, devicePtrs[r], N * sizeof(double2), cudaMemcpyDefault,
-                                    c->stream), "cvdvGetFidelity copy"))
-      return;
     arrs[r] = base + off;
-    off += N;
+    off += (size_t)1 << c->q[r];
   }
   // outer product of all registers but the last (same helper as the initialiser)
   int R = c->numReg, qLast = c->q[R - 1];
@@ -1006,7 +1222,7 @@ extern "C" int cvdvMeasureMultipleNoAlloc(const void* state, int precision, cons
   }
   {
     LaunchScope _ls(nullptr, kKReduce);
-    k_marg_final<<<(int)((bins + 255) / 256), 256, 0, s>>>(scratch, blocks, bins, probsOut);
+    launch_marg_final(scratch, blocks, bins, probsOut, s);
   }
   e = cudaPeekAtLastError();
   if (e != cudaSuccess && e != before) {
