@@ -267,6 +267,7 @@ extern "C" {
 CVDVContext* cvdvCreateEx(int numReg, int* numQubits, int precision) {
   CVDVContext* ctx = new (std::nothrow) CVDVContext();
   if (!ctx) return nullptr;
+  host_copy_context_made();
   Context* c = C(ctx);
   if (numReg <= 0 || numQubits == nullptr) return ctx;  // empty context (context.cu:10-12)
   if (numReg > kMaxRegs) {
@@ -383,6 +384,7 @@ void cvdvDestroy(CVDVContext* ctx) {
   release(c);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete ctx;
+  host_copy_context_gone();
 }
 
 void cvdvFree(CVDVContext* ctx) {

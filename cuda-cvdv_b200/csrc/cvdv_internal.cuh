@@ -365,6 +365,11 @@ void* arena_alloc(Context* ctx, size_t bytes);   // reset per flush / readout
 void arena_reset(Context* ctx);
 void* big_scratch(Context* ctx, size_t bytes);   // persistent, grown on demand
 double* host_scratch(Context* ctx, size_t count);
+// Copies device memory to host memory and waits for it (host_copy.cu); contexts count
+// themselves there for the staging memory's lifetime.
+bool copy_to_host(Context* ctx, void* dst, const void* src, size_t bytes, const char* what);
+void host_copy_context_made();
+void host_copy_context_gone();
 bool ensure_state(Context* ctx);                  // allocate both buffers
 bool flush(Context* ctx);                         // run pending stages
 // scratch address of cvdvMeasureMultipleNoAlloc on device dev (current), with its

@@ -449,10 +449,7 @@ static void husimi_wigner_route(Context* c, int r, double* husimiOut) {
     LaunchScope _ls(c, kKPhaseSpace);
     k_real_clamp<<<gblocks(NN), 256, 0, c->stream>>>(Wc, NN, (double)NN, dOut);
   }
-  if (!cuda_ok(c, cudaMemcpyAsync(husimiOut, dOut, NN * sizeof(double), cudaMemcpyDeviceToHost,
-                                  c->stream), "husimi copy"))
-    return;
-  stream_sync(c, "husimi sync");
+  copy_to_host(c, husimiOut, dOut, NN * sizeof(double), "husimi copy");
 }
 
 static void husimi_overlap_route(Context* c, int r, double* husimiOut) {
@@ -490,10 +487,7 @@ static void husimi_overlap_route(Context* c, int r, double* husimiOut) {
       e = husimi_rows(c, q, Psi, G, S, dOut);
     }
     if (!cuda_ok(c, e, "husimi launch")) return;
-    if (!cuda_ok(c, cudaMemcpyAsync(husimiOut, dOut, NN * sizeof(double), cudaMemcpyDeviceToHost, c->stream),
-                 "husimi copy"))
-      return;
-    stream_sync(c, "husimi sync");
+    copy_to_host(c, husimiOut, dOut, NN * sizeof(double), "husimi copy");
     return;
   }
   // longer registers: the circulant in chunks of slices, transformed by the pass kernel
@@ -544,10 +538,7 @@ static void husimi_overlap_route(Context* c, int r, double* husimiOut) {
     k_husimi_finalize<<<gblocks(NN), 256, 0, c->stream>>>(acc, N, dOut);
   }
   if (!cuda_ok(c, cudaGetLastError(), "husimi launch")) return;
-  if (!cuda_ok(c, cudaMemcpyAsync(husimiOut, dOut, NN * sizeof(double), cudaMemcpyDeviceToHost,
-                                  c->stream), "husimi copy"))
-    return;
-  stream_sync(c, "husimi sync");
+  copy_to_host(c, husimiOut, dOut, NN * sizeof(double), "husimi copy");
 }
 
 // The reference chooses the Wigner route when the overlap route's buffers would
@@ -574,10 +565,7 @@ void cvdvGetWigner(CVDVContext* ctx, int regIdx, double* wignerOut) {
   if (!work) return;
   double* dOut = (double*)(work + 3 * NN);
   if (!wigner_device(c, regIdx, dOut, nullptr, work)) return;
-  if (!cuda_ok(c, cudaMemcpyAsync(wignerOut, dOut, NN * sizeof(double), cudaMemcpyDeviceToHost,
-                                  c->stream), "wigner copy"))
-    return;
-  stream_sync(c, "wigner sync");
+  copy_to_host(c, wignerOut, dOut, NN * sizeof(double), "wigner copy");
 }
 
 void cvdvGetHusimiQ(CVDVContext* ctx, int regIdx, double* husimiOut) {

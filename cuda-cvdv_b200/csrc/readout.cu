@@ -721,6 +721,34 @@ __global__ void k_split(const C* __restrict__ st, uint64_t off, uint64_t cnt, do
 // ====================================================================== C API
 static Context* C(CVDVContext* p) { return static_cast<Context*>(p); }
 
+// Doubles at src[at .. at + count) of a device buffer to host memory `to`.
+struct HostPart {
+  double* to;
+  size_t at, count;
+};
+// Waits for the parts of a device buffer of `total` doubles: small buffers come back
+// in one copy to the context's pinned block (a copy per register to pageable memory
+// took 10 us each), large parts through copy_to_host.
+static bool read_back(Context* c, const std::vector<HostPart>& parts, const double* src, size_t total, const char* what) {
+  constexpr size_t kSmall = (Context::kPinnedBytes - Context::kPinnedScratchAt) / sizeof(double);
+  constexpr size_t kLarge = (2u << 20) / sizeof(double);
+  double* hs = total <= kSmall ? host_scratch(c, total) : nullptr;
+  if (hs) {
+    if (!cuda_ok(c, cudaMemcpyAsync(hs, src, total * sizeof(double), cudaMemcpyDeviceToHost, c->stream), what) ||
+        !stream_sync(c, what))
+      return false;
+    for (const HostPart& p : parts) memcpy(p.to, hs + p.at, p.count * sizeof(double));
+    return true;
+  }
+  for (const HostPart& p : parts) {
+    const bool ok = p.count >= kLarge ? copy_to_host(c, p.to, src + p.at, p.count * sizeof(double), what)
+                                      : cuda_ok(c, cudaMemcpyAsync(p.to, src + p.at, p.count * sizeof(double),
+                                                                   cudaMemcpyDeviceToHost, c->stream), what);
+    if (!ok) return false;
+  }
+  return stream_sync(c, what);
+}
+
 static bool ready(Context* c, const char* what) {
   if (c->numReg == 0 || !c->initialized) {
     set_error(c, kErrNotInitialized, "%s: state not initialised", what);
@@ -740,9 +768,9 @@ void cvdvGetState(CVDVContext* ctx, double* realOut, double* imagOut) {
   uint64_t n = c->size();
   const uint64_t chunk = 1ull << 22;
   uint64_t cnt0 = n < chunk ? n : chunk;
-  double* dre = (double*)arena_alloc(c, cnt0 * sizeof(double));
-  double* dim = (double*)arena_alloc(c, cnt0 * sizeof(double));
-  if (!dre || !dim) return;
+  double* dre = (double*)arena_alloc(c, 2 * cnt0 * sizeof(double));
+  if (!dre) return;
+  double* dim = dre + cnt0;
   for (uint64_t off = 0; off < n; off += chunk) {
     uint64_t cnt = n - off < chunk ? n - off : chunk;
     int blocks = (int)((cnt + 255) / 256 < 1184 ? (cnt + 255) / 256 : 1184);
@@ -756,13 +784,11 @@ void cvdvGetState(CVDVContext* ctx, double* realOut, double* imagOut) {
         LaunchScope _ls(ctx, kKReduce);
         k_split<float2><<<blocks, 256, 0, c->stream>>>((const float2*)c->state(), off, cnt, dre, dim);
       }
-    if (!cuda_ok(c, cudaMemcpyAsync(realOut + off, dre, cnt * sizeof(double), cudaMemcpyDeviceToHost,
-                                    c->stream), "getState copy re") ||
-        !cuda_ok(c, cudaMemcpyAsync(imagOut + off, dim, cnt * sizeof(double), cudaMemcpyDeviceToHost,
-                                    c->stream), "getState copy im"))
+    // (waits, so the next chunk may overwrite the split arrays)
+    if (!read_back(c, {{realOut + off, 0, (size_t)cnt}, {imagOut + off, (size_t)cnt0, (size_t)cnt}}, dre, 2 * (size_t)cnt0,
+                   "getState copy"))
       return;
   }
-  stream_sync(c, "getState sync");
 }
 
 double cvdvGetNorm(CVDVContext* ctx) {
@@ -775,30 +801,6 @@ double cvdvGetNorm(CVDVContext* ctx) {
                 ? reduce(c, OpNorm<double2>{(const double2*)c->state()}, c->size(), &r)
                 : reduce(c, OpNorm<float2>{(const float2*)c->state()}, c->size(), &r);
   return ok ? r.x : 0.0;
-}
-
-// Doubles at src[at .. at + count) of a device buffer to host memory `to`.
-struct HostPart {
-  double* to;
-  size_t at, count;
-};
-// Waits for the parts of a device buffer of `total` doubles: small buffers come back
-// in one copy to pinned memory (a copy per register to pageable memory took 10 us
-// each), large ones straight to their places.
-static bool read_back(Context* c, const std::vector<HostPart>& parts, const double* src, size_t total, const char* what) {
-  constexpr size_t kSmall = 1 << 17;
-  double* hs = total <= kSmall ? host_scratch(c, total) : nullptr;
-  if (hs) {
-    if (!cuda_ok(c, cudaMemcpyAsync(hs, src, total * sizeof(double), cudaMemcpyDeviceToHost, c->stream), what) ||
-        !stream_sync(c, what))
-      return false;
-    for (const HostPart& p : parts) memcpy(p.to, hs + p.at, p.count * sizeof(double));
-    return true;
-  }
-  for (const HostPart& p : parts)
-    if (!cuda_ok(c, cudaMemcpyAsync(p.to, src + p.at, p.count * sizeof(double), cudaMemcpyDeviceToHost, c->stream), what))
-      return false;
-  return stream_sync(c, what);
 }
 
 static bool measure(Context* c, const int* regIdxs, int numRegs, double* probsOut, const char* w) {
