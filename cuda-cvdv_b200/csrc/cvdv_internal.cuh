@@ -235,11 +235,13 @@ struct TableJob {
 };
 
 // What a flush will launch.  Planning allocates tables and fixes every kernel's
-// parameters (the ping-pong buffers alternate as the launches are planned); then
-// all tables are built by one launch and the planned launches run in order.
+// parameters (the ping-pong buffers alternate as the launches are planned).  The
+// planned launches go out in groups, each after one launch that builds its tables.
 struct FlushPlan {
   std::vector<TableJob> tables;
   std::vector<std::function<bool()>> launches;
+  size_t group = 1;      // launches that make the next group
+  int cur = 0;           // the buffer that holds the state after the groups that went out
 };
 
 struct Context {
