@@ -522,6 +522,214 @@ __global__ void __launch_bounds__(BPair<LOGQ>::TPR, 1)
   cl.sync();
 }
 
+// ---------------------------------------------------------------- runs of layers
+// A run of layers Rx(theta) . cd(beta) on up to three qubits above the mode in one
+// launch.  An instance is 2^(n - q) <= 8 rows: a cluster of as many CTAs holds them, one
+// row each, for the whole run, so a layer passes no global memory and no launch; the
+// Rx reads the partner row (the row index with the layer's bit flipped) from the
+// partner's shared memory.  The centred transform's twiddles exp(i theta_j) at the end
+// of one layer and exp(-i theta_j) at the start of the next commute with the Rx (all
+// rows have the same ones) and cancel: they are applied at the run's ends only.  A
+// step of its own (k_b_rxcd) takes 8-10 us however small the row, most of it launch,
+// cluster set-up, twiddle tables and the state's way through memory.  Forward / adjoint
+// sweep of 64 sets x 40 layers, a launch per layer -> per 8 layers (checkpoints every 16
+// gates): complex64 [1, 12] 381 / 629 -> 258 / 489 us, complex128 518 / 894 -> 368 / 742,
+// complex64 [1, 10] 295 / 534 -> 148 / 234.  [1, 12] with the Stockham stages instead of
+// rr_two: 269 / 501.
+//
+// A cluster barrier has two halves: a CTA arrives once it has read its partner's row
+// and waits for the others' arrival only where its own line is written again.
+constexpr int kMaxLayers = 64;  // layers of one launch
+struct LayerBits {
+  int nLayers;
+  signed char bit[kMaxLayers];  // the layer's qubit as a bit of the row index
+};
+
+template <int LOGQ>
+struct BLayer {
+  static constexpr int N = 1 << LOGQ, TPR = N >> 4;
+  // a row's shared line (rr_two's, at least the row itself)
+  template <typename C>
+  static constexpr int line() {
+    static_assert(RrTwo<C, LOGQ, 4, 0>::ok && RrTwo<C, LOGQ, 4, 0>::LINE >= N, "row line");
+    return RrTwo<C, LOGQ, 4, 0>::LINE;
+  }
+};
+
+__device__ __forceinline__ void layer_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void layer_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// v[k] *= f st^k
+template <typename C>
+__device__ __forceinline__ void mul_run(C (&v)[16], double2 f, double2 st) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    v[k] = cmul(v[k], fromd<C>(f));
+    f = dmul(f, st);
+  }
+}
+
+template <typename C, int LOGQ>
+__global__ void __launch_bounds__(BLayer<LOGQ>::TPR, 1)
+    k_b_layers(C* __restrict__ st, int logRows, int batch, const double* __restrict__ par,
+               const __grid_constant__ LayerBits A) {
+  using G = BLayer<LOGQ>;
+  constexpr int N = G::N, TPR = G::TPR;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C* sm = reinterpret_cast<C*>(smraw);
+  double2* lo = reinterpret_cast<double2*>(sm + G::template line<C>());
+  double2* hi = lo + 64;
+  cg::cluster_group cl = cg::this_cluster();
+  const int r = (int)cl.block_rank(), t = threadIdx.x;
+  const int b = (int)(blockIdx.x >> logRows);
+  C* rowp = st + ((uint64_t)blockIdx.x << LOGQ);
+  C v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = rowp[t + k * TPR];
+  b_fill_twiddles<LOGQ>(lo, t, TPR);
+  const double2 tws = ft_twiddle_step(TPR, N, 1);
+  mul_run(v, ft_twiddle(t, N, 1), tws);
+  __syncthreads();  // the twiddle tables
+  int tau = t;      // v[k] is point tau + k TPR; the partner's thread t holds the same points
+  for (int l = 0; l < A.nLayers; ++l) {
+    const int bit = A.bit[l];
+    const double th = __ldg(par + (size_t)(2 * l) * batch + b), be = __ldg(par + (size_t)(2 * l + 1) * batch + b);
+    // Rx: v <- c v - i s w with w the partner row's amplitude at the same point
+    if (l) __syncthreads();  // the transform's last exchange is read
+#pragma unroll
+    for (int k = 0; k < 16; ++k) sm[t + k * TPR] = v[k];
+    layer_arrive();
+    double s, c;
+    sincos(0.5 * th, &s, &c);
+    const double coef = be * (-M_SQRT2) * (((r >> bit) & 1) ? -1.0 : 1.0);
+    layer_wait();
+    {
+      const C* pw = cl.map_shared_rank(sm, r ^ (1 << bit));
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const double2 x = tod_b(v[k]), y = tod_b(pw[t + k * TPR]);
+        v[k] = fromd<C>(make_double2(c * x.x + s * y.y, c * x.y - s * y.x));
+      }
+    }
+    layer_arrive();
+    layer_wait();  // the partner has read this row
+    rr_two<C, 1, LOGQ, 4, 0>(v, sm, t, tau, lo, hi);
+    mul_run(v, b_kick(tau, N, coef), b_kick_step(TPR, N, coef));
+    rr_two<C, -1, LOGQ, 4, 0>(v, sm, t, tau, lo, hi);
+  }
+  mul_run(v, cconj(ft_twiddle(tau, N, 1)), cconj(tws));
+#pragma unroll
+  for (int k = 0; k < 16; ++k) rowp[tau + k * TPR] = v[k];
+}
+
+// The run walked backwards, as k_b_cdrx_adj per layer: half of the CTA's threads carry
+// psi's row and half lambda's.  part[(2 l + kind) rows + row] are the row's partials of
+// layer l's Rx (kind 0) and cd (kind 1).
+template <typename C, int LOGQ>
+__global__ void __launch_bounds__(2 * BLayer<LOGQ>::TPR, 1)
+    k_b_layers_adj(C* __restrict__ psi, C* __restrict__ lam, int logRows, int batch, const double* __restrict__ par,
+                   double2* __restrict__ part, const __grid_constant__ LayerBits A) {
+  using G = BLayer<LOGQ>;
+  constexpr int N = G::N, TPR = G::TPR, LINE = G::template line<C>(), WARPS = 2 * TPR / 32;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double ws[4][WARPS];
+  C* sm = reinterpret_cast<C*>(smraw);
+  double2* lo = reinterpret_cast<double2*>(sm + 2 * LINE);
+  double2* hi = lo + 64;
+  cg::cluster_group cl = cg::this_cluster();
+  const int r = (int)cl.block_rank(), half = threadIdx.x / TPR, t = threadIdx.x % TPR;
+  const int b = (int)(blockIdx.x >> logRows);
+  const size_t rows = (size_t)batch << logRows;
+  C* rowp = (half ? lam : psi) + ((uint64_t)blockIdx.x << LOGQ);
+  C* line = sm + half * LINE;
+  C* other = sm + (half ^ 1) * LINE;
+  const double dx = sqrt(2.0 * M_PI / (double)N);
+  C v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = rowp[t + k * TPR];
+  b_fill_twiddles<LOGQ>(lo, threadIdx.x, 2 * TPR);
+  const double2 tws = ft_twiddle_step(TPR, N, 1);
+  mul_run(v, ft_twiddle(t, N, 1), tws);
+  __syncthreads();  // the twiddle tables
+  int tau = t;
+  for (int l = A.nLayers - 1; l >= 0; --l) {
+    const int bit = A.bit[l];
+    const double th = __ldg(par + (size_t)(2 * l) * batch + b), be = __ldg(par + (size_t)(2 * l + 1) * batch + b);
+    const double kz = -M_SQRT2 * (((r >> bit) & 1) ? -1.0 : 1.0);  // K_k = kz x_k
+    const double coef = -be * kz;                                   // exp(-i beta K)
+    rr_two<C, 1, LOGQ, 4, 0>(v, line, t, tau, lo, hi);
+    // <F lambda| K |F psi> = (1/N) sum_k conj(L_k) K_k P_k for the unnormalised transforms:
+    // the halves exchange what the other needs and take eight points of a thread each
+    double cx = 0.0, cy = 0.0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) line[t + k * TPR] = half ? v[k] : v[k + 8];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int kk = tau + (half ? k + 8 : k) * TPR;
+      const double2 mine = tod_b(half ? v[k + 8] : v[k]), theirs = tod_b(other[t + k * TPR]);
+      const double2 P = half ? theirs : mine, L = half ? mine : theirs;
+      const double w = kz * ((double)kk - 0.5 * (double)(N - 1)) * dx / (double)N;
+      cx += w * (L.x * P.x + L.y * P.y);
+      cy += w * (L.x * P.y - L.y * P.x);
+    }
+    __syncthreads();
+    mul_run(v, b_kick(tau, N, coef), b_kick_step(TPR, N, coef));
+    rr_two<C, -1, LOGQ, 4, 0>(v, line, t, tau, lo, hi);
+    // Rx(-theta) and this row's half of g_rx = sum conj(l_r) (-p_{1-r} / 2)
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) line[t + k * TPR] = v[k];
+    layer_arrive();
+    double s, co, rx = 0.0, ry = 0.0;
+    sincos(-0.5 * th, &s, &co);
+    layer_wait();
+    {
+      const C* pw = cl.map_shared_rank(line, r ^ (1 << bit));
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const double2 x0 = tod_b(v[k]), x1 = tod_b(pw[t + k * TPR]);
+        if (half == 0) {
+          const double2 l0 = tod_b(other[t + k * TPR]);
+          rx -= 0.5 * (l0.x * x1.x + l0.y * x1.y);
+          ry -= 0.5 * (l0.x * x1.y - l0.y * x1.x);
+        }
+        v[k] = fromd<C>(make_double2(co * x0.x + s * x1.y, co * x0.y - s * x1.x));
+      }
+    }
+    double g[4] = {rx, ry, cx, cy};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) g[e] += __shfl_down_sync(0xffffffffu, g[e], o);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ws[e][threadIdx.x >> 5] = g[e];
+    layer_arrive();
+    layer_wait();  // the partner has read these rows, and every warp's sums are in ws
+    if (threadIdx.x < 4) {
+      double a = 0.0;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) a += ws[threadIdx.x][w];
+      double* out = reinterpret_cast<double*>(part + (size_t)(2 * l + (threadIdx.x >> 1)) * rows + blockIdx.x);
+      out[threadIdx.x & 1] = a;
+    }
+  }
+  mul_run(v, cconj(ft_twiddle(tau, N, 1)), cconj(tws));
+#pragma unroll
+  for (int k = 0; k < 16; ++k) rowp[tau + k * TPR] = v[k];
+}
+
+// out[i] = sum of the 2^logRows partials of (gate, instance) i
+__global__ void k_b_layer_sums(const double2* __restrict__ part, int logRows, int count, double2* __restrict__ out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    double2 a = make_double2(0.0, 0.0);
+    for (int k = 0; k < 1 << logRows; ++k) a = cadd(a, part[((size_t)i << logRows) + k]);
+    out[i] = a;
+  }
+}
+
 // <t| a_b> per CTA chunk (t shared by every instance when tStride == 0)
 template <typename C>
 __global__ void __launch_bounds__(kBatchThreads) k_b_dot(const C* __restrict__ a, const C* __restrict__ tg,
@@ -681,6 +889,61 @@ static cudaError_t b_rxcd(void* st, void* lam, int batch, int n, int q, int bit,
   }
 }
 
+template <typename C, int LOGQ>
+static cudaError_t b_layers_t(void* st, void* lam, int batch, int logRows, const double* par, double2* part,
+                              const LayerBits& A, cudaStream_t s) {
+  using G = BLayer<LOGQ>;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)batch << logRows);
+  cfg.blockDim = dim3(lam ? 2 * G::TPR : G::TPR);
+  cfg.dynamicSmemBytes = (size_t)(lam ? 2 : 1) * G::template line<C>() * sizeof(C) + rr_tw_slots(LOGQ) * sizeof(double2);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1u << logRows;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  auto fwd = k_b_layers<C, LOGQ>;
+  auto adj = k_b_layers_adj<C, LOGQ>;
+  cudaError_t e = lam ? cudaFuncSetAttribute(adj, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes)
+                      : cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+  if (e != cudaSuccess) return e;
+  if (lam) return cudaLaunchKernelEx(&cfg, adj, (C*)st, (C*)lam, logRows, batch, par, part, A);
+  return cudaLaunchKernelEx(&cfg, fwd, (C*)st, logRows, batch, par, A);
+}
+
+template <typename C>
+static cudaError_t b_layers(void* st, void* lam, int batch, int q, int logRows, const double* par, double2* part,
+                            const LayerBits& A, cudaStream_t s) {
+  switch (q) {
+    case 9: return b_layers_t<C, 9>(st, lam, batch, logRows, par, part, A, s);
+    case 10: return b_layers_t<C, 10>(st, lam, batch, logRows, par, part, A, s);
+    case 11: return b_layers_t<C, 11>(st, lam, batch, logRows, par, part, A, s);
+    case 12: return b_layers_t<C, 12>(st, lam, batch, logRows, par, part, A, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+// Checks a run's arguments and turns its flat bits into row-index bits.
+static bool b_layer_args(const char* fn, const void* states, int precision, int batch, int n, int q, const int* bits,
+                         int nLayers, const double* par, LayerBits* A) {
+  if (!b_check(fn, states, precision, batch, n)) return false;
+  bool ok = q >= 9 && q <= 12 && n > q && n - q <= 3 && bits && nLayers >= 1 && nLayers <= kMaxLayers && par &&
+            batch <= (1 << 24);
+  A->nLayers = nLayers;
+  for (int l = 0; ok && l < nLayers; ++l) {
+    ok = bits[l] >= q && bits[l] < n;
+    A->bit[l] = (signed char)(bits[l] - q);
+  }
+  if (!ok)
+    set_error(nullptr, kErrInvalidArg,
+              "%s: a mode of 9..12 qubits as the last register, one to three qubits above it, 1..%d layers on their bits",
+              fn, kMaxLayers);
+  return ok;
+}
+
 static bool b_rxcd_args(const char* fn, int n, int q, int bit) {
   if (q < 9 || q > 12 || q >= n || bit < q || bit >= n) {
     set_error(nullptr, kErrInvalidArg,
@@ -695,6 +958,56 @@ static bool b_rxcd_args(const char* fn, int n, int q, int bit) {
 using namespace cvdv;
 
 extern "C" {
+
+int cvdvBatchLayers(void* states, int precision, int batch, int n, int modeQubits, const int* bits, int nLayers,
+                    const double* params, void* stream) {
+  const char* fn = "cvdvBatchLayers";
+  LayerBits A{};
+  if (!b_layer_args(fn, states, precision, batch, n, modeQubits, bits, nLayers, params, &A)) return kErrInvalidArg;
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaError_t e;
+  {
+    LaunchScope _ls(nullptr, kKFft);
+    e = precision == kC128 ? b_layers<double2>(states, nullptr, batch, modeQubits, n - modeQubits, params, nullptr, A, s)
+                           : b_layers<float2>(states, nullptr, batch, modeQubits, n - modeQubits, params, nullptr, A, s);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    set_error(nullptr, kErrCuda, "%s: %s", fn, cudaGetErrorString(e));
+    return kErrCuda;
+  }
+  return kOk;
+}
+
+int cvdvBatchLayersAdjoint(void* psi, void* lam, int precision, int batch, int n, int modeQubits, const int* bits,
+                           int nLayers, const double* params, double* gOut, double* scratch, void* stream) {
+  const char* fn = "cvdvBatchLayersAdjoint";
+  LayerBits A{};
+  if (!b_layer_args(fn, psi, precision, batch, n, modeQubits, bits, nLayers, params, &A)) return kErrInvalidArg;
+  if (!lam || !gOut || !scratch) {
+    set_error(nullptr, kErrInvalidArg, "%s: null argument", fn);
+    return kErrInvalidArg;
+  }
+  cudaStream_t s = (cudaStream_t)stream;
+  const int logRows = n - modeQubits;
+  cudaError_t e;
+  {
+    LaunchScope _ls(nullptr, kKFft);
+    e = precision == kC128 ? b_layers<double2>(psi, lam, batch, modeQubits, logRows, params, (double2*)scratch, A, s)
+                           : b_layers<float2>(psi, lam, batch, modeQubits, logRows, params, (double2*)scratch, A, s);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    set_error(nullptr, kErrCuda, "%s: %s", fn, cudaGetErrorString(e));
+    return kErrCuda;
+  }
+  {
+    LaunchScope _ls(nullptr, kKReduce);
+    const int count = 2 * nLayers * batch;
+    k_b_layer_sums<<<b_grid(count), kBatchThreads, 0, s>>>((const double2*)scratch, logRows, count, (double2*)gOut);
+  }
+  return b_launch_ok(fn) ? kOk : kErrCuda;
+}
 
 int cvdvBatchRxCondDisp(void* states, int precision, int batch, int n, int modeQubits, int bit,
                         const double* thetas, const double* betas, void* stream) {

@@ -81,6 +81,10 @@ SIGNATURES = [
     ("cvdvBatchRxCondDispAdjoint",
      [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
      c_int),
+    ("cvdvBatchLayers", [c_void_p, c_int, c_int, c_int, c_int, POINTER(c_int), c_int, c_void_p, c_void_p], c_int),
+    ("cvdvBatchLayersAdjoint",
+     [c_void_p, c_void_p, c_int, c_int, c_int, c_int, POINTER(c_int), c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+     c_int),
     ("cvdvBatchOverlap", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p], c_int),
     ("cvdvBatchStructSizes", [POINTER(c_int)], None),
     ("cvdvBatchRunStage", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p], c_int),

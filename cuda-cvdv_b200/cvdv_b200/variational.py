@@ -34,6 +34,8 @@ import torch
 from . import _lib
 from .cudaCvdv import PRECISIONS, CvdvError
 
+MAX_LAYERS = 64  # layers of one cvdvBatchLayers launch
+
 GateSpec = Tuple  # ("rx", reg, qubit) | ("cd", mode_reg, ctrl_reg, ctrl_qubit)
 
 
@@ -88,6 +90,18 @@ class VariationalCircuit:
                     and (g + 1) % self.checkpoint_every != 0)
             self._steps.append((g, 2 if pair else 1))
             g += 2 if pair else 1
+        # With one to three qubits above the mode, consecutive fused layers with no
+        # checkpoint between them run as one launch (cvdvBatchLayers, at most MAX_LAYERS):
+        # the launches are (first gate, number of gates) in circuit order.
+        self._launches: List[Tuple[int, int]] = []
+        layered = 1 <= self.n - q <= 3
+        for g, k in self._steps:
+            if (layered and k == 2 and self._launches and self._launches[-1][1] >= 2
+                    and self._launches[-1][1] < 2 * MAX_LAYERS and g % self.checkpoint_every != 0):
+                self._launches[-1] = (self._launches[-1][0], self._launches[-1][1] + 2)
+            else:
+                self._launches.append((g, k))
+        self._layered = layered
 
     @property
     def n_gates(self) -> int:
@@ -106,10 +120,18 @@ class VariationalCircuit:
             _check(self._L.cvdvBatchCondDisp(_ptr(psi), self.prec, B, self.n, self.qubits[self.mode], bit,
                                              _ptr(p), sign, self._stream()))
 
+    def _bits(self, g: int, n: int):
+        """Flat bits of the fused layers of gates g .. g + n - 1, as the C call takes them."""
+        return (ctypes.c_int * (n // 2))(*[self._gates[k][1] for k in range(g, g + n, 2)])
+
     def _apply_step(self, psi: torch.Tensor, g: int, n: int, p: torch.Tensor) -> None:
-        """Gates g .. g + n - 1 (n = 2: the fused Rx + cd layer)."""
+        """Gates g .. g + n - 1 (n even: n / 2 fused Rx + cd layers)."""
         if n == 1:
             self._apply(psi, g, p[g])
+            return
+        if self._layered:
+            _check(self._L.cvdvBatchLayers(_ptr(psi), self.prec, psi.shape[0], self.n, self.qubits[self.mode],
+                                           self._bits(g, n), n // 2, _ptr(p[g]), self._stream()))
             return
         _check(self._L.cvdvBatchRxCondDisp(_ptr(psi), self.prec, psi.shape[0], self.n, self.qubits[self.mode],
                                            self._gates[g][1], _ptr(p[g]), _ptr(p[g + 1]), self._stream()))
@@ -119,6 +141,12 @@ class VariationalCircuit:
         """Adjoint of gates g + n - 1 .. g, writing their g values into gvals[g ...]."""
         if n == 1:
             self._adjoint(psi, lam, g, p[g], gvals[g])
+            return
+        if self._layered:
+            B, q = psi.shape[0], self.qubits[self.mode]
+            scratch = torch.empty((2 * n * B) << (self.n - q), dtype=torch.float64, device=psi.device)
+            _check(self._L.cvdvBatchLayersAdjoint(_ptr(psi), _ptr(lam), self.prec, B, self.n, q, self._bits(g, n),
+                                                  n // 2, _ptr(p[g]), _ptr(gvals[g]), _ptr(scratch), self._stream()))
             return
         grx = torch.view_as_real(gvals[g]).view(-1)
         gcd = torch.view_as_real(gvals[g + 1]).view(-1)
@@ -168,7 +196,7 @@ class VariationalCircuit:
     def states(self, params: torch.Tensor, psi0: torch.Tensor) -> torch.Tensor:
         """Final states (batch, 2^n) for every parameter set; psi0 is one state or one per instance."""
         p, psi = self._prepare(params, psi0)
-        for g, n in self._steps:
+        for g, n in self._launches:
             self._apply_step(psi, g, n, p)
         return psi
 
@@ -194,7 +222,7 @@ class _FidelityLoss(torch.autograd.Function):
         p, psi = circ._prepare(params, psi0)
         tgt = target.to(device="cuda", dtype=circ.cdtype).contiguous()
         checkpoints = {}
-        for g, n in circ._steps:
+        for g, n in circ._launches:
             if g % circ.checkpoint_every == 0 and g > 0:
                 checkpoints[g] = psi.clone()  # the state before gate g
             circ._apply_step(psi, g, n, p)
@@ -213,7 +241,7 @@ class _FidelityLoss(torch.autograd.Function):
         psi = psi_final.clone()
         lam = tgt.expand(B, -1).contiguous() if tgt.dim() == 1 else tgt.clone()
         gvals = torch.empty(circ.n_gates, B, dtype=torch.complex128, device=psi.device)
-        for g, n in reversed(circ._steps):
+        for g, n in reversed(circ._launches):
             circ._adjoint_step(psi, lam, g, n, p, gvals)
             ck = ctx.checkpoints.get(g)
             if ck is not None:
@@ -260,7 +288,7 @@ class _GraphPlan:
 
     def _forward(self, c: VariationalCircuit) -> None:
         self.psi.copy_(self.psi0.expand_as(self.psi))
-        for g, n in c._steps:
+        for g, n in c._launches:
             if g in self.ck:
                 self.ck[g].copy_(self.psi)  # the state before gate g
             c._apply_step(self.psi, g, n, self.p)
@@ -269,7 +297,7 @@ class _GraphPlan:
     def _backward(self, c: VariationalCircuit) -> None:
         self.back.copy_(self.psi)
         self.lam.copy_(self.tgt.expand_as(self.lam))
-        for g, n in reversed(c._steps):
+        for g, n in reversed(c._launches):
             c._adjoint_step(self.back, self.lam, g, n, self.p, self.gvals)
             ck = self.ck.get(g)
             if ck is not None:

@@ -228,6 +228,17 @@ int cvdvBatchRxCondDisp(void* states, int precision, int batch, int n, int modeQ
 int cvdvBatchRxCondDispAdjoint(void* psi, void* lam, int precision, int batch, int n, int modeQubits, int bit,
                                const double* thetas, const double* betas, double* gRx, double* gCd,
                                void* stream);
+/* A run of nLayers (1..64) such layers in one launch, for one to three qubit bits above
+ * the mode: layer l acts on flat bit bits[l] (host array) with Rx(params[2 l batch + b])
+ * then cd(params[(2 l + 1) batch + b]) (device array, gate by gate). */
+int cvdvBatchLayers(void* states, int precision, int batch, int n, int modeQubits, const int* bits, int nLayers,
+                    const double* params, void* stream);
+/* Adjoint of the run: the layers' inverses applied to psi and lam from the last to the
+ * first, with g of gate i (2 l the Rx, 2 l + 1 the cd) at gOut[2 (i batch + b)].  scratch
+ * is a device array of 4 nLayers batch 2^(n - modeQubits) doubles that the call may
+ * overwrite until its work on the stream is done. */
+int cvdvBatchLayersAdjoint(void* psi, void* lam, int precision, int batch, int n, int modeQubits, const int* bits,
+                           int nLayers, const double* params, double* gOut, double* scratch, void* stream);
 /* out[2b], out[2b+1] = <target| states_b> (target shared by every instance, or
  * one per instance when targetPerInstance != 0). */
 int cvdvBatchOverlap(const void* states, const void* target, int precision, int batch, int n,
