@@ -46,6 +46,10 @@ constexpr size_t stage_smem() {
   return (size_t)(kStageThreads * E + kStageThreads * E / 16) * sizeof(C) + (64 + (1 << (L - 6))) * sizeof(double2);
 }
 
+// after it, each warp's constants of a quadratic phase (phase_run): E for each of its rows
+constexpr int kStageQuads = 128;
+constexpr size_t stage_quad_bytes() { return (size_t)(kStageThreads / 32) * kStageQuads * sizeof(double2); }
+
 template <typename C> struct StageReal;
 template <> struct StageReal<double2> { using t = double; };
 template <> struct StageReal<float2> { using t = float; };
@@ -73,6 +77,57 @@ __device__ __forceinline__ C phase_factor(const CvdvBatchPhase& P, int j, int N,
   return mk(sc * c, sc * s);
 }
 
+// q m mod 1 (in -1/2 .. 1/2) for a phase of q m turns, m an integer that a double holds
+__device__ __forceinline__ double stage_turns(double q, double m) { return fma(q, m, -rint(q * m)); }
+__device__ __forceinline__ double2 turn_factor(double p) {
+  double s, c;
+  sincospi(2.0 * p, &s, &c);
+  return make_double2(c, s);
+}
+
+// A phase without a cubic term on the points t + k TPR of a row.  With u = 2 j - N + 1 and
+// dx^2 = 2 pi / N its turns are a quadratic in the integer u,
+//   tw (N-1) u / (4N) + (g0 + z h0) / 2pi + (a1 + z b1) dx u / 4pi + (a2 + z b2) u^2 / (4N),
+// so a thread needs its value at its first point and its step (a sincospi each), a
+// running product, and the E constants exp(2 pi i q (2 TPR)^2 k^2) of the quadratic
+// part, which the row's lanes in the warp evaluate one each into `kq`.  Evaluating the
+// polynomial per point took about 25 FP64 operations, the conversions of its integers
+// and a fast sine and cosine each, about as long as the transforms between the phases;
+// this takes 8, and is exact to FP64 where the fast intrinsic was to 4e-7.
+// STAGENOTE
+template <typename C, int LOGN, int LOGE>
+__device__ __forceinline__ void phase_run(C (&v)[1 << LOGE], const CvdvBatchPhase& P, int t, double zs, double2* kq) {
+  constexpr int E = 1 << LOGE, N = 1 << LOGN, TPR = N >> LOGE, LANES = TPR < 32 ? TPR : 32;
+  constexpr double inv4N = 1.0 / (4.0 * N);
+  const int u0 = 2 * t - N + 1;
+  const double dx = sqrt(2.0 * M_PI / (double)N);
+  const double lin = (P.a1 + zs * P.b1) * (dx / (4.0 * M_PI)), q = (P.a2 + zs * P.b2) * inv4N;
+  // tw (N-1) u mod 4N in integers
+  const int w = (P.tw * (N - 1)) & (4 * N - 1);
+  double p0 = (double)((int)((long long)w * u0) & (4 * N - 1)) * inv4N + stage_turns(lin, (double)u0) +
+              (P.g0 + zs * P.h0) * (0.5 / M_PI);
+  double p1 = (double)((int)((long long)w * (2 * TPR)) & (4 * N - 1)) * inv4N + stage_turns(lin, 2.0 * TPR);
+  const bool quad = P.a2 != 0.0 || P.b2 != 0.0;  // the same for every row of the task
+  if (quad) {
+    p0 += stage_turns(q, (double)u0 * (double)u0);
+    p1 += stage_turns(q, 4.0 * TPR * (double)u0);
+    __syncwarp();  // the last run's constants are read
+    const int lane = t & (LANES - 1);
+#pragma unroll
+    for (int k = lane; k < E; k += LANES) kq[k] = turn_factor(stage_turns(q, 4.0 * TPR * TPR * (double)(k * k)));
+    __syncwarp();
+  }
+  double2 f = turn_factor(p0);
+  f.x *= P.scale;
+  f.y *= P.scale;
+  const double2 st = turn_factor(p1);
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    v[k] = cmul(v[k], fromd<C>(quad ? dmul(f, kq[k]) : f));
+    f = dmul(f, st);
+  }
+}
+
 template <typename C, int LOGN, int LOGE>
 __device__ __forceinline__ void stage_row_task(C* __restrict__ st, const CvdvBatchTask& T,
                                                const CvdvBatchProgram& Pg, unsigned char* smraw) {
@@ -88,6 +143,10 @@ __device__ __forceinline__ void stage_row_task(C* __restrict__ st, const CvdvBat
   const uint64_t rowIdx = (uint64_t)T.first + (valid ? row : 0);
   C* src = st + T.stateOffset + (rowIdx << LOGN);
   C* smrow = sm + row * RS;
+  // the quadratic constants: E for each row's lanes of a warp
+  double2* kqs = reinterpret_cast<double2*>(smraw + stage_smem<C>());
+  double2* kq = kqs + (tid >> 5) * kStageQuads + (TPR < 32 ? ((tid & 31) / TPR) * E : 0);
+  static_assert(TPR >= 32 || (32 / TPR) * E <= kStageQuads, "constants per warp");
   for (int i = tid; i < 64 + (N >> 6); i += kStageThreads) {
     const int e = i < 64 ? i : (i - 64) << 6;
     double s, c;
@@ -104,8 +163,12 @@ __device__ __forceinline__ void stage_row_task(C* __restrict__ st, const CvdvBat
     if (op == 0) {
       const CvdvBatchPhase P = Pg.phase[d++];
       const double zs = (P.ctrlBit >= 0 && (((rowIdx << LOGN) >> P.ctrlBit) & 1ull)) ? -1.0 : 1.0;
+      if (P.a3 == 0.0) {
+        phase_run<C, LOGN, LOGE>(v, P, t, zs, kq);
+      } else {
 #pragma unroll
-      for (int k = 0; k < E; ++k) v[k] = cmul(v[k], phase_factor<C>(P, t + k * TPR, N, zs));
+        for (int k = 0; k < E; ++k) v[k] = cmul(v[k], phase_factor<C>(P, t + k * TPR, N, zs));
+      }
     } else if (op == 1 || op == 2) {
       // one transform body for both directions (keeps the kernel's code small):
       // the unnormalised inverse DFT is conj(DFT(conj(x)))
@@ -218,7 +281,7 @@ int cvdvBatchRunStage(void* states, int precision, const CvdvBatchTask* tasks, i
   {
     LaunchScope _ls(nullptr, kKFft);
     if (precision == kC128) {
-      const size_t smem = stage_smem<double2>();
+      const size_t smem = stage_smem<double2>() + stage_quad_bytes();
       if (!attr128) {
         e = cudaFuncSetAttribute(k_batch_stage<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr128 = e == cudaSuccess;
@@ -228,7 +291,7 @@ int cvdvBatchRunStage(void* states, int precision, const CvdvBatchTask* tasks, i
         e = cudaGetLastError();
       }
     } else {
-      const size_t smem = stage_smem<float2>();
+      const size_t smem = stage_smem<float2>() + stage_quad_bytes();
       if (!attr64) {
         e = cudaFuncSetAttribute(k_batch_stage<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr64 = e == cudaSuccess;
