@@ -45,6 +45,10 @@ TASK_DTYPE = np.dtype([("stateOffset", "i8"), ("kind", "i4"), ("n", "i4"), ("log
 OP_DIAG, OP_FWD, OP_INV, OP_PARITY = 0, 1, 2, 3
 SQRT2 = math.sqrt(2.0)
 THREADS = 512
+# A stage launches a CTA per task up to this many (self.grid at least), so an SM that
+# finishes early takes the next task; past it the CTAs walk the list.  512 circuits, 1283
+# tasks a stage: 3.17 ms per 20 stages against 3.53 with 148 CTAs.
+MAX_CTAS = 1024
 
 
 def loge_options(m: int, prec: int) -> List[int]:
@@ -56,6 +60,21 @@ def loge_options(m: int, prec: int) -> List[int]:
 
 def default_loge(m: int, prec: int) -> int:
     return 5 if (prec == 1 and m >= 13) else 4
+
+
+def adaptive_loge(m: int, prec: int, tasks_per_stage: float) -> int:
+    """default_loge for a batch of that many tasks a stage at the default shapes, or the
+    next smaller ones where a stage does not fill the chip's 148 CTAs twice: its time is
+    then the longest row task's latency, and fewer amplitudes a thread are more threads
+    on a row.  Stages of 96 circuits (154 tasks, modes 2^8..2^13, complex64): 30 us with 16
+    amplitudes a thread on the 2^13-point rows, 47 with 32; of 300 circuits (790 tasks): 86
+    and 83.  16 circuits (21 tasks, 2^10..2^12): 21 us with 8 amplitudes a thread, 26 with 16."""
+    e = default_loge(m, prec)
+    if tasks_per_stage < 74 and m <= 12:
+        e = 3
+    elif tasks_per_stage < 296:
+        e = min(e, 4)
+    return e if e in loge_options(m, prec) else default_loge(m, prec)
 
 
 def struct_sizes() -> Tuple[int, int, int]:
@@ -219,7 +238,8 @@ class BatchedCircuits:
                  pair_chunk: int = 4096, grid: int = 148, row_loge: Optional[Dict[int, int]] = None) -> None:
         """instances: dicts with ``qubits`` ([1]*Q + [m]) and ``gates`` [(name, args)];
         row_loge: amplitudes per thread (log2) of the row tasks per mode length m
-        (default 4, or 5 for complex64 modes of 2^13 and 2^14 points)."""
+        (default 4, or 5 for complex64 modes of 2^13 and 2^14 points; less for batches
+        that do not fill the chip, adaptive_loge).  grid: CTAs of a stage, at least."""
         self.prec = PRECISIONS[precision]
         self.cdtype = torch.complex128 if self.prec == 0 else torch.complex64
         self.instances = list(instances)
@@ -247,13 +267,14 @@ class BatchedCircuits:
 
     # ---------------------------------------------------------------- compile
     def _compile(self) -> None:
+        self._tasks_per_stage = self._count_tasks() / max(1, self.n_stages)
         progs: List[np.void] = []
         stage_tasks: List[List[np.void]] = [[] for _ in range(self.n_stages)]
         for i, inst in enumerate(self.instances):
             q = inst["qubits"]
             n, m = sum(q), q[-1]
             mode = len(q) - 1
-            logE = self.row_loge.get(m, default_loge(m, self.prec))
+            logE = self._loge(m)
             rows_per_task = max(1, THREADS // ((1 << m) >> logE))
             for s, (name, args) in enumerate(inst["gates"]):
                 if name in self.QUBIT_GATES:
@@ -308,6 +329,21 @@ class BatchedCircuits:
             self._validate(arr)
             self._tasks.append((torch.from_numpy(arr.view(np.uint8).copy()).cuda(), len(arr)))
 
+    def _count_tasks(self) -> int:
+        """Tasks of all stages at the default shapes."""
+        total = 0
+        for inst in self.instances:
+            n, m = sum(inst["qubits"]), inst["qubits"][-1]
+            rows = 1 << (n - m)
+            per = max(1, THREADS // ((1 << m) >> default_loge(m, self.prec)))
+            pairs = sum(1 for name, _ in inst["gates"] if name in ("h", "rx", "ry"))
+            total += (len(inst["gates"]) - pairs) * -(-rows // per) + pairs * -(-(1 << (n - 1)) // self.pair_chunk)
+        return total
+
+    def _loge(self, m: int) -> int:
+        """Amplitudes per thread (log2) of the row tasks of 2^m points: as asked for, or by the batch's size."""
+        return self.row_loge.get(m, adaptive_loge(m, self.prec, self._tasks_per_stage))
+
     def _row_tasks(self, i: int, n: int, m: int, prog: int, per: int, logE: int) -> List[np.void]:
         out = []
         rows = 1 << (n - m)
@@ -351,7 +387,8 @@ class BatchedCircuits:
         for tasks, nt in self._tasks:
             code = self._L.cvdvBatchRunStage(ctypes.c_void_p(self.states.data_ptr()), self.prec,
                                              ctypes.c_void_p(tasks.data_ptr()), nt,
-                                             ctypes.c_void_p(self._progs.data_ptr()), self.grid, stream)
+                                             ctypes.c_void_p(self._progs.data_ptr()),
+                                             max(self.grid, min(nt, MAX_CTAS)), stream)
             if code:
                 raise CvdvError(_lib.last_error(None)[1])
 
@@ -409,7 +446,7 @@ class BatchedCircuits:
                 m = inst["qubits"][-1]
                 work[m] = work.get(m, 0) + (1 << sum(inst["qubits"]))
             for m in sorted(work, key=lambda k: -work[k]):
-                keep = self.row_loge.get(m, default_loge(m, self.prec))
+                keep = self._loge(m)
                 for e in loge_options(m, self.prec):
                     if e == keep:
                         continue
