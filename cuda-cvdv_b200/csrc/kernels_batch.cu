@@ -533,9 +533,10 @@ __global__ void __launch_bounds__(BPair<LOGQ>::TPR, 1)
 // step of its own (k_b_rxcd) takes 8-10 us however small the row, most of it launch,
 // cluster set-up, twiddle tables and the state's way through memory.  Forward / adjoint
 // sweep of 64 sets x 40 layers, a launch per layer -> per 8 layers (checkpoints every 16
-// gates): complex64 [1, 12] 381 / 629 -> 258 / 489 us, complex128 518 / 894 -> 368 / 742,
-// complex64 [1, 10] 295 / 534 -> 148 / 234.  [1, 12] with the Stockham stages instead of
-// rr_two: 269 / 501.
+// gates): complex64 [1, 12] 381 / 629 -> 267 / 494 us, complex128 508 / 885 -> 379 / 764,
+// complex64 [1, 10] 295 / 535 -> 155 / 240.  With rr_two instead of the Stockham stages
+// [1, 12] took 258 / 489, but rows of 2^9 points have one tree of twiddle powers there and
+// two with it: after 40 layers the complex64 gradients were off by 1.8e-5 instead of 3.7e-6.
 //
 // A cluster barrier has two halves: a CTA arrives once it has read its partner's row
 // and waits for the others' arrival only where its own line is written again.
@@ -547,13 +548,7 @@ struct LayerBits {
 
 template <int LOGQ>
 struct BLayer {
-  static constexpr int N = 1 << LOGQ, TPR = N >> 4;
-  // a row's shared line (rr_two's, at least the row itself)
-  template <typename C>
-  static constexpr int line() {
-    static_assert(RrTwo<C, LOGQ, 4, 0>::ok && RrTwo<C, LOGQ, 4, 0>::LINE >= N, "row line");
-    return RrTwo<C, LOGQ, 4, 0>::LINE;
-  }
+  static constexpr int N = 1 << LOGQ, TPR = N >> 4, LINE = N + (N >> 4);  // a row's padded shared line
 };
 
 __device__ __forceinline__ void layer_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -577,7 +572,7 @@ __global__ void __launch_bounds__(BLayer<LOGQ>::TPR, 1)
   constexpr int N = G::N, TPR = G::TPR;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
-  double2* lo = reinterpret_cast<double2*>(sm + G::template line<C>());
+  double2* lo = reinterpret_cast<double2*>(sm + G::LINE);
   double2* hi = lo + 64;
   cg::cluster_group cl = cg::this_cluster();
   const int r = (int)cl.block_rank(), t = threadIdx.x;
@@ -590,12 +585,11 @@ __global__ void __launch_bounds__(BLayer<LOGQ>::TPR, 1)
   const double2 tws = ft_twiddle_step(TPR, N, 1);
   mul_run(v, ft_twiddle(t, N, 1), tws);
   __syncthreads();  // the twiddle tables
-  int tau = t;      // v[k] is point tau + k TPR; the partner's thread t holds the same points
   for (int l = 0; l < A.nLayers; ++l) {
     const int bit = A.bit[l];
     const double th = __ldg(par + (size_t)(2 * l) * batch + b), be = __ldg(par + (size_t)(2 * l + 1) * batch + b);
     // Rx: v <- c v - i s w with w the partner row's amplitude at the same point
-    if (l) __syncthreads();  // the transform's last exchange is read
+    // (the transforms' last exchange ended in a barrier: the line is free)
 #pragma unroll
     for (int k = 0; k < 16; ++k) sm[t + k * TPR] = v[k];
     layer_arrive();
@@ -613,13 +607,13 @@ __global__ void __launch_bounds__(BLayer<LOGQ>::TPR, 1)
     }
     layer_arrive();
     layer_wait();  // the partner has read this row
-    rr_two<C, 1, LOGQ, 4, 0>(v, sm, t, tau, lo, hi);
-    mul_run(v, b_kick(tau, N, coef), b_kick_step(TPR, N, coef));
-    rr_two<C, -1, LOGQ, 4, 0>(v, sm, t, tau, lo, hi);
+    rr_stages<C, 1, LOGQ, 0, 4>(v, sm, t, lo, hi);
+    mul_run(v, b_kick(t, N, coef), b_kick_step(TPR, N, coef));
+    rr_stages<C, -1, LOGQ, 0, 4>(v, sm, t, lo, hi);
   }
-  mul_run(v, cconj(ft_twiddle(tau, N, 1)), cconj(tws));
+  mul_run(v, cconj(ft_twiddle(t, N, 1)), cconj(tws));
 #pragma unroll
-  for (int k = 0; k < 16; ++k) rowp[tau + k * TPR] = v[k];
+  for (int k = 0; k < 16; ++k) rowp[t + k * TPR] = v[k];
 }
 
 // The run walked backwards, as k_b_cdrx_adj per layer: half of the CTA's threads carry
@@ -630,7 +624,7 @@ __global__ void __launch_bounds__(2 * BLayer<LOGQ>::TPR, 1)
     k_b_layers_adj(C* __restrict__ psi, C* __restrict__ lam, int logRows, int batch, const double* __restrict__ par,
                    double2* __restrict__ part, const __grid_constant__ LayerBits A) {
   using G = BLayer<LOGQ>;
-  constexpr int N = G::N, TPR = G::TPR, LINE = G::template line<C>(), WARPS = 2 * TPR / 32;
+  constexpr int N = G::N, TPR = G::TPR, LINE = G::LINE, WARPS = 2 * TPR / 32;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double ws[4][WARPS];
   C* sm = reinterpret_cast<C*>(smraw);
@@ -651,23 +645,21 @@ __global__ void __launch_bounds__(2 * BLayer<LOGQ>::TPR, 1)
   const double2 tws = ft_twiddle_step(TPR, N, 1);
   mul_run(v, ft_twiddle(t, N, 1), tws);
   __syncthreads();  // the twiddle tables
-  int tau = t;
   for (int l = A.nLayers - 1; l >= 0; --l) {
     const int bit = A.bit[l];
     const double th = __ldg(par + (size_t)(2 * l) * batch + b), be = __ldg(par + (size_t)(2 * l + 1) * batch + b);
     const double kz = -M_SQRT2 * (((r >> bit) & 1) ? -1.0 : 1.0);  // K_k = kz x_k
     const double coef = -be * kz;                                   // exp(-i beta K)
-    rr_two<C, 1, LOGQ, 4, 0>(v, line, t, tau, lo, hi);
+    rr_stages<C, 1, LOGQ, 0, 4>(v, line, t, lo, hi);
     // <F lambda| K |F psi> = (1/N) sum_k conj(L_k) K_k P_k for the unnormalised transforms:
     // the halves exchange what the other needs and take eight points of a thread each
     double cx = 0.0, cy = 0.0;
-    __syncthreads();
 #pragma unroll
     for (int k = 0; k < 8; ++k) line[t + k * TPR] = half ? v[k] : v[k + 8];
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const int kk = tau + (half ? k + 8 : k) * TPR;
+      const int kk = t + (half ? k + 8 : k) * TPR;
       const double2 mine = tod_b(half ? v[k + 8] : v[k]), theirs = tod_b(other[t + k * TPR]);
       const double2 P = half ? theirs : mine, L = half ? mine : theirs;
       const double w = kz * ((double)kk - 0.5 * (double)(N - 1)) * dx / (double)N;
@@ -675,10 +667,9 @@ __global__ void __launch_bounds__(2 * BLayer<LOGQ>::TPR, 1)
       cy += w * (L.x * P.y - L.y * P.x);
     }
     __syncthreads();
-    mul_run(v, b_kick(tau, N, coef), b_kick_step(TPR, N, coef));
-    rr_two<C, -1, LOGQ, 4, 0>(v, line, t, tau, lo, hi);
+    mul_run(v, b_kick(t, N, coef), b_kick_step(TPR, N, coef));
+    rr_stages<C, -1, LOGQ, 0, 4>(v, line, t, lo, hi);
     // Rx(-theta) and this row's half of g_rx = sum conj(l_r) (-p_{1-r} / 2)
-    __syncthreads();
 #pragma unroll
     for (int k = 0; k < 16; ++k) line[t + k * TPR] = v[k];
     layer_arrive();
@@ -716,9 +707,9 @@ __global__ void __launch_bounds__(2 * BLayer<LOGQ>::TPR, 1)
       out[threadIdx.x & 1] = a;
     }
   }
-  mul_run(v, cconj(ft_twiddle(tau, N, 1)), cconj(tws));
+  mul_run(v, cconj(ft_twiddle(t, N, 1)), cconj(tws));
 #pragma unroll
-  for (int k = 0; k < 16; ++k) rowp[tau + k * TPR] = v[k];
+  for (int k = 0; k < 16; ++k) rowp[t + k * TPR] = v[k];
 }
 
 // out[i] = sum of the 2^logRows partials of (gate, instance) i
@@ -896,7 +887,7 @@ static cudaError_t b_layers_t(void* st, void* lam, int batch, int logRows, const
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)batch << logRows);
   cfg.blockDim = dim3(lam ? 2 * G::TPR : G::TPR);
-  cfg.dynamicSmemBytes = (size_t)(lam ? 2 : 1) * G::template line<C>() * sizeof(C) + rr_tw_slots(LOGQ) * sizeof(double2);
+  cfg.dynamicSmemBytes = (size_t)(lam ? 2 : 1) * G::LINE * sizeof(C) + rr_tw_slots(LOGQ) * sizeof(double2);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

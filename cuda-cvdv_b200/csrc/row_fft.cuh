@@ -264,8 +264,8 @@ __device__ __forceinline__ void rr_stages(C (&v)[1 << LOGE], C* smrow, int t, co
 // w^4 in complex128) come from the tables too: products of w alone multiply its error
 // by u, up to 31 where radix 16 has 15.  Error of a three-layer network on [13, 6]
 // against extended precision: complex128 2.5e-14 with w alone, 1.6e-14 with w^16, 1.1e-14
-// with w^4 and w^16, as with the radix-16 stages (complex64 2.5e-6, 1.7e-6, 2.1e-6).  For radix
-// 32 the upper half is formed as it is applied, so only 17 powers are live at once.
+// with w^4 and w^16, as with the radix-16 stages (complex64 2.5e-6, 1.7e-6, 2.1e-6).  For radix 32
+// the upper half is formed as it is applied, so only 17 powers are live at once.
 template <typename C, int DIR, int RAD>
 __device__ __forceinline__ void mul_powers(C (&x)[RAD], const double2* lo, const double2* hi, int e) {
   constexpr int RT = RAD > 16 ? 16 : RAD;
