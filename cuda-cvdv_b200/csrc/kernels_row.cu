@@ -1165,7 +1165,7 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
       return false;
     }
     if (rowSums && !col) {
-      const int logE = q < 8 || (q <= 12 && rowr_small(ctx)) ? 3 : q >= 13 ? 5 : 4;
+      const int logE = rowr_log_e(ctx->precision == kC128, q, rowr_small(ctx));
       const int tpr = 1 << (q - logE);
       P.rowSums = ctx->rowSums;
       ctx->rowSumParts = tpr < 32 ? 1 : tpr / 32;

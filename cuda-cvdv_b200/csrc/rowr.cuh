@@ -219,11 +219,12 @@ __device__ __forceinline__ void l2_prefetch_tile(const void* p, uint32_t bytes) 
 // (complex64 2^14-point rows store 16-byte pieces with it: 2.33 against 1.63 ms per
 // 2^28 state), and shapes of 8 or 16 amplitudes a thread, which keep tables, read them
 // in short pieces (2^8-point columns 2.23 against 1.54 ms, 2^12-point 3.11 against
-// 2.76; only the 2^7-point shape gains, 1.84 against 2.41).
+// 2.76; only the 2^7-point shape gains, 1.84 against 2.41; in complex64 its second tree
+// of twiddle powers would cost half as much error again, so it keeps the stages there).
 template <typename C, int LOGM, int LOGE, int LOGR, bool COL>
 constexpr bool rr_use_two() {
   using T = RrTwo<C, LOGM, LOGE, COL ? LOGR : 0>;
-  return T::ok && ((LOGE == 5 && (COL || 32 / T::G * sizeof(C) >= 32)) || LOGM == 7);
+  return T::ok && ((LOGE == 5 && (COL || 32 / T::G * sizeof(C) >= 32)) || (LOGM == 7 && sizeof(C) == 16));
 }
 // Whether the shape's quadratic runs go without a table: with 32 amplitudes a thread
 // the two sincospi of a run are worth the loads they save, above all after rr_two, whose
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOG
   const int t = COL ? (tid >> LOGR) : tid & (TPR - 1);
   C* smrow = sm + row * RS;
   const int logS = COL ? P.logS : 0;
-  if constexpr (LOGM < 8) row &= P.rowMask;  // (longer rows: LOGR = 0 where rows are few)
+  if constexpr (LOGM <= 8) row &= P.rowMask;  // (longer rows: LOGR = 0 where rows are few)
 
   const int scM = P.logTwN - LOGM;
   for (int i = tid; i < rr_tw_slots(LOGM); i += NT) {
@@ -388,20 +389,27 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOG
 // largest row k_rowr takes (one CTA: 2^13 complex128 / 2^14 complex64 points)
 inline int rowr_max_log(int precision) { return precision == kC128 ? 13 : 14; }
 
-// Rows of 2^13 and 2^14 points keep 32 amplitudes per thread (256 / 512 threads; two
-// exchanges in shared memory per transform instead of three: complex128 [13, 13] network
-// rows 8.4 against 9.6 ms, columns 12.6 against 13.9), everything else 16, and rows
-// shorter than 2^8 points 8
+// log2 of the amplitudes a thread keeps of a row of 2^logM points.  Rows of 2^13 and 2^14
+// points: 32 (256 / 512 threads; two exchanges in shared memory per transform instead of
+// three: complex128 [13, 13] network rows 8.4 against 9.6 ms, columns 12.6 against 13.9).
+// Otherwise 16, and in complex128 8 for rows shorter than 2^8 points and, up to 2^12, for
+// small states (below).  Complex64 stays at 16: a transform's norm loses 4e-8 there and
+// 8e-8 with radix-8 stages, whose constants' float roundings all shrink it (the error
+// of a 60-gate circuit is this drift).
+constexpr int rowr_log_e(bool c128, int logM, bool small) {
+  return logM >= 13 ? 5 : c128 && (logM < 8 || small) ? 3 : 4;
+}
+
 template <typename C, int LOGM>
 struct RrShape {
-  static constexpr int LOGE = LOGM < 8 ? 3 : LOGM >= 13 ? 5 : 4;
-  static constexpr int LOGR = LOGM < 8 ? 10 - LOGM : LOGM - LOGE < 8 ? 8 - (LOGM - LOGE) : 0;
+  static constexpr int LOGE = rowr_log_e(sizeof(C) == sizeof(double2), LOGM, false);
+  static constexpr int LOGR = LOGM < 8 ? 7 - (LOGM - LOGE) : LOGM - LOGE < 8 ? 8 - (LOGM - LOGE) : 0;
 };
 
 // Rows of 2^8 .. 2^12 points of a state below 2^kRowrSmallLog amplitudes run one row
-// per CTA at 8 amplitudes a thread (radix-8 stages): such a state does not fill the
-// chip, so a program takes the latency of one CTA's chain, and twice the warps on a
-// row shorten it.
+// per CTA (two at 2^8 points in complex64: a warp), at 8 amplitudes a thread in
+// complex128: such a state does not fill the chip, so a program takes the latency of
+// one CTA's chain, and more warps and CTAs shorten it.  SMALLNOTE
 constexpr int kRowrSmallLog = 19;
 inline bool rowr_small(Context* ctx) { return ctx->totalQbt < kRowrSmallLog; }
 
@@ -449,7 +457,8 @@ static cudaError_t launch_rowr_t(Context* ctx, const void* in, void* out, const 
   // column form: at least two columns a CTA while it stays within 512 threads
   constexpr int LOGR = (COL && LOGR0 == 0 && (sizeof(C) << LOGM) < (128u << 10)) ? 1 : LOGR0;
   if constexpr (LOGM >= 8 && LOGM <= 12) {
-    if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, 0, 3, COL>(ctx, in, out, P);
+    constexpr int SE = rowr_log_e(sizeof(C) == sizeof(double2), LOGM, true), SR = LOGM - SE < 5 ? 5 - (LOGM - SE) : 0;
+    if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, SR, SE, COL>(ctx, in, out, P);
   }
   return launch_rowr_s<C, LOGM, LOGR, LOGE, COL>(ctx, in, out, P);
 }
