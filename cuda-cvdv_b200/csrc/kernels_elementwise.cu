@@ -6,6 +6,7 @@
 // that stay resident in L1/L2.
 
 #include "cvdv_internal.cuh"
+#include "turns.cuh"
 
 namespace cvdv {
 
@@ -25,12 +26,10 @@ struct TableBatch {
   TableTerm term[T];
 };
 
-// Table entry (b, j) = prod over terms.  Polynomial terms are summed into one
-// FP64 phase first (the same x_j expression as gridX in the reference,
-// src/cuda/kernels/utils.cuh:5-7, and the same coeff*x*x*... evaluation order
-// as kernelPhaseX/X2/X3, src/cuda/kernels/gates.cuh:5-16,184-209); the FT
-// twiddle is generated exactly from the integer (N-1)(2j-N+1) mod 4N so its
-// argument carries no rounding however large N is.
+// Table entry (b, j) = prod over terms.  Terms of degree one and two and transform
+// twiddles are summed in turns, in two words (turns.cuh), and take one sine and cosine;
+// cubic terms are summed in radians, in the reference's order of operations (x = (idx -
+// (dim-1)*0.5)*dx, kernelPhaseX3, src/cuda/kernels/gates.cuh:5-16,184-209).
 //
 // All tables of a flush are built by one launch: a table is 2^8 .. 2^15 entries, a
 // launch of its own took about 3 us however short, and a circuit has several per
@@ -54,33 +53,45 @@ __global__ void __launch_bounds__(kTableThreads) k_build_tables(const __grid_con
     const int logM = H.logN - H.permLogC;
     j = ((j & ((1 << logM) - 1)) << H.permLogC) + (j >> logM);
   }
-  const double x = ((double)j - (double)(N - 1) * 0.5) * H.dx;
-  double ph = 0.0;
-  bool anyPoly = false;
+  // twiddles and terms of degree one and two in turns, cubic terms in radians
+  const int u = 2 * j - N + 1;
+  const double inv4N = 0.25 / (double)N;
+  const LinTurns L = lin_turns(H.logN);
+  Turns<double2> p;
+  double cubic = 0.0;
+  bool anyTurns = false, anyCubic = false;
   double2 f = make_double2(1.0, 0.0);
   for (int t = H.term0; t < H.term0 + H.nTerms; ++t) {
     const TableTerm& D = B.term[t];
     if (D.kind == kTermPoly) {
-      double v;
-      if (D.power == 1) v = D.coeff * x;
-      else if (D.power == 2) v = D.coeff * x * x;
-      else v = D.coeff * x * x * x;
       const bool neg = (D.ctrlMode == 1 && ((b >> D.ctrlLocal) & 1)) || (D.ctrlMode == 2 && ((j >> D.ctrlLocal) & 1));
-      ph += neg ? -v : v;
-      anyPoly = true;
+      const double c = neg ? -D.coeff : D.coeff;
+      if (D.power == 1) {
+        double ch, cl;
+        Turns<double2>::scale(c, L.hi, L.lo, ch, cl);
+        p.add(ch, cl, (double)u);
+        anyTurns = true;
+      } else if (D.power == 2) {
+        p.add(c * inv4N, 0.0, (double)u * (double)u);
+        anyTurns = true;
+      } else {
+        const double x = 0.5 * (double)u * H.dx;
+        cubic += c * x * x * x;
+        anyCubic = true;
+      }
     } else if (D.kind == kTermFtTw) {
-      const long long n = N;
-      const long long m = ((n - 1) * (2LL * j - n + 1)) & (4 * n - 1);  // mod 4N, N a power of two
-      double s, c;
-      sincospi((double)(D.sign) * (double)m / (double)(2 * n), &s, &c);
-      f = dmul(f, make_double2(c, s));
+      const long long n = N;  // (N-1) u mod 4N, N a power of two
+      const long long m = (((n - 1) * u + 2 * n) & (4 * n - 1)) - 2 * n;
+      p.add_hi((double)D.sign * (double)m * inv4N);
+      anyTurns = true;
     } else if (D.kind == kTermBit) {
       f = dmul(f, ((j >> D.bit) & 1) ? D.g1 : D.g0);
     }
   }
-  if (anyPoly) {
+  if (anyTurns) f = dmul(p.root(), f);
+  if (anyCubic) {
     double s, c;
-    sincos(ph, &s, &c);
+    sincos(cubic, &s, &c);
     f = dmul(make_double2(c, s), f);
   }
   H.out[e] = f;

@@ -808,7 +808,6 @@ static cudaError_t launch_rowq_t(Context* ctx, const void* in, void* out, const 
 }
 
 // ---------------------------------------------------------------- host side
-int row_log_tile(int precision) { return precision == kC128 ? 12 : 13; }
 
 bool row_eligible(Context* ctx, int reg) {
   if (ctx->flw[reg] != 0) return false;
@@ -1048,7 +1047,11 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
     // have uncontrolled c x^2 terms too (finite ones: the phases are reduced mod 1).
     {
       const int lo = ctx->flw[reg], hi = lo + q;
-      bool linOnly = (useC || toRowr) && !regTerms.empty();
+      // (Short registers, tiny states and 2^8-point columns in complex128 keep the table: its
+      // entries are rounded once, as their twiddles are, where a running product of 8 doubles
+      // a transform's error; the loads take as long as the sines and cosines there.)
+      const bool tables = ctx->precision == kC128 && !useC && (q < 8 || rowr_tiny(ctx) || (col && q == 8));
+      bool linOnly = (useC || toRowr) && !tables && !regTerms.empty();
       const bool quads = toRowr && rowr_quads(ctx, q, col);
       int nPl = 0;
       for (const Term& t : regTerms) {
@@ -1081,7 +1084,6 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
       }
       D.regC = (double)((1 << q) - 1) * 0.5;
       D.regDx = ctx->dx[reg];
-      D.linTurns = ctx->dx[reg] / (4.0 * CVDV_PI);
     }
     if (!regTerms.empty()) {
       double2* tab = (double2*)arena_alloc(ctx, ((size_t)1 << (q + D.nCtrl)) * sizeof(double2));
@@ -1165,7 +1167,7 @@ bool launch_row_program(Context* ctx, int reg, const std::vector<HostRowOp>& ops
       return false;
     }
     if (rowSums && !col) {
-      const int logE = rowr_log_e(ctx->precision == kC128, q, rowr_small(ctx));
+      const int logE = rowr_log_e(ctx->precision == kC128, q, rowr_small(ctx), rowr_tiny(ctx));
       const int tpr = 1 << (q - logE);
       P.rowSums = ctx->rowSums;
       ctx->rowSumParts = tpr < 32 ? 1 : tpr / 32;

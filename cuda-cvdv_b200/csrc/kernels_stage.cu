@@ -20,6 +20,7 @@
 #include "../../include/cvdv.h"
 #include "cvdv_internal.cuh"
 #include "row_fft.cuh"
+#include "turns.cuh"
 
 namespace cvdv {
 
@@ -77,14 +78,6 @@ __device__ __forceinline__ C phase_factor(const CvdvBatchPhase& P, int j, int N,
   return mk(sc * c, sc * s);
 }
 
-// q m mod 1 (in -1/2 .. 1/2) for a phase of q m turns, m an integer that a double holds
-__device__ __forceinline__ double stage_turns(double q, double m) { return fma(q, m, -rint(q * m)); }
-__device__ __forceinline__ double2 turn_factor(double p) {
-  double s, c;
-  sincospi(2.0 * p, &s, &c);
-  return make_double2(c, s);
-}
-
 // A phase without a cubic term on the points t + k TPR of a row.  With u = 2 j - N + 1 and
 // dx^2 = 2 pi / N its turns are a quadratic in the integer u,
 //   tw (N-1) u / (4N) + (g0 + z h0) / 2pi + (a1 + z b1) dx u / 4pi + (a2 + z b2) u^2 / (4N),
@@ -94,37 +87,57 @@ __device__ __forceinline__ double2 turn_factor(double p) {
 // polynomial per point took about 25 FP64 operations, the conversions of its integers
 // and a fast sine and cosine each, about as long as the transforms between the phases;
 // this takes 8, and is exact to FP64 where the fast intrinsic was to 4e-7.
-// 96 circuits of 50 gates: 3.42 -> 3.30 ms, error 9.3e-6 -> 4.1e-6.
+// 96 circuits of 50 gates: 3.42 -> 3.30 ms, error 9.3e-6 -> 4.1e-6.  In complex128 the turns
+// are kept in two words (turns.cuh): a displacement on 2^11 points 3.0e-15 (per point) -> 1.2e-15.
 template <typename C, int LOGN, int LOGE>
 __device__ __forceinline__ void phase_run(C (&v)[1 << LOGE], const CvdvBatchPhase& P, int t, double zs, double2* kq) {
   constexpr int E = 1 << LOGE, N = 1 << LOGN, TPR = N >> LOGE, LANES = TPR < 32 ? TPR : 32;
   constexpr double inv4N = 1.0 / (4.0 * N);
   const int u0 = 2 * t - N + 1;
-  const double dx = sqrt(2.0 * M_PI / (double)N);
-  const double lin = (P.a1 + zs * P.b1) * (dx / (4.0 * M_PI)), q = (P.a2 + zs * P.b2) * inv4N;
-  // tw (N-1) u mod 4N in integers
+  constexpr LinTurns L = lin_turns(LOGN);
+  constexpr double perTurn = 0.5 / M_PI, perTurnLo = -9.839338337591243e-18;  // 1 / (2 pi) in two words
+  double linH, linL, constH, constL;
+  Turns<C>::scale(P.a1 + zs * P.b1, L.hi, L.lo, linH, linL);
+  Turns<C>::scale(P.g0 + zs * P.h0, perTurn, perTurnLo, constH, constL);
+  const double q = (P.a2 + zs * P.b2) * inv4N;
+  // tw (N-1) u / (4N) turns, in -1/2 .. 1/2
   const int w = (P.tw * (N - 1)) & (4 * N - 1);
-  double p0 = (double)((int)((long long)w * u0) & (4 * N - 1)) * inv4N + stage_turns(lin, (double)u0) +
-              (P.g0 + zs * P.h0) * (0.5 / M_PI);
-  double p1 = (double)((int)((long long)w * (2 * TPR)) & (4 * N - 1)) * inv4N + stage_turns(lin, 2.0 * TPR);
+  auto twiddle = [&](int u) {
+    return (double)(((int)((long long)w * u + 2 * N) & (4 * N - 1)) - 2 * N) * inv4N;
+  };
+  Turns<C> p0, p1;
+  p0.add_hi(twiddle(u0));
+  p1.add_hi(twiddle(2 * TPR));
+  p0.add(linH, linL, (double)u0);
+  p1.add(linH, linL, 2.0 * TPR);
+  p0.add(constH, constL, 1.0);
   const bool quad = P.a2 != 0.0 || P.b2 != 0.0;  // the same for every row of the task
   if (quad) {
-    p0 += stage_turns(q, (double)u0 * (double)u0);
-    p1 += stage_turns(q, 4.0 * TPR * (double)u0);
+    p0.add(q, 0.0, (double)u0 * (double)u0);
+    p1.add(q, 0.0, 4.0 * TPR * (double)u0);
     __syncwarp();  // the last run's constants are read
     const int lane = t & (LANES - 1);
 #pragma unroll
-    for (int k = lane; k < E; k += LANES) kq[k] = turn_factor(stage_turns(q, 4.0 * TPR * TPR * (double)(k * k)));
+    for (int k = lane; k < E; k += LANES) {
+      Turns<C> pk;
+      pk.add(q, 0.0, 4.0 * TPR * TPR * (double)(k * k));
+      kq[k] = pk.root();
+    }
     __syncwarp();
   }
-  double2 f = turn_factor(p0);
+  double2 f = p0.root();
   f.x *= P.scale;
   f.y *= P.scale;
-  const double2 st = turn_factor(p1);
+  const double2 st = p1.root();
+  // in complex128 from the eighth point's factor anew: a step's rounding is repeated
+  // 7 + 1 times at most instead of 15
+  constexpr bool ANCHOR = E >= 16 && sizeof(C) == sizeof(double2);
+  double2 eighth = f;
+  if constexpr (ANCHOR) eighth = dmul(f, p1.times(8.0).root());
 #pragma unroll
   for (int k = 0; k < E; ++k) {
     v[k] = cmul(v[k], fromd<C>(quad ? dmul(f, kq[k]) : f));
-    f = dmul(f, st);
+    f = ANCHOR && k == 7 ? eighth : dmul(f, st);
   }
 }
 

@@ -177,9 +177,80 @@ __device__ __forceinline__ C tw2(const double2* lo, const double2* hi, int e) {
   return fromd<C>(w);
 }
 
-template <typename C, int DIR, int LOGM, int LOGRAD, int LOGNS, int LOGE>
-__device__ __forceinline__ void rr_butterflies(C (&v)[1 << LOGE], int t, const double2* lo,
-                                               const double2* hi) {
+// Where a transform's twiddles come from.  SplitTw: the split tables, one product and a
+// tree of powers per butterfly.  FullTw: w_M^e for all e < M in shared memory, each
+// rounded once.  StageTw: the same, in the order in which the stages read them: entry
+// u ns + jm is w_(ns R)^(u jm) of the stage of radix R after ns points' worth of stages
+// (1 <= u < R, jm < ns), so a warp reads consecutive entries (by e, a stage's strides are
+// powers of two and most lanes' entries share a bank: a rotation, a displacement and a squeeze
+// of a 2^11-point complex128 state take 49 us instead of 41, of a complex64 one of 2^12 58
+// instead of 46).
+struct SplitTw {
+  static constexpr bool kByStage = false;
+  const double2 *lo, *hi;
+};
+template <typename C>
+struct FullTw {
+  static constexpr bool kByStage = false;
+  const C* w;
+};
+template <typename C>
+struct StageTw {
+  static constexpr bool kByStage = true;
+  const C* w;
+};
+template <int DIR, typename C>
+__device__ __forceinline__ C tw_dir(C w) {
+  return DIR > 0 ? w : mk(w.x, -w.y);
+}
+// log2 of a full stage's radix, by the amplitudes a thread keeps
+__host__ __device__ constexpr int rr_log_radix(int logE) { return logE >= 5 ? 5 : (logE == 3 ? 3 : 4); }
+// exponent of w_M at entry y of a StageTw table (0 below the second stage's first entry)
+template <int LOGM, int LOGE>
+__device__ __forceinline__ int stage_tw_exponent(int y) {
+  constexpr int LR = rr_log_radix(LOGE);
+  int e = 0;
+#pragma unroll
+  for (int logNs = LR; logNs < LOGM; logNs += LR) {
+    const int logR = LOGM - logNs < LR ? LOGM - logNs : LR;
+    if (y >> logNs) e = ((y >> logNs) * (y & ((1 << logNs) - 1))) << (LOGM - logNs - logR);
+  }
+  return e;
+}
+
+// x[u] *= w_M^(e u) for u < RAD
+template <typename C, int DIR, int RAD>
+__device__ __forceinline__ void stage_powers(C (&x)[RAD], const SplitTw& T, int e) {
+  // powers w^u as a tree (w^(u + 2^j) = w^u w^(2^j)); for radix 32 the upper
+  // half is formed as it is applied, so only 17 powers are live at once
+  constexpr int RT = RAD > 16 ? 16 : RAD;
+  C w[RT + 1];
+  w[1] = tw2<C, DIR>(T.lo, T.hi, e);
+#pragma unroll
+  for (int p = 1; p < RT / 2; p <<= 1) {
+    w[2 * p] = cmul(w[p], w[p]);
+#pragma unroll
+    for (int u = 1; u < p; ++u) w[p + u] = cmul(w[p], w[u]);
+  }
+#pragma unroll
+  for (int u = RT / 2 + 1; u < RT; ++u) w[u] = cmul(w[RT / 2], w[u - RT / 2]);
+  if constexpr (RAD > 16) w[16] = cmul(w[8], w[8]);
+#pragma unroll
+  for (int u = 1; u < RT; ++u) x[u] = cmul(x[u], w[u]);
+  if constexpr (RAD > 16) {
+    x[16] = cmul(x[16], w[16]);
+#pragma unroll
+    for (int u = 17; u < RAD; ++u) x[u] = cmul(x[u], cmul(w[16], w[u - 16]));
+  }
+}
+template <typename C, int DIR, int RAD>
+__device__ __forceinline__ void stage_powers(C (&x)[RAD], const FullTw<C>& T, int e) {
+#pragma unroll
+  for (int u = 1; u < RAD; ++u) x[u] = cmul(x[u], tw_dir<DIR>(T.w[e * u]));
+}
+
+template <typename C, int DIR, int LOGM, int LOGRAD, int LOGNS, int LOGE, typename TW>
+__device__ __forceinline__ void rr_butterflies(C (&v)[1 << LOGE], int t, const TW& tw) {
   constexpr int E = 1 << LOGE, RAD = 1 << LOGRAD, NB = E / RAD, TPR = 1 << (LOGM - LOGE);
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
@@ -188,27 +259,12 @@ __device__ __forceinline__ void rr_butterflies(C (&v)[1 << LOGE], int t, const d
     for (int u = 0; u < RAD; ++u) x[u] = v[b + NB * u];
     if constexpr (LOGNS > 0) {
       const int jm = (t + b * TPR) & ((1 << LOGNS) - 1);
-      // w_{ns R}^{jm u} = w_M^{(jm u) << (LOGM - LOGNS - LOGRAD)}; powers as a tree
-      // powers w^u as a tree (w^(u + 2^j) = w^u w^(2^j)); for radix 32 the upper
-      // half is formed as it is applied, so only 17 powers are live at once
-      constexpr int RT = RAD > 16 ? 16 : RAD;
-      C w[RT + 1];
-      w[1] = tw2<C, DIR>(lo, hi, jm << (LOGM - LOGNS - LOGRAD));
+      // w_{ns R}^{jm u} = w_M^{(jm u) << (LOGM - LOGNS - LOGRAD)}
+      if constexpr (TW::kByStage) {
 #pragma unroll
-      for (int p = 1; p < RT / 2; p <<= 1) {
-        w[2 * p] = cmul(w[p], w[p]);
-#pragma unroll
-        for (int u = 1; u < p; ++u) w[p + u] = cmul(w[p], w[u]);
-      }
-#pragma unroll
-      for (int u = RT / 2 + 1; u < RT; ++u) w[u] = cmul(w[RT / 2], w[u - RT / 2]);
-      if constexpr (RAD > 16) w[16] = cmul(w[8], w[8]);
-#pragma unroll
-      for (int u = 1; u < RT; ++u) x[u] = cmul(x[u], w[u]);
-      if constexpr (RAD > 16) {
-        x[16] = cmul(x[16], w[16]);
-#pragma unroll
-        for (int u = 17; u < RAD; ++u) x[u] = cmul(x[u], cmul(w[16], w[u - 16]));
+        for (int u = 1; u < RAD; ++u) x[u] = cmul(x[u], tw_dir<DIR>(tw.w[(u << LOGNS) + jm]));
+      } else {
+        stage_powers<C, DIR, RAD>(x, tw, jm << (LOGM - LOGNS - LOGRAD));
       }
     }
     bfly<C, DIR, RAD>(x);
@@ -244,19 +300,23 @@ __device__ __forceinline__ void rr_exchange(C (&v)[1 << LOGE], C* smrow, int t) 
 struct NoHook {
   __device__ __forceinline__ void operator()() const {}
 };
+template <typename C, int DIR, int LOGM, int S, int LOGE, typename TW, typename H>
+__device__ __forceinline__ void rr_stages_tw(C (&v)[1 << LOGE], C* smrow, int t, const TW& tw, H after) {
+  constexpr int LR = rr_log_radix(LOGE);
+  constexpr int NF = LOGM / LR, REM = LOGM % LR;
+  if constexpr (S < NF) {
+    rr_butterflies<C, DIR, LOGM, LR, LR * S, LOGE>(v, t, tw);
+    if constexpr (S + 1 < NF || REM) rr_exchange<C, LOGM, LR, LR * S, LOGE, LR>(v, smrow, t);
+    if constexpr ((REM > 0 && S + 1 == NF) || (REM == 0 && S + 2 == NF)) after();
+    rr_stages_tw<C, DIR, LOGM, S + 1, LOGE>(v, smrow, t, tw, after);
+  } else if constexpr (REM > 0) {
+    rr_butterflies<C, DIR, LOGM, REM, LR * NF, LOGE>(v, t, tw);
+  }
+}
 template <typename C, int DIR, int LOGM, int S, int LOGE = 4, typename H = NoHook>
 __device__ __forceinline__ void rr_stages(C (&v)[1 << LOGE], C* smrow, int t, const double2* lo,
                                           const double2* hi, H after = H()) {
-  constexpr int LR = LOGE >= 5 ? 5 : (LOGE == 3 ? 3 : 4);  // log2 of the full stages' radix
-  constexpr int NF = LOGM / LR, REM = LOGM % LR;
-  if constexpr (S < NF) {
-    rr_butterflies<C, DIR, LOGM, LR, LR * S, LOGE>(v, t, lo, hi);
-    if constexpr (S + 1 < NF || REM) rr_exchange<C, LOGM, LR, LR * S, LOGE, LR>(v, smrow, t);
-    if constexpr ((REM > 0 && S + 1 == NF) || (REM == 0 && S + 2 == NF)) after();
-    rr_stages<C, DIR, LOGM, S + 1, LOGE, H>(v, smrow, t, lo, hi, after);
-  } else if constexpr (REM > 0) {
-    rr_butterflies<C, DIR, LOGM, REM, LR * NF, LOGE>(v, t, lo, hi);
-  }
+  rr_stages_tw<C, DIR, LOGM, S, LOGE>(v, smrow, t, SplitTw{lo, hi}, after);
 }
 
 // ---------------------------------------------------------------- one CTA exchange
@@ -267,17 +327,21 @@ __device__ __forceinline__ void rr_stages(C (&v)[1 << LOGE], C* smrow, int t, co
 // with w^4 and w^16, as with the radix-16 stages (complex64 2.5e-6, 1.7e-6, 2.1e-6).  For radix 32
 // the upper half is formed as it is applied, so only 17 powers are live at once.
 template <typename C, int DIR, int RAD>
-__device__ __forceinline__ void mul_powers(C (&x)[RAD], const double2* lo, const double2* hi, int e) {
+__device__ __forceinline__ void mul_powers(C (&x)[RAD], const FullTw<C>& T, int e) {
+  stage_powers<C, DIR, RAD>(x, T, e);
+}
+template <typename C, int DIR, int RAD>
+__device__ __forceinline__ void mul_powers(C (&x)[RAD], const SplitTw& T, int e) {
   constexpr int RT = RAD > 16 ? 16 : RAD;
   C w[RT + 1];
 #pragma unroll
   for (int p = 1; p < RT; p <<= 1) {
-    if (p == 1 || (p == 4 && sizeof(C) == 16)) w[p] = tw2<C, DIR>(lo, hi, e * p);
+    if (p == 1 || (p == 4 && sizeof(C) == 16)) w[p] = tw2<C, DIR>(T.lo, T.hi, e * p);
     else w[p] = cmul(w[p / 2], w[p / 2]);
 #pragma unroll
     for (int u = 1; u < p; ++u) w[p + u] = cmul(w[p], w[u]);
   }
-  if constexpr (RAD > 16) w[16] = tw2<C, DIR>(lo, hi, e * 16);
+  if constexpr (RAD > 16) w[16] = tw2<C, DIR>(T.lo, T.hi, e * 16);
 #pragma unroll
   for (int u = 1; u < RT; ++u) x[u] = cmul(x[u], w[u]);
   if constexpr (RAD > 16) {
@@ -318,13 +382,12 @@ struct RrTwo {
   static constexpr int LINE = LOGI == 0 ? LINE0 : LINE0 + ((W / I > 1 ? W / I : 1) - LINE0 % W + W) % W;
 };
 
-template <typename C, int DIR, int LOGM, int LOGE, int LOGI, typename H = NoHook>
-__device__ __forceinline__ void rr_two(C (&v)[1 << LOGE], C* line, int t, int& tau, const double2* lo,
-                                       const double2* hi, H after = H()) {
+template <typename C, int DIR, int LOGM, int LOGE, int LOGI, typename TW, typename H = NoHook>
+__device__ __forceinline__ void rr_two(C (&v)[1 << LOGE], C* line, int t, int& tau, const TW& tw, H after = H()) {
   using S = RrTwo<C, LOGM, LOGE, LOGI>;
   constexpr int E = S::E, G = S::G, EG = E / G;
   bfly<C, DIR, E>(v);
-  mul_powers<C, DIR, E>(v, lo, hi, tau);
+  mul_powers<C, DIR, E>(v, tw, tau);
   __syncthreads();  // the line is free: every group has read its last exchange
   {
     C* p = line + tau + S::PAD * (tau >> LOGE);
@@ -338,7 +401,7 @@ __device__ __forceinline__ void rr_two(C (&v)[1 << LOGE], C* line, int t, int& t
   for (int j = 0; j < E; ++j) v[j] = reg[g + G * j + S::PAD * ((G * j) >> LOGE)];
   bfly<C, DIR, E>(v);
   if constexpr (G > 1) {
-    mul_powers<C, DIR, E>(v, lo, hi, g << LOGE);
+    mul_powers<C, DIR, E>(v, tw, g << LOGE);
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < E; ++c) reg[c * (G + 1) + g] = v[c];

@@ -6,6 +6,7 @@
 
 #include "cvdv_internal.cuh"
 #include "row_fft.cuh"
+#include "turns.cuh"
 
 namespace cvdv {
 
@@ -39,7 +40,6 @@ struct RowDiag {
   int ftSign;
   int hasQuad;  // k_rowr, 32 amplitudes a thread: the run also has c2 x^2 (uncontrolled terms' sum)
   double c2;
-  double linTurns;         // turns per unit of u = 2 n - N + 1 of the phase x_n: dx / (4 pi)
   double2 quad[kMaxRowE];  // exp(2 pi i c2 TPR^2 k^2 / N) for the kernel's E amplitudes a thread
   int nPl;
   double plC[2];
@@ -94,10 +94,6 @@ __device__ __forceinline__ double2 ft_tw_ratio(long long d, long long N, int s) 
   return make_double2(c, sn);
 }
 
-// q m mod 1 (in -1/2 .. 1/2) for a phase of q m turns, m an integer that a double holds:
-// one rounding, however many turns
-__device__ __forceinline__ double turns(double q, double m) { return fma(q, m, -rint(q * m)); }
-
 // A diagonal run on the amplitudes t + k TPR (k < E) of a row.  Register terms of
 // degree up to two, transform twiddles and bilinear terms need no table: with
 // u = 2 n - N + 1 and x_n = dx u / 2, dx^2 = 2 pi / N, they are
@@ -116,6 +112,13 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
   const double2 rs = D.hasRowF ? eval_factor(D.rowF, rowBase) : make_double2(1.0, 0.0);
   // running factor of element t + k TPR: rs times the linear phase, advanced by st per k
   double2 f = rs, st = make_double2(1.0, 0.0);
+  // In complex128 the product starts anew from every eighth element's, so a step's rounding
+  // is repeated 7 + 3 times at most instead of 31 (32 amplitudes a thread): a transform of
+  // random amplitudes on 2^13 points 1.6e-15 -> 0.7e-15, for a third sine and cosine a run
+  // (rotation, displacement and squeeze on the columns of a 2^24 state 0.85 -> 0.88 ms).
+  constexpr bool ANCHORS = E >= 16 && sizeof(C) == sizeof(double2);
+  constexpr int kAnchor = 8;
+  double2 anchor = rs, stA = make_double2(1.0, 0.0);
   const bool lin = D.nLin || D.nPl || D.ftSign || (QUAD && D.hasQuad);
   if (lin) {
     double a = 0.0;
@@ -128,23 +131,38 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
     }
     for (int k = 0; k < D.nPl; ++k)
       a += (D.plCtrl[k] >= 0 && ((rowBase >> D.plCtrl[k]) & 1ull)) ? -D.plC[k] : D.plC[k];
-    a *= D.linTurns;
+    constexpr LinTurns L = lin_turns(LOGM);
+    double ah, al;
+    Turns<C>::scale(a, L.hi, L.lo, ah, al);
     const int u0 = 2 * t - N + 1;
     // s (N-1) u mod 4N in integers: at most 3 2^28 for the runs of a program
     constexpr double inv4N = 1.0 / (4.0 * N);
     const int w = (D.ftSign * (N - 1)) & (4 * N - 1);
-    double p0 = (double)((int)((long long)w * u0) & (4 * N - 1)) * inv4N + turns(a, (double)u0);
-    double p1 = (double)((int)((long long)w * (2 * TPR)) & (4 * N - 1)) * inv4N + turns(a, 2.0 * TPR);
+    auto twiddle = [&](int u) {  // s (N-1) u / (4N) turns, in -1/2 .. 1/2
+      return (double)(((int)((long long)w * u + 2 * N) & (4 * N - 1)) - 2 * N) * inv4N;
+    };
+    Turns<C> p0, p1;
+    p0.add_hi(twiddle(u0));
+    p1.add_hi(twiddle(2 * TPR));
+    p0.add(ah, al, (double)u0);
+    p1.add(ah, al, 2.0 * TPR);
     if (QUAD && D.hasQuad) {
       const double q = D.c2 * inv4N;
-      p0 += turns(q, (double)u0 * (double)u0);
-      p1 += turns(q, 4.0 * TPR * (double)u0);
+      p0.add(q, 0.0, (double)u0 * (double)u0);
+      p1.add(q, 0.0, 4.0 * TPR * (double)u0);
     }
-    double s0, c0;
-    sincospi(2.0 * p0, &s0, &c0);
-    sincospi(2.0 * p1, &st.y, &st.x);
-    f = dmul(rs, make_double2(c0, s0));
+    f = dmul(rs, p0.root());
+    st = p1.root();
+    if constexpr (ANCHORS) {
+      anchor = f;
+      stA = p1.times(kAnchor).root();
+    }
   }
+  // on to the next element's factor, from the last anchor's every kAnchor elements
+  auto next = [&](int k) {
+    if (ANCHORS && (k + 1) % kAnchor == 0) f = anchor = dmul(anchor, stA);
+    else f = dmul(f, st);
+  };
   if (D.tab) {
     int seg = 0;
     for (int c = 0; c < D.nCtrl; ++c) seg |= (int)((rowBase >> D.ctrlShift[c]) & 1ull) << c;
@@ -157,7 +175,7 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         if (D.hasRowF || lin) w[k] = dmul(w[k], f);
-        if (lin) f = dmul(f, st);
+        if (lin) next(k0 + k);
         v[k0 + k] = cmul(v[k0 + k], fromd<C>(w[k]));
       }
     }
@@ -165,13 +183,13 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
 #pragma unroll
     for (int k = 0; k < E; ++k) {
       v[k] = cmul(v[k], fromd<C>(dmul(f, D.quad[k])));
-      f = dmul(f, st);
+      next(k);
     }
   } else if (lin) {
 #pragma unroll
     for (int k = 0; k < E; ++k) {
       v[k] = cmul(v[k], fromd<C>(f));
-      f = dmul(f, st);
+      next(k);
     }
   } else if (D.hasRowF) {
     const C c = fromd<C>(rs);
@@ -283,7 +301,7 @@ __device__ __forceinline__ void row_sum_part(const C (&v)[E], double* out) {
 // A state of fewer rows than a CTA holds (nRows < 2^LOGR, both powers of two) runs
 // as one tile whose surplus thread groups repeat its rows: they read the same
 // input and write the same values.
-template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
+template <typename C, int LOGM, int LOGR, int LOGE, bool COL, bool FULL>
 __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOGR, LOGE>() ? 1 : 2)
     k_rowr(const C* __restrict__ in, C* __restrict__ out, uint64_t nTiles, const __grid_constant__ RowProgram P) {
   constexpr int E = 1 << LOGE, M = 1 << LOGM, TPR = M >> LOGE, NT = TPR << LOGR;
@@ -295,8 +313,7 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOG
   constexpr bool PF = COL && ONE && TWO;  // the next tile is copied ahead
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
-  double2* lo = reinterpret_cast<double2*>(sm + (RS << LOGR));  // w_M^e, e < 64
-  double2* hi = lo + 64;                                         // w_M^(64 h), h < M / 64
+  C* tws = sm + (RS << LOGR);  // the twiddles
   const int tid = threadIdx.x;
   // column form: the CTA's 2^LOGR adjacent columns interleave lane by lane, so a
   // warp's load covers 32 / 2^LOGR points of every column in runs of 2^LOGR
@@ -307,10 +324,24 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOG
   if constexpr (LOGM <= 8) row &= P.rowMask;  // (longer rows: LOGR = 0 where rows are few)
 
   const int scM = P.logTwN - LOGM;
-  for (int i = tid; i < rr_tw_slots(LOGM); i += NT) {
-    const int e = i < 64 ? i : (i - 64) << 6;
-    if (e < M) lo[i] = __ldg(P.tw + ((size_t)e << scM));  // lo and hi are one array
-  }
+  const auto tw = [&] {
+    if constexpr (FULL && TWO) {
+      for (int e = tid; e < M; e += NT) tws[e] = fromd<C>(__ldg(P.tw + ((size_t)e << scM)));
+      return FullTw<C>{tws};
+    } else if constexpr (FULL) {
+#pragma unroll 8
+      for (int y = tid; y < M; y += NT)
+        tws[y] = fromd<C>(__ldg(P.tw + ((size_t)stage_tw_exponent<LOGM, LOGE>(y) << scM)));
+      return StageTw<C>{tws};
+    } else {
+      double2* lo = reinterpret_cast<double2*>(tws);  // w_M^e, e < 64, then w_M^(64 h), h < M / 64
+      for (int i = tid; i < rr_tw_slots(LOGM); i += NT) {
+        const int e = i < 64 ? i : (i - 64) << 6;
+        if (e < M) lo[i] = __ldg(P.tw + ((size_t)e << scM));
+      }
+      return SplitTw{lo, lo + 64};
+    }
+  }();
   __syncthreads();
   // copies a tile's amplitudes into sm in thread order (sm[tid + k NT] becomes v[k])
   auto fetch = [&](uint64_t tile) {
@@ -369,11 +400,11 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOG
           }
         };
         const HookIf<decltype(next)> hook{PF && more && o == lastFft, next};
-        if (op.dir > 0) rr_two<C, 1, LOGM, LOGE, LOGI>(v, smrow, t, tau, lo, hi, hook);
-        else rr_two<C, -1, LOGM, LOGE, LOGI>(v, smrow, t, tau, lo, hi, hook);
+        if (op.dir > 0) rr_two<C, 1, LOGM, LOGE, LOGI>(v, smrow, t, tau, tw, hook);
+        else rr_two<C, -1, LOGM, LOGE, LOGI>(v, smrow, t, tau, tw, hook);
       } else {
-        if (op.dir > 0) rr_stages<C, 1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
-        else rr_stages<C, -1, LOGM, 0, LOGE>(v, smrow, t, lo, hi);
+        if (op.dir > 0) rr_stages_tw<C, 1, LOGM, 0, LOGE>(v, smrow, t, tw, NoHook());
+        else rr_stages_tw<C, -1, LOGM, 0, LOGE>(v, smrow, t, tw, NoHook());
       }
     }
     if constexpr (!COL) {
@@ -392,17 +423,15 @@ inline int rowr_max_log(int precision) { return precision == kC128 ? 13 : 14; }
 // log2 of the amplitudes a thread keeps of a row of 2^logM points.  Rows of 2^13 and 2^14
 // points: 32 (256 / 512 threads; two exchanges in shared memory per transform instead of
 // three: complex128 [13, 13] network rows 8.4 against 9.6 ms, columns 12.6 against 13.9).
-// Otherwise 16, and in complex128 8 for rows shorter than 2^8 points and, up to 2^12, for
-// small states (below).  Complex64 stays at 16: a transform's norm loses 4e-8 there and
-// 8e-8 with radix-8 stages, whose constants' float roundings all shrink it (the error
-// of a 60-gate circuit is this drift).
-constexpr int rowr_log_e(bool c128, int logM, bool small) {
-  return logM >= 13 ? 5 : c128 && (logM < 8 || small) ? 3 : 4;
+// Otherwise 16, and up to 2^12 points 8 for tiny states and, in complex128, for small ones
+// (below) and for rows shorter than 2^8 points.
+constexpr int rowr_log_e(bool c128, int logM, bool small, bool tiny) {
+  return logM >= 13 ? 5 : tiny || (c128 && (small || logM < 8)) ? 3 : 4;
 }
 
 template <typename C, int LOGM>
 struct RrShape {
-  static constexpr int LOGE = rowr_log_e(sizeof(C) == sizeof(double2), LOGM, false);
+  static constexpr int LOGE = rowr_log_e(sizeof(C) == sizeof(double2), LOGM, false, false);
   static constexpr int LOGR = LOGM < 8 ? 7 - (LOGM - LOGE) : LOGM - LOGE < 8 ? 8 - (LOGM - LOGE) : 0;
 };
 
@@ -412,9 +441,23 @@ struct RrShape {
 // one CTA's chain, and more warps and CTAs shorten it.  A rotation, a displacement and a
 // squeeze on 2^10-point rows of a complex128 state, small shape against full tiles: 26
 // against 39 us at 2^18 amplitudes, 40 and 39 at 2^19, 56 and 52 at 2^20 (columns 28 / 39,
-// 45 / 38, 70 / 48; complex64 rows 31 / 34, 31 / 33, 49 / 39).
+// 45 / 38, 70 / 48; complex64 rows 31 / 34, 31 / 33, 49 / 39).  States below a k_row tile
+// (rowr_tiny) take 8 amplitudes a thread in both precisions, on twiddles rounded once: the
+// radix-8 arithmetic of the tile passes (in complex64 the norm drifts by -3e-8 a transform of
+// 2^12 points, by -4e-8 with radix-16 stages).
+inline int row_log_tile(int precision) { return precision == kC128 ? 12 : 13; }  // of a k_row CTA
 constexpr int kRowrSmallLog = 19;
 inline bool rowr_small(Context* ctx) { return ctx->totalQbt < kRowrSmallLog; }
+inline bool rowr_tiny(Context* ctx) { return ctx->totalQbt < row_log_tile(ctx->precision); }
+
+// Whether shapes of 2^logM-point rows (columns) keep all twiddles, each rounded once: short
+// registers and 2^8-point columns, where the table is 4 KB at most.  (Tiny states do at every
+// length.)  A power tree multiplies the rounding of w by up to 15.  Relative error of a
+// transform of random amplitudes, tree -> table: 2^8-point columns 6.6e-16 -> 2.2e-16 in
+// complex128, 2.2e-7 -> 1.1e-7 in complex64; a 2^10-point state 4.5e-16 -> 2.3e-16 and
+// 2.2e-7 -> 1.2e-7.  The other shapes keep the tree: their tables would take the shared
+// memory of the rows.
+constexpr bool rr_full(int logM, bool col) { return logM < 8 || (col && logM == 8); }
 
 // The constants of the quadratic runs for a kernel of 2^logE amplitudes a thread:
 // 4 c2 TPR^2 k^2 / (4 N) turns, reduced mod 1 before the 64-bit sine and cosine.
@@ -425,19 +468,24 @@ inline void fill_quads(RowProgram& P, int logM, int logE) {
     if (!D.hasQuad) continue;
     const double q = D.c2 / N;
     for (int k = 0; k < 1 << logE; ++k) {
-      const double m = tpr2 * (double)(k * k), p = fma(q, m, -rint(q * m));
-      D.quad[k] = make_double2(cos(2.0 * CVDV_PI * p), sin(2.0 * CVDV_PI * p));
+      // (the last quarter turns are exact, so the angle keeps its digits)
+      const double m = tpr2 * (double)(k * k), p = fma(q, m, -rint(q * m)), n = rint(4.0 * p);
+      const double ang = 2.0 * CVDV_PI * (p - 0.25 * n), c = cos(ang), s = sin(ang);
+      const int quarter = (int)n & 3;
+      D.quad[k] = quarter == 0 ? make_double2(c, s) : quarter == 1 ? make_double2(-s, c)
+                : quarter == 2 ? make_double2(-c, -s) : make_double2(s, -c);
     }
   }
 }
 
-template <typename C, int LOGM, int LOGR, int LOGE, bool COL>
+template <typename C, int LOGM, int LOGR, int LOGE, bool COL, bool FULL>
 static cudaError_t launch_rowr_s(Context* ctx, const void* in, void* out, const RowProgram& program) {
   RowProgram P = program;
   if constexpr (rr_quads<C, LOGM, LOGE, LOGR, COL>()) fill_quads(P, LOGM, LOGE);
   constexpr int NT = 1 << (LOGM - LOGE + LOGR);
-  const size_t smem = (size_t)rr_line_slots<C, LOGM, LOGE, LOGR, COL>() * (1 << LOGR) * sizeof(C) + rr_tw_slots(LOGM) * sizeof(double2);
-  auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL>;
+  const size_t smem = (size_t)rr_line_slots<C, LOGM, LOGE, LOGR, COL>() * (1 << LOGR) * sizeof(C) +
+                      (FULL ? sizeof(C) << LOGM : rr_tw_slots(LOGM) * sizeof(double2));
+  auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL, FULL>;
   static int resident = 0;  // CTAs per SM of this instantiation, asked once
   cudaError_t e = cudaSuccess;
   if (!resident) {
@@ -459,11 +507,15 @@ static cudaError_t launch_rowr_t(Context* ctx, const void* in, void* out, const 
   constexpr int LOGE = RrShape<C, LOGM>::LOGE, LOGR0 = RrShape<C, LOGM>::LOGR;
   // column form: at least two columns a CTA while it stays within 512 threads
   constexpr int LOGR = (COL && LOGR0 == 0 && (sizeof(C) << LOGM) < (128u << 10)) ? 1 : LOGR0;
-  if constexpr (LOGM >= 8 && LOGM <= 12) {
-    constexpr int SE = rowr_log_e(sizeof(C) == sizeof(double2), LOGM, true), SR = LOGM - SE < 5 ? 5 - (LOGM - SE) : 0;
-    if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, SR, SE, COL>(ctx, in, out, P);
+  if constexpr (LOGM <= 12) {
+    constexpr bool C128 = sizeof(C) == sizeof(double2);
+    constexpr int SR = LOGM < 8 ? 8 - LOGM : 0;  // (a warp at 8 amplitudes a thread)
+    if (rowr_tiny(ctx)) return launch_rowr_s<C, LOGM, SR, 3, COL, true>(ctx, in, out, P);
+    constexpr bool TWO_ROWS = !C128 && LOGM == 8;  // two rows fill a warp
+    if constexpr (LOGM >= 8)
+      if (rowr_small(ctx)) return launch_rowr_s<C, LOGM, TWO_ROWS, C128 ? 3 : 4, COL, rr_full(LOGM, COL)>(ctx, in, out, P);
   }
-  return launch_rowr_s<C, LOGM, LOGR, LOGE, COL>(ctx, in, out, P);
+  return launch_rowr_s<C, LOGM, LOGR, LOGE, COL, rr_full(LOGM, COL)>(ctx, in, out, P);
 }
 
 template <typename C, bool COL>
