@@ -68,9 +68,11 @@ def adaptive_loge(m: int, prec: int, tasks_per_stage: float) -> int:
     then the longest row task's latency, and fewer amplitudes a thread are more threads
     on a row.  Stages of 96 circuits (154 tasks, modes 2^8..2^13, complex64): 30 us with 16
     amplitudes a thread on the 2^13-point rows, 47 with 32; of 300 circuits (790 tasks): 86
-    and 83.  16 circuits (21 tasks, 2^10..2^12): 21 us with 8 amplitudes a thread, 26 with 16."""
+    and 83.  Below 74 tasks complex128 rows take 8; complex64 rows stay at 16, whose transforms
+    lose less of the norm: 12 circuits of 120 gates on 2^10 points are off by 5.1e-6, with 8
+    by 6.8e-6 (23.6 and 19.6 us a stage)."""
     e = default_loge(m, prec)
-    if tasks_per_stage < 74 and m <= 12:
+    if prec == 0 and tasks_per_stage < 74 and m <= 12:
         e = 3
     elif tasks_per_stage < 296:
         e = min(e, 4)

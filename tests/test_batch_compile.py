@@ -125,3 +125,16 @@ def test_program_record_limits_and_row_shapes():
     # a row task's amplitudes per thread: the row fits 512 threads; complex128 at most 16
     assert loge_options(8, 0) == [3, 4] and loge_options(14, 1) == [5]
     assert loge_options(13, 0) == [4] and loge_options(12, 1) == [3, 4, 5]
+
+
+def test_row_shapes_by_batch_size():
+    """Fewer amplitudes a thread for stages that do not fill the chip; complex64 keeps 16,
+    whose transforms lose less of the norm than radix-8 stages'."""
+    from cvdv_b200.batch import adaptive_loge
+    for m in range(8, 15):
+        for tasks in (1, 73.9, 74, 295.9, 296, 5000):
+            c64, c128 = adaptive_loge(m, 1, tasks), adaptive_loge(m, 0, tasks)
+            wide = 5 if m == 14 or (m == 13 and tasks >= 296) else 4  # (2^14 points need 32: 512 threads a row)
+            assert c64 == wide
+            if m <= 13:
+                assert c128 == (3 if tasks < 74 and m <= 12 else 4)
