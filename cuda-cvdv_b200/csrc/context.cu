@@ -726,14 +726,29 @@ static bool launch_product(Context* ctx, std::vector<const double2*>& arrs, int 
   return ok;
 }
 
+// What planning has come to.
+static FlushPlan::Reached planned(const Context* ctx) {
+  const FlushPlan& plan = *ctx->plan;
+  return {ctx->cur, !ctx->productPending && !ctx->seqProdLast && !plan.blocked && !plan.partial};
+}
+
+void plan_launch(Context* ctx, std::function<bool()> go) {
+  ctx->plan->launches.push_back({std::move(go), planned(ctx->parent ? ctx->parent : ctx)});
+}
+
 // Launches what has been planned since the last group: the tables, then the kernels.
 static bool issue_plan(Context* ctx) {
   FlushPlan& plan = *ctx->plan;
+  if (plan.failed) return false;
   bool ok = launch_tables(ctx, plan.tables);
-  for (size_t k = 0; ok && k < plan.launches.size(); ++k) ok = plan.launches[k]();
+  for (size_t k = 0; ok && k < plan.launches.size(); ++k) {
+    plan.reached = plan.launches[k].before;
+    ok = plan.launches[k].go();
+  }
+  if (ok) plan.reached = planned(ctx);
+  plan.failed = !ok;
   plan.tables.clear();
   plan.launches.clear();
-  plan.cur = ctx->cur;
   return ok;
 }
 
@@ -882,6 +897,7 @@ static bool plan_flush(Context* ctx) {
     if (blocked >= 0) {
       ctx->permReg = blocked;
       ctx->permLogC = rowc_log_cluster();
+      ctx->plan->blocked = true;
     }
   }
   const bool early = ops.size() >= kEarlyOps;
@@ -919,6 +935,7 @@ static bool plan_flush(Context* ctx) {
         ctx->permReg = op.rowReg;
         ctx->permLogC = rowc_log_cluster();
       }
+      ctx->plan->blocked = ctx->permReg >= 0;
       continue;
     }
     if (!op.st) {  // standalone diagonal run
@@ -950,16 +967,18 @@ bool flush(Context* ctx) {
   }
   if (ctx->plan) return plan_flush(ctx);  // a register's context: part of its parent's flush
   FlushPlan plan;
-  plan.cur = ctx->cur;
-  const bool product = ctx->productPending;
   ctx->plan = &plan;
-  const bool ok = plan_flush(ctx) && issue_plan(ctx);
+  plan.reached = planned(ctx);
+  const bool ok = plan_flush(ctx);
+  const bool out = issue_plan(ctx);  // (what was planned before an error too)
   ctx->plan = nullptr;
-  if (!ok) {
-    ctx->cur = plan.cur;  // what was planned but not launched has not moved the state
-    if (product) ctx->initialized = false;  // the product state was not formed, or only in part used
+  ctx->seqProdLast = ctx->seqProdOuter = nullptr;  // (left where an error came before the sequence)
+  if (!out) {
+    // what was planned but not launched has not moved the state
+    ctx->cur = plan.reached.cur;
+    if (!plan.reached.state) ctx->initialized = false;
   }
-  return ok;
+  return ok && out;
 }
 
 }  // namespace cvdv

@@ -237,11 +237,24 @@ struct TableJob {
 // What a flush will launch.  Planning allocates tables and fixes every kernel's
 // parameters (the ping-pong buffers alternate as the launches are planned).  The
 // planned launches go out in groups, each after one launch that builds its tables.
+// Every launch is kept with what the flush has come to before it, so that a flush that
+// fails there leaves the state of the launches that were accepted.
 struct FlushPlan {
+  struct Reached {
+    int cur;     // the buffer that holds the state
+    bool state;  // it holds one: the product formed, natural order, between passes of no transform
+  };
+  struct Launch {
+    std::function<bool()> go;
+    Reached before;
+  };
   std::vector<TableJob> tables;
-  std::vector<std::function<bool()>> launches;
+  std::vector<Launch> launches;
   size_t group = 1;      // launches that make the next group
-  int cur = 0;           // the buffer that holds the state after the groups that went out
+  Reached reached{};     // by the launches that went out
+  bool failed = false;   // one of them was refused
+  bool blocked = false;  // planning has come to a state in a cluster row kernel's blocked order
+  bool partial = false;  // ... to one between the passes of a transform
 };
 
 struct Context {
@@ -357,6 +370,7 @@ void harvest_timing(Context* ctx);
 // < 0), or, while a flush is being planned, keeps it for the flush to run.
 template <typename F>
 bool enqueue(Context* ctx, int kind, const char* what, F f);
+void plan_launch(Context* ctx, std::function<bool()> go);  // keeps a launch in ctx->plan
 extern std::atomic<unsigned long long> g_launches;
 
 void set_error(Context* ctx, int code, const char* fmt, ...);
@@ -465,7 +479,7 @@ bool enqueue(Context* ctx, int kind, const char* what, F f) {
     return cuda_ok(ctx, e, what);
   };
   if (!ctx->plan) return go();
-  ctx->plan->launches.emplace_back(std::move(go));
+  plan_launch(ctx, std::move(go));
   return true;
 }
 

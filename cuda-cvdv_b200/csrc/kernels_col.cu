@@ -316,6 +316,7 @@ static bool run_col_chain(Context* ctx, int reg, const std::vector<int>& dirs,
                                      : col_dispatch<float2>(ctx, in, out, logL, P, kind, d1, d2);
     });
     if (ok) ctx->cur ^= 1;
+    if (ok && ctx->plan && !ctx->parent) ctx->plan->partial = kind == kColFirst || kind == kColMiddle;
     return ok;
   };
   auto too_long = [&]() {

@@ -318,6 +318,7 @@ static bool run_passes(Context* ctx, const void* src, void* const* dsts, uint64_
           return cudaGetLastError();
         }))
       return false;
+    if (ctx->plan && !ctx->parent) ctx->plan->partial = !P.last && (ctx->plan->partial || outp == src);
     in = outp;
     logNs += P.logR;
   }

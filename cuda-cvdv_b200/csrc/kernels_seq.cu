@@ -394,7 +394,6 @@ bool launch_seq(Context* ctx, const std::vector<HostSeqOp>& ops) {
     P.prodLast = ctx->seqProdLast;
     P.prodOuter = ctx->seqProdOuter;
     P.prodQ = ctx->q[ctx->numReg - 1];
-    ctx->seqProdLast = ctx->seqProdOuter = nullptr;
   }
   int nd = 0;
   for (const HostSeqOp& h : ops) {
@@ -487,7 +486,7 @@ bool launch_seq(Context* ctx, const std::vector<HostSeqOp>& ops) {
   if (blocks > cap) blocks = cap;
   const bool narrow = ctx->totalQbt <= 31;  // every flat index fits 32 bits
   void* st = ctx->state();
-  return enqueue(ctx, kKSeq, "qubit-gate sequence launch", [=] {
+  const bool ok = enqueue(ctx, kKSeq, "qubit-gate sequence launch", [=] {
     if (ctx->precision == kC128) {
       if (narrow) seq_dispatch<double2, uint32_t>(ctx, st, nb, (unsigned)blocks, nSites, P);
       else seq_dispatch<double2, uint64_t>(ctx, st, nb, (unsigned)blocks, nSites, P);
@@ -497,6 +496,8 @@ bool launch_seq(Context* ctx, const std::vector<HostSeqOp>& ops) {
     }
     return cudaGetLastError();
   });
+  ctx->seqProdLast = ctx->seqProdOuter = nullptr;  // (formed, if it was to be)
+  return ok;
 }
 
 }  // namespace cvdv

@@ -1,0 +1,98 @@
+"""Host code of the library without a GPU, on a stand-in CUDA runtime (host_runtime.py)."""
+
+import ctypes
+
+import pytest
+
+from . import host_runtime
+
+
+@pytest.fixture(scope="module")
+def L(tmp_path_factory):
+    return host_runtime.load(tmp_path_factory.mktemp("host"))
+
+
+def context(L, qubits, precision=0):
+    h = L.cvdvCreateEx(len(qubits), (ctypes.c_int * len(qubits))(*qubits), precision)
+    L.cvdvClearError(h)
+    return h
+
+
+def error(L, h):
+    buf = ctypes.create_string_buffer(512)
+    return L.cvdvGetLastError(h, buf, 512), buf.value.decode()
+
+
+def set_state(L, h):
+    n = L.cvdvGetTotalSize(h)
+    L.cvdvSetStateFromDevicePtr(h, ctypes.create_string_buffer(16 * n))
+    assert error(L, h)[0] == 0
+
+
+def test_stand_in_runs_a_circuit(L):
+    h = context(L, [1, 10])
+    set_state(L, h)
+    before = L.fake_launches()
+    L.cvdvRotation(h, 1, 0.3)
+    L.cvdvFlush(h)
+    assert error(L, h) == (0, "") and L.fake_launches() > before
+    L.cvdvDestroy(h)
+
+
+@pytest.mark.parametrize("count", [3, 12])  # one group of launches, several
+def test_a_failed_launch_leaves_the_launched_prefix(L, count):
+    """Each parity gate is one launch into the other buffer: after a refused launch the
+    state is the buffer that the last accepted one wrote."""
+    for k in range(count + 1):
+        h = context(L, [2, 2])
+        set_state(L, h)
+        start = L.cvdvGetStateDevicePtr(h)
+        for _ in range(count):
+            L.cvdvParity(h, 0)
+        L.fake_fail_at(L.fake_launches() + k if k < count else -1)
+        L.cvdvFlush(h)
+        L.fake_fail_at(-1)
+        assert (error(L, h)[0] != 0) == (k < count)
+        L.cvdvClearError(h)
+        assert (L.cvdvGetStateDevicePtr(h) != start) == bool(k & 1), k
+        L.cvdvDestroy(h)
+
+
+def test_a_failed_launch_before_the_product_leaves_no_state(L):
+    """Two launches form the product of the register arrays: without them there is no
+    state, after them the gates that were launched count."""
+    for k in range(5):
+        h = context(L, [2, 2])
+        arrays = [ctypes.create_string_buffer(64) for _ in range(2)]
+        L.cvdvInitFromSeparable(h, (ctypes.c_void_p * 2)(*[ctypes.addressof(a) for a in arrays]), 2)
+        for _ in range(3):
+            L.cvdvParity(h, 0)
+        L.fake_fail_at(L.fake_launches() + k)
+        L.cvdvFlush(h)
+        L.fake_fail_at(-1)
+        assert error(L, h)[0] != 0
+        L.cvdvClearError(h)
+        L.cvdvGetNorm(h)
+        assert (error(L, h)[0] == 0) == (k >= 2), k
+        L.cvdvDestroy(h)
+
+
+def test_a_failed_launch_inside_a_transform_leaves_no_state(L):
+    """A transform of a 2^15-point column is two launches: between them neither buffer
+    holds a state."""
+    kernels, states = [], []
+    for k in range(8):
+        h = context(L, [15, 3])
+        set_state(L, h)
+        L.cvdvFtQ2P(h, 0)
+        L.fake_fail_at(L.fake_launches() + k)
+        L.cvdvFlush(h)
+        L.fake_fail_at(-1)
+        if error(L, h)[0] == 0:
+            break
+        kernels.append("k_colr" in L.fake_last_kernel().decode())
+        L.cvdvClearError(h)
+        L.cvdvGetNorm(h)
+        states.append(error(L, h)[0] == 0)
+        L.cvdvDestroy(h)
+    assert kernels[-2:] == [True, True] and states == [True] * (len(states) - 1) + [False]
