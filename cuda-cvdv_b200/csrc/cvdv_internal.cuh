@@ -217,6 +217,8 @@ struct TimingRec {
   int kind;
 };
 
+constexpr int kMaxDevices = 64;  // of one process, for what is kept per device
+
 struct Context;
 
 // A factor table to build: entry [seg][j] of register length 2^logN, seg over the

@@ -793,8 +793,8 @@ static cudaError_t launch_rowq_t(Context* ctx, const void* in, void* out, const 
   cfg.numAttrs = 1;
   // as many clusters as are resident at once (asked once per device), each
   // walking its share of the rows
-  static int clusters[64] = {};
-  const int dev = ctx->device >= 0 && ctx->device < 64 ? ctx->device : 0;
+  static int clusters[kMaxDevices] = {};
+  const int dev = ctx->device >= 0 && ctx->device < kMaxDevices ? ctx->device : 0;
   if (!clusters[dev]) {
     cfg.gridDim = dim3((unsigned)(NC * 1024));
     int n = 0;

@@ -270,6 +270,25 @@ __global__ void __launch_bounds__(kStageThreads, 1)
 
 using namespace cvdv;
 
+template <typename C>
+static cudaError_t launch_stage(void* states, const CvdvBatchTask* tasks, int nTasks, const CvdvBatchProgram* programs,
+                                int gridCtas, cudaStream_t s) {
+  const size_t smem = stage_smem<C>() + stage_quad_bytes();
+  // the shared-memory opt-in is set once per device (so later calls can be captured)
+  static std::atomic<bool> optedIn[kMaxDevices];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const bool known = dev >= 0 && dev < kMaxDevices;
+  if (!known || !optedIn[dev].load()) {
+    e = cudaFuncSetAttribute(k_batch_stage<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (known) optedIn[dev].store(true);
+  }
+  k_batch_stage<C><<<gridCtas, kStageThreads, smem, s>>>((C*)states, tasks, nTasks, programs);
+  return cudaGetLastError();
+}
+
 extern "C" {
 
 void cvdvBatchStructSizes(int* sizes) {
@@ -289,31 +308,10 @@ int cvdvBatchRunStage(void* states, int precision, const CvdvBatchTask* tasks, i
   if (nTasks == 0) return kOk;
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaSuccess;
-  // the shared-memory opt-in is set once per process (so later calls can be captured)
-  static bool attr128 = false, attr64 = false;
   {
     LaunchScope _ls(nullptr, kKFft);
-    if (precision == kC128) {
-      const size_t smem = stage_smem<double2>() + stage_quad_bytes();
-      if (!attr128) {
-        e = cudaFuncSetAttribute(k_batch_stage<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr128 = e == cudaSuccess;
-      }
-      if (e == cudaSuccess) {
-        k_batch_stage<double2><<<gridCtas, kStageThreads, smem, s>>>((double2*)states, tasks, nTasks, programs);
-        e = cudaGetLastError();
-      }
-    } else {
-      const size_t smem = stage_smem<float2>() + stage_quad_bytes();
-      if (!attr64) {
-        e = cudaFuncSetAttribute(k_batch_stage<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr64 = e == cudaSuccess;
-      }
-      if (e == cudaSuccess) {
-        k_batch_stage<float2><<<gridCtas, kStageThreads, smem, s>>>((float2*)states, tasks, nTasks, programs);
-        e = cudaGetLastError();
-      }
-    }
+    e = precision == kC128 ? launch_stage<double2>(states, tasks, nTasks, programs, gridCtas, s)
+                           : launch_stage<float2>(states, tasks, nTasks, programs, gridCtas, s);
   }
   if (e != cudaSuccess) {
     set_error(nullptr, kErrCuda, "%s: %s", fn, cudaGetErrorString(e));

@@ -486,13 +486,16 @@ static cudaError_t launch_rowr_s(Context* ctx, const void* in, void* out, const 
   const size_t smem = (size_t)rr_line_slots<C, LOGM, LOGE, LOGR, COL>() * (1 << LOGR) * sizeof(C) +
                       (FULL ? sizeof(C) << LOGM : rr_tw_slots(LOGM) * sizeof(double2));
   auto kern = k_rowr<C, LOGM, LOGR, LOGE, COL, FULL>;
-  static int resident = 0;  // CTAs per SM of this instantiation, asked once
-  cudaError_t e = cudaSuccess;
+  // CTAs per SM of this instantiation: opted in and asked once per device
+  static std::atomic<int> perDevice[kMaxDevices];
+  const bool known = ctx->device >= 0 && ctx->device < kMaxDevices;
+  int resident = known ? perDevice[ctx->device].load(std::memory_order_acquire) : 0;
   if (!resident) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, NT, smem);
     if (e != cudaSuccess || resident < 1) return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+    if (known) perDevice[ctx->device].store(resident, std::memory_order_release);
   }
   uint64_t nTiles = ctx->size() >> (LOGM + LOGR);
   if (nTiles < 1) nTiles = 1;

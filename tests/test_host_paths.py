@@ -29,6 +29,12 @@ def set_state(L, h):
     assert error(L, h)[0] == 0
 
 
+def device_array(L, count):
+    p = ctypes.c_void_p()
+    assert L.cudaMalloc(ctypes.byref(p), 8 * count) == 0
+    return p
+
+
 def test_stand_in_runs_a_circuit(L):
     h = context(L, [1, 10])
     set_state(L, h)
@@ -96,3 +102,26 @@ def test_a_failed_launch_inside_a_transform_leaves_no_state(L):
         states.append(error(L, h)[0] == 0)
         L.cvdvDestroy(h)
     assert kernels[-2:] == [True, True] and states == [True] * (len(states) - 1) + [False]
+
+
+def test_a_second_device_opts_in_to_shared_memory(L):
+    """2^8-point columns of a large complex128 state take 70 KB of shared memory: every
+    device a process uses has to opt in."""
+    for device in (0, 1, 0):
+        L.fake_set_device(device)
+        h = context(L, [8, 11])
+        set_state(L, h)
+        L.cvdvRotation(h, 0, 0.3)
+        L.cvdvFlush(h)
+        assert error(L, h) == (0, ""), device
+        L.cvdvDestroy(h)
+    L.fake_set_device(0)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_stages_opt_in_on_every_device(L, precision):
+    states, tasks, programs = device_array(L, 64), device_array(L, 64), device_array(L, 1024)
+    for device in (0, 1, 0):
+        L.fake_set_device(device)
+        assert L.cvdvBatchRunStage(states, precision, tasks, 1, programs, 1, None) == 0, device
+    L.fake_set_device(0)
