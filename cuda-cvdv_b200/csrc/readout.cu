@@ -771,6 +771,7 @@ void cvdvGetState(CVDVContext* ctx, double* realOut, double* imagOut) {
   if (!ctx) return;
   Context* c = C(ctx);
   if (!ready(c, "cvdvGetState") || !realOut || !imagOut) return;
+  arena_reset(c);
   uint64_t n = c->size();
   const uint64_t chunk = 1ull << 22;
   uint64_t cnt0 = n < chunk ? n : chunk;

@@ -125,3 +125,16 @@ def test_batch_stages_opt_in_on_every_device(L, precision):
         L.fake_set_device(device)
         assert L.cvdvBatchRunStage(states, precision, tasks, 1, programs, 1, None) == 0, device
     L.fake_set_device(0)
+
+
+def test_state_readbacks_take_no_more_memory(L):
+    h = context(L, [22], precision=1)
+    set_state(L, h)
+    re, im = ((ctypes.c_double * (1 << 22))() for _ in range(2))
+    L.cvdvGetState(h, re, im)
+    L.cvdvGetState(h, re, im)
+    held = L.fake_device_bytes()
+    for _ in range(3):
+        L.cvdvGetState(h, re, im)
+    assert error(L, h)[0] == 0 and L.fake_device_bytes() == held
+    L.cvdvDestroy(h)
