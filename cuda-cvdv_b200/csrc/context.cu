@@ -99,6 +99,7 @@ int global_error(char* msg, int len) {
 
 bool cuda_ok(Context* ctx, cudaError_t e, const char* what) {
   if (e == cudaSuccess) return true;
+  cudaGetLastError();  // reported here: the next launch's check must not find it again
   set_error(ctx, kErrCuda, "%s: %s", what, cudaGetErrorString(e));
   return false;
 }

@@ -5,6 +5,8 @@
 // the per-element work is a handful of FP64 multiplies against factor tables
 // that stay resident in L1/L2.
 
+#include <cudaTypedefs.h>
+
 #include "cvdv_internal.cuh"
 #include "turns.cuh"
 
@@ -538,9 +540,28 @@ __global__ void __launch_bounds__(256) k_gather_arrays(const __grid_constant__ G
   }
 }
 
+// Whether [p, p + bytes) lies in one allocation, as a copy call checks before it reads.
+// False where the driver cannot tell.
+static bool in_one_allocation(const void* p, size_t bytes) {
+  static const PFN_cuMemGetAddressRange_v3020 range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &found) != cudaSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  if (!range || range(&base, &size, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return false;
+  return bytes <= size - (size_t)((uintptr_t)p - (uintptr_t)base);
+}
+
 // Copies the register arrays (of any memory) to dst, back to back, on the context's
-// stream.  Arrays in this device's memory, 16-byte aligned and of 2^16 elements at
-// most in total (larger ones are the copy engine's), are gathered by one kernel.
+// stream.  Arrays in this device's memory, 16-byte aligned, whole, and of 2^16 elements at
+// most in total (larger ones are the copy engine's) are gathered by one kernel; the
+// others go by copy calls, which refuse an array that ends before its register.
 bool copy_register_arrays(Context* ctx, void* const* arrays, double2* dst, const char* what) {
   const int R = ctx->numReg;
   GatherDesc D;
@@ -556,7 +577,8 @@ bool copy_register_arrays(Context* ctx, void* const* arrays, double2* dst, const
       cudaGetLastError();
       gather = false;
     } else {
-      gather = a.type == cudaMemoryTypeDevice && a.device == ctx->device;
+      gather = a.type == cudaMemoryTypeDevice && a.device == ctx->device &&
+               in_one_allocation(arrays[r], sizeof(double2) << ctx->q[r]);
     }
     D.src[r] = (const double2*)arrays[r];
     D.end[r] = (unsigned)total;

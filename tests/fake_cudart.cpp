@@ -4,6 +4,7 @@
 // runtime refuses: copies outside an allocation or to a null pointer, and launches with
 // more than 48 KB of dynamic shared memory for which the kernel has not opted in on the
 // current device.  fake_* are the tests' controls.
+#include <cuda.h>
 #include <cuda_runtime_api.h>
 
 #include <cstdint>
@@ -173,6 +174,21 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   auto it = find(p);
   a->type = it == blocks.end() ? cudaMemoryTypeUnregistered : it->second.device < 0 ? cudaMemoryTypeHost : cudaMemoryTypeDevice;
   a->device = it == blocks.end() ? -1 : it->second.device;
+  return cudaSuccess;
+}
+static CUresult address_range(CUdeviceptr* base, size_t* size, CUdeviceptr p) {
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  auto it = find((const void*)(uintptr_t)p);
+  if (it == blocks.end()) return CUDA_ERROR_NOT_FOUND;
+  *base = (CUdeviceptr)it->first;
+  *size = it->second.bytes;
+  return CUDA_SUCCESS;
+}
+cudaError_t cudaGetDriverEntryPointByVersion(const char* name, void** f, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult* found) {
+  const bool known = !strcmp(name, "cuMemGetAddressRange");
+  *f = known ? (void*)address_range : nullptr;
+  if (found) *found = known ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
   return cudaSuccess;
 }
 cudaError_t cudaGetSymbolAddress(void** p, const void* symbol) {

@@ -138,3 +138,18 @@ def test_state_readbacks_take_no_more_memory(L):
         L.cvdvGetState(h, re, im)
     assert error(L, h)[0] == 0 and L.fake_device_bytes() == held
     L.cvdvDestroy(h)
+
+
+def test_short_register_arrays_are_refused(L):
+    """A device array with fewer amplitudes than its register is an error, not a read
+    past its end; with enough of them, at whatever offset, it is taken."""
+    h = context(L, [4, 5])
+    a, b = device_array(L, 2 << 4), device_array(L, (2 << 5) - 2)
+    for short in ((a, b), (ctypes.c_void_p(a.value + 16), device_array(L, 2 << 5))):
+        L.cvdvInitFromSeparable(h, (ctypes.c_void_p * 2)(*short), 2)
+        assert error(L, h)[0] != 0
+        L.cvdvClearError(h)
+    c = device_array(L, 2 << 6)
+    L.cvdvInitFromSeparable(h, (ctypes.c_void_p * 2)(a, c.value + (16 << 5)), 2)
+    assert error(L, h)[0] == 0
+    L.cvdvDestroy(h)
