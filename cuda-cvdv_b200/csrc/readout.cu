@@ -732,13 +732,30 @@ struct HostPart {
   double* to;
   size_t at, count;
 };
+// Whether the host can write all parts itself: results may go to device memory too, by
+// copy calls only.
+static bool host_memory(const std::vector<HostPart>& parts) {
+  const double* next = nullptr;
+  for (const HostPart& p : parts) {
+    if (p.to != next) {  // (parts that follow one another are one array)
+      cudaPointerAttributes a{};
+      if (cudaPointerGetAttributes(&a, p.to) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      if (a.type == cudaMemoryTypeDevice) return false;
+    }
+    next = p.to + p.count;
+  }
+  return true;
+}
 // Waits for the parts of a device buffer of `total` doubles: small buffers come back
 // in one copy to the context's pinned block (a copy per register to pageable memory
 // took 10 us each), large parts through copy_to_host.
 static bool read_back(Context* c, const std::vector<HostPart>& parts, const double* src, size_t total, const char* what) {
   constexpr size_t kSmall = (Context::kPinnedBytes - Context::kPinnedScratchAt) / sizeof(double);
   constexpr size_t kLarge = (2u << 20) / sizeof(double);
-  double* hs = total <= kSmall ? host_scratch(c, total) : nullptr;
+  double* hs = total <= kSmall && host_memory(parts) ? host_scratch(c, total) : nullptr;
   if (hs) {
     if (!cuda_ok(c, cudaMemcpyAsync(hs, src, total * sizeof(double), cudaMemcpyDeviceToHost, c->stream), what) ||
         !stream_sync(c, what))

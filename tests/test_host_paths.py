@@ -153,3 +153,13 @@ def test_short_register_arrays_are_refused(L):
     L.cvdvInitFromSeparable(h, (ctypes.c_void_p * 2)(a, c.value + (16 << 5)), 2)
     assert error(L, h)[0] == 0
     L.cvdvDestroy(h)
+
+
+def test_readouts_into_device_memory_are_copied(L):
+    """The host writes no results to memory that is not its own."""
+    h = context(L, [3, 4])
+    set_state(L, h)
+    out = device_array(L, 8)
+    L.cvdvMeasureMultiple(h, (ctypes.c_int * 1)(0), 1, ctypes.cast(out, ctypes.POINTER(ctypes.c_double)))
+    assert error(L, h)[0] == 0 and L.fake_copied_to(out) == 64
+    L.cvdvDestroy(h)
