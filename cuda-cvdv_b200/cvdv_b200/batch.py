@@ -15,8 +15,8 @@ follow the single-instance path exactly (thresholds 1e-12 / 1e-15, rint for the
 rotation's quarter turns, dropped global phases), so every instance matches
 ``CudaCvdv`` running the same gates.
 
-Tuning: ``autotune()`` times candidates on the compiled batch: the persistent
-grid size, the pair-gate chunk (the 2x2-gate tasks' shape), and, per mode
+Tuning: ``autotune()`` times candidates on the compiled batch: the limit on
+a stage's CTAs, the pair-gate chunk (the 2x2-gate tasks' shape), and, per mode
 length 2^m of the batch, the row tasks' amplitudes per thread 2^logE -- which
 is both the radix schedule of their transforms (radix-8, 16 or 32 Stockham
 stages) and the rows a CTA holds (512 2^logE / 2^m) -- by coordinate descent
@@ -45,8 +45,8 @@ TASK_DTYPE = np.dtype([("stateOffset", "i8"), ("kind", "i4"), ("n", "i4"), ("log
 OP_DIAG, OP_FWD, OP_INV, OP_PARITY = 0, 1, 2, 3
 SQRT2 = math.sqrt(2.0)
 THREADS = 512
-# A stage launches a CTA per task up to this many (self.grid at least), so an SM that
-# finishes early takes the next task; past it the CTAs walk the list.  512 circuits, 1283
+# A stage launches a CTA per task up to this many unless the caller sets a limit, so an SM
+# that finishes early takes the next task; past it the CTAs walk the list.  512 circuits, 1283
 # tasks a stage: 3.17 ms per 20 stages against 3.53 with 148 CTAs.
 MAX_CTAS = 1024
 
@@ -237,15 +237,16 @@ class BatchedCircuits:
     QUBIT_GATES = ("h", "rx", "ry", "rz")
 
     def __init__(self, instances: Sequence[Dict[str, Any]], precision: str = "complex64",
-                 pair_chunk: int = 4096, grid: int = 148, row_loge: Optional[Dict[int, int]] = None) -> None:
+                 pair_chunk: int = 4096, grid: Optional[int] = None, row_loge: Optional[Dict[int, int]] = None) -> None:
         """instances: dicts with ``qubits`` ([1]*Q + [m]) and ``gates`` [(name, args)];
         row_loge: amplitudes per thread (log2) of the row tasks per mode length m
         (default 4, or 5 for complex64 modes of 2^13 and 2^14 points; less for batches
-        that do not fill the chip, adaptive_loge).  grid: CTAs of a stage, at least."""
+        that do not fill the chip, adaptive_loge).  grid: CTAs of a stage, at most (default
+        MAX_CTAS); a stage of fewer tasks launches a CTA per task."""
         self.prec = PRECISIONS[precision]
         self.cdtype = torch.complex128 if self.prec == 0 else torch.complex64
         self.instances = list(instances)
-        self.grid = grid
+        self.grid = MAX_CTAS if grid is None else grid
         self.pair_chunk = pair_chunk
         self.row_loge: Dict[int, int] = dict(row_loge or {})
         for m, e in self.row_loge.items():
@@ -324,8 +325,8 @@ class BatchedCircuits:
 
         self._tasks = []
         for tl in stage_tasks:
-            # the CTAs take tasks round-robin: largest first, so the long row programs
-            # start in the first wave instead of trailing the stage
+            # largest first: the long row programs start in the first wave instead of
+            # trailing the stage (CTAs take tasks in order, each every grid-th one)
             tl = sorted(tl, key=cost, reverse=True)
             arr = np.array(tl, dtype=TASK_DTYPE) if tl else np.zeros(0, dtype=TASK_DTYPE)
             self._validate(arr)
@@ -390,7 +391,7 @@ class BatchedCircuits:
             code = self._L.cvdvBatchRunStage(ctypes.c_void_p(self.states.data_ptr()), self.prec,
                                              ctypes.c_void_p(tasks.data_ptr()), nt,
                                              ctypes.c_void_p(self._progs.data_ptr()),
-                                             max(self.grid, min(nt, MAX_CTAS)), stream)
+                                             min(max(nt, 1), self.grid), stream)
             if code:
                 raise CvdvError(_lib.last_error(None)[1])
 
@@ -422,7 +423,7 @@ class BatchedCircuits:
         e1.synchronize()
         return e0.elapsed_time(e1) / reps
 
-    def autotune(self, grids: Sequence[int] = (148, 296), chunks: Sequence[int] = (2048, 8192),
+    def autotune(self, grids: Sequence[int] = (148, 296, MAX_CTAS), chunks: Sequence[int] = (2048, 8192),
                  reps: int = 3, tune_rows: bool = True) -> Tuple[int, int]:
         """Time every (grid, pair chunk) pair on the compiled batch and keep the
         fastest; then, per mode length (largest total work first), every row-task
