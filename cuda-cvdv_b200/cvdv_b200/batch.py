@@ -266,11 +266,12 @@ class BatchedCircuits:
         self.states = torch.zeros(self.total, dtype=self.cdtype, device="cuda")
         self._L = _lib.load()
         self._graph = None
+        # (counted once: the row shapes stay the same while other settings are tuned)
+        self._tasks_per_stage = self._count_tasks() / max(1, self.n_stages)
         self._compile()
 
     # ---------------------------------------------------------------- compile
     def _compile(self) -> None:
-        self._tasks_per_stage = self._count_tasks() / max(1, self.n_stages)
         progs: List[np.void] = []
         stage_tasks: List[List[np.void]] = [[] for _ in range(self.n_stages)]
         for i, inst in enumerate(self.instances):
@@ -333,7 +334,7 @@ class BatchedCircuits:
             self._tasks.append((torch.from_numpy(arr.view(np.uint8).copy()).cuda(), len(arr)))
 
     def _count_tasks(self) -> int:
-        """Tasks of all stages at the default shapes."""
+        """Tasks of all stages at the default shapes and the constructor's pair chunk."""
         total = 0
         for inst in self.instances:
             n, m = sum(inst["qubits"]), inst["qubits"][-1]

@@ -37,3 +37,20 @@ def test_the_grid_limits_the_ctas(launches, grid, limit, count):
     b = BatchedCircuits(circuits(count), grid=grid) if grid else BatchedCircuits(circuits(count))
     b.run()
     assert launches == [(count, min(count, limit))] * 2
+
+
+def test_tuning_the_chunk_keeps_the_row_shapes(launches, monkeypatch):
+    """Every trial of grids and chunks has the row shapes the batch was made with, and the
+    shapes that the row trials keep are those of the best time."""
+    # 150 tasks a stage as made, 450 with chunks of 1024 pairs: on both sides of a shape's line
+    b = BatchedCircuits(circuits(100, m=13, gates=[("h", (0, 0)), ("d", (1, 0.3 + 0.1j))]))
+    shapes, trials = {13: b._loge(13)}, []
+
+    def clock(self, reps):
+        trials.append((self.grid, self.pair_chunk, self._loge(13)))
+        return 1.0 + (self._loge(13) != shapes[13])  # the first trial's settings are the fastest
+
+    monkeypatch.setattr(BatchedCircuits, "_time", clock)
+    best = b.autotune(grids=(148, 296), chunks=(1024, 8192))
+    assert [t[2] for t in trials[:4]] == [shapes[13]] * 4
+    assert best == (148, 1024) and b.row_loge == shapes
