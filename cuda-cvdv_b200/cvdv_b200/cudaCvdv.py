@@ -206,7 +206,7 @@ class CudaCvdv:
 
     def stateTensor(self) -> torch.Tensor:
         """(addition) zero-copy torch view of the live device state (complex128
-        or complex64), valid until the next gate runs."""
+        or complex64), valid until the next gate runs.  It keeps the simulator alive."""
         ptr = self._L.cvdvGetStateDevicePtr(self.ctx)
         self._check()
         if not ptr:
@@ -218,7 +218,9 @@ class CudaCvdv:
                                         "data": (int(ptr), False), "version": 3,
                                         "stream": None}
         self._L.cvdvSynchronize(self.ctx)
-        return torch.as_tensor(_View(), device="cuda")
+        view = _View()
+        view.simulator = self  # torch keeps the view, so the memory lives as long as the tensor
+        return torch.as_tensor(view, device="cuda")
 
     def getXGrid(self, r: int) -> npt.NDArray[np.float64]:
         N = self.register_dims[r]
