@@ -91,6 +91,11 @@ long fake_launches() { return launches; }
 void fake_fail_at(long n) { failAt = n; }  // the n-th launch from the start fails; -1: none
 const char* fake_last_kernel() { return lastKernel.c_str(); }
 void fake_set_device(int d) { current = d; }
+void fake_count_up() {  // the doubles of every device block become 0, 1, 2, ...
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  for (auto& b : blocks)
+    for (size_t i = 0; b.second.device >= 0 && i < b.second.bytes / 8; ++i) ((double*)b.first)[i] = (double)i;
+}
 size_t fake_copied_to(const void* p) {  // bytes of the last copy to p (0: none)
   std::lock_guard<std::recursive_mutex> lk(mu);
   auto it = copiedTo.find((uintptr_t)p);
@@ -153,10 +158,12 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t bytes, cudaMemcpyKind, cudaStream_t) {
-  std::lock_guard<std::recursive_mutex> lk(mu);
-  if (!inside(d, bytes) || !inside(s, bytes)) return done(cudaErrorInvalidValue);
+  {
+    std::lock_guard<std::recursive_mutex> lk(mu);
+    if (!inside(d, bytes) || !inside(s, bytes)) return done(cudaErrorInvalidValue);
+    copiedTo[(uintptr_t)d] = bytes;
+  }
   memmove(d, s, bytes);
-  copiedTo[(uintptr_t)d] = bytes;
   return cudaSuccess;
 }
 cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind, cudaStream_t) {

@@ -1,7 +1,9 @@
 """Host code of the library without a GPU, on a stand-in CUDA runtime (host_runtime.py)."""
 
 import ctypes
+import threading
 
+import numpy as np
 import pytest
 
 from . import host_runtime
@@ -163,3 +165,37 @@ def test_readouts_into_device_memory_are_copied(L):
     L.cvdvMeasureMultiple(h, (ctypes.c_int * 1)(0), 1, ctypes.cast(out, ctypes.POINTER(ctypes.c_double)))
     assert error(L, h)[0] == 0 and L.fake_copied_to(out) == 64
     L.cvdvDestroy(h)
+
+
+@pytest.mark.parametrize("readers", [1, 3])  # one takes the staged chunks and their threads, the others plain copies
+@pytest.mark.parametrize("shift", [0, 40])
+def test_large_readbacks_arrive_whole(L, readers, shift):
+    n = 1 << 22
+    hs = [context(L, [22], precision=1) for _ in range(readers)]
+    outs = [np.full(2 * n + 1024, -1.0) for _ in hs]
+    for h in hs:
+        set_state(L, h)
+        L.cvdvGetNorm(h)
+
+    def first(out):  # on a page, or off it
+        return (-out.ctypes.data // 8) % 512 + shift
+
+    def read(h, out):
+        L.cvdvGetState(h, *(ctypes.cast(out.ctypes.data + 8 * (first(out) + k * n), ctypes.POINTER(ctypes.c_double))
+                            for k in range(2)))
+
+    for h, out in zip(2 * hs, 2 * outs):
+        read(h, out)  # (the split arrays have their place from the second on)
+    L.fake_count_up()
+    for out in outs:
+        out[:] = -1.0
+    threads = [threading.Thread(target=read, args=a) for a in zip(hs, outs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for h, out in zip(hs, outs):
+        got, at = out[first(out): first(out) + 2 * n], first(out)
+        assert error(L, h)[0] == 0 and (np.diff(got) == 1).all()
+        assert (out[:at] == -1).all() and (out[at + 2 * n:] == -1).all()
+        L.cvdvDestroy(h)
