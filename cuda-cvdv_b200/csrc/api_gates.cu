@@ -370,9 +370,6 @@ static void release(Context* c) {
     if (p) cudaFree(p);
     p = nullptr;
   }
-  if (c->hostScratch) cudaFreeHost(c->hostScratch);
-  c->hostScratch = nullptr;
-  c->hostScratchCap = 0;
   c->allocElems = 0;
   c->initialized = false;
   c->pending.clear();

@@ -178,19 +178,11 @@ void* big_scratch(Context* ctx, size_t bytes) {
 }
 
 double* host_scratch(Context* ctx, size_t count) {
-  size_t bytes = count * sizeof(double);
-  if (ctx->waitErr && bytes <= Context::kPinnedBytes - Context::kPinnedScratchAt)
-    return (double*)((char*)ctx->waitErr + Context::kPinnedScratchAt);
-  if (bytes <= ctx->hostScratchCap) return ctx->hostScratch;
-  if (ctx->hostScratch) cudaFreeHost(ctx->hostScratch);
-  ctx->hostScratch = nullptr;
-  ctx->hostScratchCap = 0;
-  if (cudaMallocHost(&ctx->hostScratch, bytes) != cudaSuccess) {
-    set_error(ctx, kErrAlloc, "pinned host scratch (%zu bytes) failed", bytes);
+  if (!ctx->waitErr || count * sizeof(double) > Context::kPinnedBytes - Context::kPinnedScratchAt) {
+    set_error(ctx, kErrAlloc, "no pinned block for %zu values", count);
     return nullptr;
   }
-  ctx->hostScratchCap = bytes;
-  return ctx->hostScratch;
+  return (double*)((char*)ctx->waitErr + Context::kPinnedScratchAt);
 }
 
 bool ensure_state(Context* ctx) {

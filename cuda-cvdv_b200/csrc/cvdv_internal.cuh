@@ -297,10 +297,6 @@ struct Context {
   void* big = nullptr;
   size_t bigCap = 0;
 
-  // pinned host staging for small D2H results
-  double* hostScratch = nullptr;
-  size_t hostScratchCap = 0;
-
   std::vector<Stage> pending;
   // Basis-change cancellation: FtQ2P(r) after FtP2Q(r) (or the reverse) with only
   // stages that leave register r untouched in between is the identity; both are
@@ -382,7 +378,7 @@ bool stream_sync(Context* ctx, const char* what);
 void* arena_alloc(Context* ctx, size_t bytes);   // reset per flush / readout
 void arena_reset(Context* ctx);
 void* big_scratch(Context* ctx, size_t bytes);   // persistent, grown on demand
-double* host_scratch(Context* ctx, size_t count);
+double* host_scratch(Context* ctx, size_t count);  // small results, in the context's pinned block
 // Copies device memory to host memory and waits for it (host_copy.cu); contexts count
 // themselves there for the staging memory's lifetime.
 bool copy_to_host(Context* ctx, void* dst, const void* src, size_t bytes, const char* what);
