@@ -311,6 +311,11 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOG
   constexpr int LOGI = COL ? LOGR : 0;
   constexpr bool TWO = rr_use_two<C, LOGM, LOGE, LOGR, COL>();
   constexpr bool PF = COL && ONE && TWO;  // the next tile is copied ahead
+  // The first tile is loaded while the twiddles are fetched: in complex128, where it makes up
+  // for the two-word phases (rotation, displacement and squeeze of 2^10-point columns of a 2^22
+  // state 160 -> 152 us, of 2^13-point rows of a 2^24 state 723 -> 711); complex64 is slower
+  // with it (2^10-point columns 116 -> 118).
+  constexpr bool AHEAD = !PF && sizeof(C) == sizeof(double2);
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
   C* tws = sm + (RS << LOGR);  // the twiddles
@@ -322,6 +327,19 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOG
   C* smrow = sm + row * RS;
   const int logS = COL ? P.logS : 0;
   if constexpr (LOGM <= 8) row &= P.rowMask;  // (longer rows: LOGR = 0 where rows are few)
+
+  C v[E];
+  if constexpr (AHEAD) {
+    uint64_t base;
+    if constexpr (COL) {
+      const uint64_t c = ((uint64_t)blockIdx.x << LOGR) + (uint64_t)row;
+      base = (c & ((1ull << logS) - 1)) + ((c >> logS) << (LOGM + logS));
+    } else {
+      base = ((uint64_t)blockIdx.x << (LOGM + LOGR)) + ((uint64_t)row << LOGM);
+    }
+#pragma unroll
+    for (int k = 0; k < E; ++k) v[k] = in[base + ((uint64_t)(t + k * TPR) << logS)];
+  }
 
   const int scM = P.logTwN - LOGM;
   const auto tw = [&] {
@@ -377,14 +395,13 @@ __global__ void __launch_bounds__(1 << (LOGM - LOGE + LOGR), rr_one<C, LOGM, LOG
       if (ONE && more) l2_prefetch_tile(in + ((tile + gridDim.x) << (LOGM + LOGR)), TILE_BYTES);
       rowBase = (tile << (LOGM + LOGR)) + ((uint64_t)row << LOGM);
     }
-    C v[E];
     int tau = t;  // v[k] is point tau + k TPR of the row
     if constexpr (PF) {
       cp_async_wait_all();
       __syncthreads();
 #pragma unroll
       for (int k = 0; k < E; ++k) v[k] = sm[tid + k * NT];  // (the exchanges wait for all to be read)
-    } else {
+    } else if (!AHEAD || tile != blockIdx.x) {
 #pragma unroll
       for (int k = 0; k < E; ++k) v[k] = in[rowBase + ((uint64_t)(t + k * TPR) << logS)];
     }
