@@ -749,7 +749,12 @@ static bool issue_plan(Context* ctx) {
 // number of launches, one more than twice the last group's.  The GPU then works on the
 // first ops while the host plans the rest (7-10 us an op), and a long queue still takes
 // few table launches (8 us each with their gaps, more than a short queue's planning).
-// The [9, 10] network, 25 ops: 683 against 740 us per pass.
+// Per pass, in groups against all at once: the [9, 10] network of 6 layers 709-719 against
+// 775-783 us, of 3 layers (8 ops) 403-411 against 428-434; [7, 8] of 3 layers 282-285 against
+// 307-309; 60 gates on [2, 8, 9, 1] 817-820 against 876-886, 16 of them 364-368 against 381-385.
+// Below 8 ops the second table launch costs what the earlier start gains (the [9, 10] network of
+// 2 layers 313-321 against 330-333, of 1 layer 252-255 against 242), and where the kernels are
+// long it makes no difference ([13, 13], 3 layers: 21.8 against 21.9 ms).
 constexpr size_t kEarlyOps = 8;
 static bool issue_early(Context* ctx) {
   FlushPlan* plan = ctx->plan;
