@@ -1,19 +1,19 @@
-// Batched independent circuits: one persistent launch per gate stage.
+// Batched independent circuits: one launch per gate stage.
 //
 // Every instance of the batch has its own layout [1-qubit registers..., mode]
 // and gate list; at stage s each instance applies its s-th gate.  The host turns
 // those gates into tasks (CvdvBatchTask): a row program -- the mode's transforms,
 // parity and diagonal phases, on a group of rows -- or a 2x2 gate on a qubit bit
-// over a range of pairs.  A grid of persistent 512-thread CTAs walks the stage's
-// task list; the task decides the code path, so instances with different gates
-// and mode sizes share one launch.
+// over a range of pairs.  The stage's 512-thread CTAs, one per task up to the caller's
+// limit, walk its task list; the task decides the code path, so instances with different
+// gates and mode sizes share one launch.
 //
-// Row programs keep each row in registers (16 amplitudes per thread for modes
-// up to 2^12 points, 32 for 2^13 and 2^14) and use the Stockham stages of the
-// row kernels; diagonal phases are evaluated per element from a small phase
-// polynomial (FP64 argument with exact transform twiddles, reduced mod 2 pi,
-// then sin/cos in the state's precision), so nothing has to be tabulated per
-// instance.
+// Row programs keep each row in registers (8, 16 or 32 amplitudes per thread, the
+// task's choice) and use the Stockham stages of the row kernels; diagonal phases are
+// running products from a small phase polynomial (phase_run), or evaluated per element
+// where it has a cubic term (phase_factor: FP64 argument with exact transform twiddles,
+// reduced mod 2 pi, then sin/cos in the state's precision), so nothing has to be
+// tabulated per instance.
 
 #include <cmath>
 
@@ -29,8 +29,9 @@ constexpr int kStageThreads = 512;
 // Amplitudes per thread of a row task, 2^LOGE with LOGE = 3, 4 or 5 (radix-8, 16 or
 // 32 Stockham stages; 512 2^LOGE / N rows per CTA), chosen per task (the
 // autotuner's knob).  A row must fit the 512 threads (N / 2^LOGE <= 512) and the
-// CTA's rows the shared memory (complex128: 2^LOGE <= 16).  The default is 32 for
-// complex64 rows of 2^13 and 2^14 points, else 16.
+// CTA's rows the shared memory (complex128: 2^LOGE <= 16).  By default 32 for complex64
+// rows of 2^13 and 2^14 points, else 16, and less for stages that do not fill the chip
+// (adaptive_loge in batch.py, with the times).
 template <typename C> constexpr int stage_max_log() { return sizeof(C) == sizeof(float2) ? 14 : 13; }
 template <typename C> constexpr int stage_max_loge() { return sizeof(C) == sizeof(float2) ? 5 : 4; }
 template <typename C, int LOGN, int LOGE>

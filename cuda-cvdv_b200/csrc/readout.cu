@@ -2,10 +2,13 @@
 //
 // Reductions are two-level and deterministic where they produce a scalar: a
 // fixed grid writes one partial per block, a single block sums the partials in
-// a fixed order.  Marginals accumulate per-block shared-memory histograms with
-// warp aggregation (one shared atomic per warp when every lane of the warp
-// falls in the same bin, which is the case whenever the selected registers are
-// not the lowest 5 index bits), then sum the per-block histograms bin by bin.
+// a fixed order.  Marginals of single registers have one owner per partial
+// (k_marg_axis), several registers above a tile share one pass (k_marg_tiles), and
+// those of registers above a row program's come from the row sums it wrote.  Joint
+// marginals accumulate per-block shared-memory histograms with warp aggregation (one
+// shared atomic per warp when every lane of the warp falls in the same bin, which is
+// the case whenever the selected registers are not the lowest 5 index bits), then sum
+// the per-block histograms bin by bin; past the histogram's size they use global atomics.
 
 #include <cmath>
 #include <cstring>

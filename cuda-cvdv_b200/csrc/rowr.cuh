@@ -27,16 +27,16 @@ struct RowDiag {
   FactorList rowF;     // factors constant along a row
   FactorList elemF;    // per-element factors (bilinear terms with the row register)
   // Bilinear terms c x_row x_other (other register and control bit off the row)
-  // taken out of elemF for k_rowr: along one row they are the linear phase
+  // taken out of elemF for k_rowr and k_rowq: along one row they are the linear phase
   // a (m - regC) regDx with a = sum c x_other (+-1 by the control bit).  The other
   // register is side 1 of each XXFactor.
   int nLin;
   double regC, regDx;
   XXFactor lin[kMaxXX];
-  // k_rowq: a run whose register terms are linear phases (no table): transform
-  // twiddles, the sum of their signs s giving exp(i pi s (N-1)(2n-N+1)/(2N)) at
-  // point n, and terms c x_n (x_n = (n - regC) regDx), each negated when its
-  // control bit (a row bit, or none: -1) is set
+  // A run whose register terms are linear phases (no table; k_rowq, and k_rowr outside
+  // the shapes that keep tables): transform twiddles, the sum of their signs s giving
+  // exp(i pi s (N-1)(2n-N+1)/(2N)) at point n, and terms c x_n (x_n = (n - regC) regDx),
+  // each negated when its control bit (a row bit, or none: -1) is set
   int ftSign;
   int hasQuad;  // k_rowr, 32 amplitudes a thread: the run also has c2 x^2 (uncontrolled terms' sum)
   double c2;
@@ -95,13 +95,14 @@ __device__ __forceinline__ double2 ft_tw_ratio(long long d, long long N, int s) 
 }
 
 // A diagonal run on the amplitudes t + k TPR (k < E) of a row.  Register terms of
-// degree up to two, transform twiddles and bilinear terms need no table: with
+// degree up to two, transform twiddles and bilinear terms need no table (the shapes that
+// keep one all the same: launch_row_program): with
 // u = 2 n - N + 1 and x_n = dx u / 2, dx^2 = 2 pi / N, they are
 //   c2 x^2 = c2 u^2 / (4 N),  a x = a dx u / (4 pi),  twiddle = s (N-1) u / (4 N)
 // turns.  From u0 = 2 t - N + 1 a thread's points are u0 + 2 TPR k, so the factor is
 //   [value at u0] [step]^k [exp(2 pi i (4 c2 / 4 N) TPR^2 k^2)]:
-// two sincospi on turns reduced mod 1, a running product, and (c2 != 0)
-// E constants in the kernel's parameters.  Runs with a controlled c x^2, a cubic or a
+// two sincospi on turns reduced mod 1 (three in complex128), a running product, and
+// (c2 != 0) E constants in the kernel's parameters.  Runs with a controlled c x^2, a cubic or a
 // qubit term keep a table, and so do quadratic runs on shapes other than rr_quads:
 // the sincospi cost more than the loads with 8 or 16 amplitudes a thread (a 2^8-point
 // register's rotation, displacement and squeeze on a 2^26 complex128 state: 2.38 ms

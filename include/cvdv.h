@@ -165,7 +165,7 @@ void* cvdvGetStream(CVDVContext* ctx);
  * on): transforms of a register that is not the last one run as register-resident
  * column DFTs (one pass up to 2^8 points, two passes up to 2^16) instead of the
  * shared-memory tile passes.  flags bit 3 (default on): a run of transforms and
- * diagonal gates on such a register (2^8 .. 2^13 points, 2^14 in complex64) runs
+ * diagonal gates on such a register (2^4 .. 2^13 points, 2^14 in complex64) runs
  * as one pass with each column held on chip.  flags bit 4 (default on): after
  * cvdvInitFromSeparable on two or more registers, the queued stages that act on
  * one register of 2^8 .. 2^14 points alone, ahead of every stage that couples it
