@@ -29,7 +29,7 @@ struct TableBatch {
 };
 
 // Table entry (b, j) = prod over terms.  Terms of degree one and two and transform
-// twiddles are summed in turns, in two words (turns.cuh), and take one sine and cosine;
+// twiddles are summed in turns (turns.cuh) and take one sine and cosine;
 // cubic terms are summed in radians, in the reference's order of operations (x = (idx -
 // (dim-1)*0.5)*dx, kernelPhaseX3, src/cuda/kernels/gates.cuh:5-16,184-209).
 //
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kTableThreads) k_build_tables(const __grid_con
   const int u = 2 * j - N + 1;
   const double inv4N = 0.25 / (double)N;
   const LinTurns L = lin_turns(H.logN);
-  Turns<double2> p;
+  Turns1<true> p;
   double cubic = 0.0;
   bool anyTurns = false, anyCubic = false;
   double2 f = make_double2(1.0, 0.0);
@@ -69,12 +69,10 @@ __global__ void __launch_bounds__(kTableThreads) k_build_tables(const __grid_con
       const bool neg = (D.ctrlMode == 1 && ((b >> D.ctrlLocal) & 1)) || (D.ctrlMode == 2 && ((j >> D.ctrlLocal) & 1));
       const double c = neg ? -D.coeff : D.coeff;
       if (D.power == 1) {
-        double ch, cl;
-        Turns<double2>::scale(c, L.hi, L.lo, ch, cl);
-        p.add(ch, cl, (double)u);
+        p.add(turn_rate(c, L.hi, L.lo), (double)u);
         anyTurns = true;
       } else if (D.power == 2) {
-        p.add(c * inv4N, 0.0, (double)u * (double)u);
+        p.add({c * inv4N, 0.0}, (double)u * (double)u);
         anyTurns = true;
       } else {
         const double x = 0.5 * (double)u * H.dx;
@@ -84,7 +82,7 @@ __global__ void __launch_bounds__(kTableThreads) k_build_tables(const __grid_con
     } else if (D.kind == kTermFtTw) {
       const long long n = N;  // (N-1) u mod 4N, N a power of two
       const long long m = (((n - 1) * u + 2 * n) & (4 * n - 1)) - 2 * n;
-      p.add_hi((double)D.sign * (double)m * inv4N);
+      p.add({(double)D.sign * inv4N, 0.0}, (double)m);
       anyTurns = true;
     } else if (D.kind == kTermBit) {
       f = dmul(f, ((j >> D.bit) & 1) ? D.g1 : D.g0);

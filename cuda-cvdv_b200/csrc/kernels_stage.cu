@@ -16,6 +16,7 @@
 // tabulated per instance.
 
 #include <cmath>
+#include <type_traits>
 
 #include "../../include/cvdv.h"
 #include "cvdv_internal.cuh"
@@ -88,8 +89,9 @@ __device__ __forceinline__ C phase_factor(const CvdvBatchPhase& P, int j, int N,
 // polynomial per point took about 25 FP64 operations, the conversions of its integers
 // and a fast sine and cosine each, about as long as the transforms between the phases;
 // this takes 8, and is exact to FP64 where the fast intrinsic was to 4e-7.
-// 96 circuits of 50 gates: 3.42 -> 3.30 ms, error 9.3e-6 -> 4.1e-6.  In complex128 the turns
-// are kept in two words (turns.cuh): a displacement on 2^11 points 3.0e-15 (per point) -> 1.2e-15.
+// 96 circuits of 50 gates: 3.42 -> 3.30 ms, error 9.3e-6 -> 4.1e-6.  In complex128 the
+// products keep their low words (turns.cuh) and a run of 16 starts anew at the eighth point: a
+// displacement on 2^11 points is off by 0.9e-15 (3.0e-15 with the phases evaluated per point).
 template <typename C, int LOGN, int LOGE>
 __device__ __forceinline__ void phase_run(C (&v)[1 << LOGE], const CvdvBatchPhase& P, int t, double zs, double2* kq) {
   constexpr int E = 1 << LOGE, N = 1 << LOGN, TPR = N >> LOGE, LANES = TPR < 32 ? TPR : 32;
@@ -97,31 +99,29 @@ __device__ __forceinline__ void phase_run(C (&v)[1 << LOGE], const CvdvBatchPhas
   const int u0 = 2 * t - N + 1;
   constexpr LinTurns L = lin_turns(LOGN);
   constexpr double perTurn = 0.5 / M_PI, perTurnLo = -9.839338337591243e-18;  // 1 / (2 pi) in two words
-  double linH, linL, constH, constL;
-  Turns<C>::scale(P.a1 + zs * P.b1, L.hi, L.lo, linH, linL);
-  Turns<C>::scale(P.g0 + zs * P.h0, perTurn, perTurnLo, constH, constL);
-  const double q = (P.a2 + zs * P.b2) * inv4N;
+  const TurnRate lin = turn_rate(P.a1 + zs * P.b1, L.hi, L.lo), q = {(P.a2 + zs * P.b2) * inv4N, 0.0};
   // tw (N-1) u / (4N) turns, in -1/2 .. 1/2
   const int w = (P.tw * (N - 1)) & (4 * N - 1);
   auto twiddle = [&](int u) {
     return (double)(((int)((long long)w * u + 2 * N) & (4 * N - 1)) - 2 * N) * inv4N;
   };
-  Turns<C> p0, p1;
-  p0.add_hi(twiddle(u0));
-  p1.add_hi(twiddle(2 * TPR));
-  p0.add(linH, linL, (double)u0);
-  p1.add(linH, linL, 2.0 * TPR);
-  p0.add(constH, constL, 1.0);
+  // (a run of 8 repeats a sum's rounding too seldom to pay for the second word: small batches)
+  constexpr bool C128 = sizeof(C) == sizeof(double2);
+  using Turns = std::conditional_t<C128 && E >= 16, Turns2, Turns1<C128>>;
+  Turns p0(twiddle(u0)), p1(twiddle(2 * TPR));
+  p0.add(lin, (double)u0);
+  p1.add(lin, 2.0 * TPR);
+  p0.add(turn_rate(P.g0 + zs * P.h0, perTurn, perTurnLo), 1.0);
   const bool quad = P.a2 != 0.0 || P.b2 != 0.0;  // the same for every row of the task
   if (quad) {
-    p0.add(q, 0.0, (double)u0 * (double)u0);
-    p1.add(q, 0.0, 4.0 * TPR * (double)u0);
+    p0.add(q, (double)u0 * (double)u0);
+    p1.add(q, 4.0 * TPR * (double)u0);
     __syncwarp();  // the last run's constants are read
     const int lane = t & (LANES - 1);
 #pragma unroll
     for (int k = lane; k < E; k += LANES) {
-      Turns<C> pk;
-      pk.add(q, 0.0, 4.0 * TPR * TPR * (double)(k * k));
+      Turns pk;
+      pk.add(q, 4.0 * TPR * TPR * (double)(k * k));
       kq[k] = pk.root();
     }
     __syncwarp();
@@ -132,7 +132,7 @@ __device__ __forceinline__ void phase_run(C (&v)[1 << LOGE], const CvdvBatchPhas
   const double2 st = p1.root();
   // in complex128 from the eighth point's factor anew: a step's rounding is repeated
   // 7 + 1 times at most instead of 15
-  constexpr bool ANCHOR = E >= 16 && sizeof(C) == sizeof(double2);
+  constexpr bool ANCHOR = E >= 16 && C128;
   double2 eighth = f;
   if constexpr (ANCHOR) eighth = dmul(f, p1.times(8.0).root());
 #pragma unroll

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cmath>
+#include <type_traits>
 
 #include "cvdv_internal.cuh"
 #include "row_fft.cuh"
@@ -133,8 +134,7 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
     for (int k = 0; k < D.nPl; ++k)
       a += (D.plCtrl[k] >= 0 && ((rowBase >> D.plCtrl[k]) & 1ull)) ? -D.plC[k] : D.plC[k];
     constexpr LinTurns L = lin_turns(LOGM);
-    double ah, al;
-    Turns<C>::scale(a, L.hi, L.lo, ah, al);
+    const TurnRate lr = turn_rate(a, L.hi, L.lo);
     const int u0 = 2 * t - N + 1;
     // s (N-1) u mod 4N in integers: at most 3 2^28 for the runs of a program
     constexpr double inv4N = 1.0 / (4.0 * N);
@@ -142,15 +142,14 @@ __device__ __forceinline__ void rr_diag(C (&v)[1 << LOGE], const RowDiag& D, uin
     auto twiddle = [&](int u) {  // s (N-1) u / (4N) turns, in -1/2 .. 1/2
       return (double)(((int)((long long)w * u + 2 * N) & (4 * N - 1)) - 2 * N) * inv4N;
     };
-    Turns<C> p0, p1;
-    p0.add_hi(twiddle(u0));
-    p1.add_hi(twiddle(2 * TPR));
-    p0.add(ah, al, (double)u0);
-    p1.add(ah, al, 2.0 * TPR);
+    using Turns = std::conditional_t<sizeof(C) == sizeof(double2), Turns2, Turns1<false>>;
+    Turns p0(twiddle(u0)), p1(twiddle(2 * TPR));
+    p0.add(lr, (double)u0);
+    p1.add(lr, 2.0 * TPR);
     if (QUAD && D.hasQuad) {
-      const double q = D.c2 * inv4N;
-      p0.add(q, 0.0, (double)u0 * (double)u0);
-      p1.add(q, 0.0, 4.0 * TPR * (double)u0);
+      const TurnRate q = {D.c2 * inv4N, 0.0};
+      p0.add(q, (double)u0 * (double)u0);
+      p1.add(q, 4.0 * TPR * (double)u0);
     }
     f = dmul(rs, p0.root());
     st = p1.root();
